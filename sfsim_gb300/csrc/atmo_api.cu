@@ -19,8 +19,6 @@
 
 namespace sfsim {
 template <class Real>
-size_t point_scatter_smem(const BuildDims& d, bool first);
-template <class Real>
 size_t ray_scatter_smem(const BuildDims& d);
 }
 
@@ -317,6 +315,7 @@ BuildDims make_dims(const sfsim_atmo_config& c, int B) {
   std::vector<DirLocal> v;
   sphere_directions(c.sphere_steps >> 1, c.sphere_steps, M_PI, v);
   d.P = (int)v.size();
+  d.T = d.P > 0 ? c.sphere_steps >> 1 : 0;
   sphere_directions(c.ray_steps >> 2, c.ray_steps, M_PI / 2, v);
   d.Ph = (int)v.size();
   d.sun_scale = (d.n2 - 1) / (1 - std::exp(-3.6));
@@ -328,7 +327,7 @@ BuildDims make_dims(const sfsim_atmo_config& c, int B) {
 
 template <class Real>
 int check_smem(const BuildDims& d) {
-  if (point_scatter_smem<Real>(d, true) > kMaxSmem)
+  if (point_scatter_capacity<Real>(d) > kMaxSmem)
     return fail(SFSIM_ATMO_ESHAPE, "elevation x heading slab of point scatter exceeds shared memory");
   if (ray_scatter_smem<Real>(d) > kMaxSmem)
     return fail(SFSIM_ATMO_ESHAPE, "sun elevation x heading plane of ray scatter exceeds shared memory");
@@ -381,7 +380,6 @@ struct Work {
   Vec4<Real>*T, *E0, *dE[2], *Eacc[2];
   Vec4<Real>*S1R, *M, *dS[2], *Sacc[2];
   Real* J;
-  Real* hrows;  // point scatter's heading rows per (height, sun elevation)
   float *oT, *oE, *oS, *oM;  // device outputs when the caller passes host buffers
   unsigned char* sun;        // sun-ray optical-depth tables, kSunTableBytes per atmosphere (FP32 builds), or NULL
 };
@@ -407,10 +405,9 @@ size_t carve(Work<Real>& w, char* base, const BuildDims& d, bool outputs, bool s
   w.setup.rowinfo = c.take<RowInfo>(B * d.rows());
   w.setup.rowmap = c.take<Remap2<Real>>(B * d.rows());
   w.setup.rows = c.take<RowSample<Real>>(B * d.rows() * d.S);
-  w.setup.sdirs = c.take<SphereDir<Real>>(B * d.n0 * (long long)(d.P + 1));
-  w.setup.pdirs = c.take<SphereDir<Real>>(B * d.n0 * (long long)dir_row(d.P));
-  w.setup.dimage = c.take<unsigned char>(B * d.n0 * dir_image_stride(d, sizeof(Real)));
-  w.setup.pcount = c.take<int2>(B * d.n0);
+  w.setup.rings = c.take<SphereRing<Real>>(B * d.n0 * (long long)(d.T + 1));
+  w.setup.dirs4 = c.take<Real>(4LL * (d.P + 1));
+  w.setup.offsets = c.take<Real>(sizeof(Real) == 8 ? B * d.n0 * (long long)d.P : 0);
   w.setup.prow = c.take<PointRow<Real>>(B * d.n0 * d.n2);
   w.setup.hdvs = c.take<double>(d.n3);
   w.setup.erow = c.take<SurfRow<Real>>(B * d.nE());
@@ -424,7 +421,6 @@ size_t carve(Work<Real>& w, char* base, const BuildDims& d, bool outputs, bool s
   w.S1R = c.take<Vec4<Real>>(B * d.n4());
   w.M = c.take<Vec4<Real>>(B * d.n4());
   w.J = c.take<Real>(3 * B * d.n4());  // planar [atmosphere][channel][node]
-  w.hrows = c.take<Real>(B * d.n0 * d.n2 * heading_rows_stride(d));
   for (int i = 0; i < 2; i++) {
     w.dS[i] = c.take<Vec4<Real>>(B * d.n4());
     w.Sacc[i] = c.take<Vec4<Real>>(B * d.n4());
@@ -670,11 +666,10 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
     tm.mark_end(ss);
     if (fork) CUDA_TRY(cudaEventRecord(g_side_sr[tm.dev], ss));
     tm.mark_begin(5);
-    if (launch_point_scatter<Real>(w.params, d, w.setup.rowinfo, w.setup.pdirs, w.setup.dimage, w.setup.pcount,
-                                   w.setup.prow,
-                                   w.setup.geom, dS_prev, M_first, dE_prev, w.hrows, w.J, st))
+    if (launch_point_scatter<Real>(w.params, d, w.setup.rowinfo, w.setup.rings, w.setup.dirs4, w.setup.offsets,
+                                   w.setup.prow, w.setup.geom, dS_prev, M_first, dE_prev, w.J, st))
       return fail(SFSIM_ATMO_ECUDA, "point scatter launch configuration failed");
-    launches += 2;
+    launches++;
     tm.mark_end();
     if (jsum) {
       launch_add_to_sum<Real>(d.n4(), d.B, w.J, jsum, it == 0, st);
@@ -874,9 +869,12 @@ int census_impl(const sfsim_atmo_config& cfg, unsigned long long* out, int n) {
   sphere_directions(cfg.sphere_steps >> 1, cfg.sphere_steps, M_PI, dirs);
   Work<Real> w;
   size_t bytes = carve<Real>(w, nullptr, d, false, false);
-  if ((rc = ensure_arena(dev, bytes + 256))) return rc;
+  const size_t sdirs_at = (bytes + 255) & ~size_t(255), nsd = (size_t)d.n0 * (d.P + 1);
+  const size_t count_at = (sdirs_at + sizeof(SphereDir<Real>) * nsd + 255) & ~size_t(255);
+  if ((rc = ensure_arena(dev, count_at + 256))) return rc;
   carve<Real>(w, (char*)g_arena[dev].base, d, false, false);
-  unsigned long long* dcount = reinterpret_cast<unsigned long long*>((char*)g_arena[dev].base + bytes);
+  SphereDir<Real>* dsd = reinterpret_cast<SphereDir<Real>*>((char*)g_arena[dev].base + sdirs_at);
+  unsigned long long* dcount = reinterpret_cast<unsigned long long*>((char*)g_arena[dev].base + count_at);
   cudaStream_t st = g_stream[dev];
   CUDA_TRY(cudaMemcpyAsync(w.params, &hp, sizeof(AtmoParams), cudaMemcpyHostToDevice, st));
   if (!dirs.empty()) {
@@ -884,6 +882,7 @@ int census_impl(const sfsim_atmo_config& cfg, unsigned long long* out, int n) {
   }
   CUDA_TRY(cudaMemsetAsync(dcount, 0, 2 * sizeof(unsigned long long), st));
   launch_setup<Real>(w.params, d, w.dirs, w.hdirs, w.setup, st);
+  launch_sphere_dirs<Real>(w.params, d, w.dirs, dsd, st);
   launch_first_order_census<Real>(w.params, d, w.setup.rowinfo, w.setup.rows, w.setup.geom, dcount, st);
   CUDA_TRY(cudaGetLastError());
   unsigned long long cnt[2] = {0, 0};
@@ -891,8 +890,8 @@ int census_impl(const sfsim_atmo_config& cfg, unsigned long long* out, int n) {
   CUDA_TRY(cudaStreamSynchronize(st));
   const unsigned long long lit = cnt[0], climb = cnt[1];
   // ground directions of the point-scatter sphere per height
-  std::vector<SphereDir<Real>> sd((size_t)d.n0 * (d.P + 1));
-  CUDA_TRY(cudaMemcpy(sd.data(), w.setup.sdirs, sizeof(SphereDir<Real>) * sd.size(), cudaMemcpyDeviceToHost));
+  std::vector<SphereDir<Real>> sd(nsd);
+  CUDA_TRY(cudaMemcpy(sd.data(), dsd, sizeof(SphereDir<Real>) * sd.size(), cudaMemcpyDeviceToHost));
   unsigned long long ground = 0, flat = 0;
   for (int i = 0; i < d.n0; i++)
     for (int k = 0; k < d.P; k++) {
@@ -1572,6 +1571,22 @@ int static_scratch_base(int dev, void** base) {
   return 0;
 }
 
+// What the static array's limit counts beside the scratch tables: the row
+// tables and direction lists per (height, sun elevation) pair that point
+// scatter no longer keeps.  They stay in the count so that the configurations
+// the entry point accepts stay the same.
+template <class Real>
+size_t static_margin(const BuildDims& d) {
+  auto up = [](long long x) { return (size_t)((x + 255) & ~255LL); };
+  const long long n = d.P + 16, n8 = (n + 7) / 8 * 8, R = sizeof(Real);
+  const size_t lists = up(sizeof(SphereDir<Real>) * d.n0 * (d.P + 1LL)) + up(sizeof(SphereDir<Real>) * d.n0 * n) +
+                       up(d.n0 * ((n8 * (9 * R + 4) + 15) & ~15LL)) + up(sizeof(int2) * d.n0);
+  const size_t rows = up(R * d.n0 * d.n2 * 2 * n8 * (d.n3 + 2) * 3);
+  const size_t kept = up(sizeof(SphereRing<Real>) * d.n0 * (d.T + 1LL)) + up(R * 4 * (d.P + 1LL)) +
+                      up(R == 8 ? R * d.n0 * d.P : 0);
+  return lists + rows > kept ? lists + rows - kept : 0;
+}
+
 template <class Real>
 int build_static_impl(const sfsim_atmo_config& cfg, float* T, float* E, float* S, float* M, cudaStream_t st) {
   int dev = 0;
@@ -1581,8 +1596,9 @@ int build_static_impl(const sfsim_atmo_config& cfg, float* T, float* E, float* S
   if ((rc = check_smem<Real>(d))) return rc;
   Work<Real> w;
   const size_t bytes = carve<Real>(w, nullptr, d, false, false);
-  if (bytes > kStaticScratchBytes)
-    return fail(SFSIM_ATMO_ETOOBIG, "the build needs " + std::to_string(bytes) +
+  const size_t counted = bytes + static_margin<Real>(d);
+  if (counted > kStaticScratchBytes)
+    return fail(SFSIM_ATMO_ETOOBIG, "the build needs " + std::to_string(counted) +
                                         " bytes of scratch, more than the 67108864-byte static array");
   AtmoParams hp;
   if ((rc = make_params(cfg, hp))) return rc;

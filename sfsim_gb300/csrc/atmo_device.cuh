@@ -637,6 +637,29 @@ __device__ inline void segment_depth(const AtmoParams& P, d3 x, d3 D, int steps,
   segment_depth_q<Real>(P, c0, dot3(x, D), dot3(D, D), mag3(D), steps, tau);
 }
 
+// segment_depth with the samples over a warp's lanes (every lane gets the sum).
+template <class Real>
+__device__ inline void segment_depth_warp(const AtmoParams& P, d3 x, d3 D, int steps, int lane, Real tau[3]) {
+  const double c0 = (mag3(x) - P.R) * (mag3(x) + P.R), du = 1.0 / steps, L = mag3(D);
+  const QForm f = segment_q_form(c0, dot3(x, D), dot3(D, D), du);
+  Real sr = 0, cr = 0, sm = 0, cm = 0;
+  for (int n = lane; n < steps; n += 32) {
+    const Real w = fma(Real(n), (Real)du, (Real)f.w0);
+    const Real q = fma(w, fma(w, (Real)f.C, (Real)f.B), (Real)f.A);
+    const Real h = height_from_q<Real, 5>(q, Bulk<Real>::hpoly(P), Bulk<Real>::alpha(P), Bulk<Real>::beta(P));
+    kahan_add(sr, cr, Bulk<Real>::exp2(h * Bulk<Real>::kr(P)));
+    kahan_add(sm, cm, Bulk<Real>::exp2(h * Bulk<Real>::km(P)));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sr += __shfl_xor_sync(0xffffffffu, sr, o);
+    sm += __shfl_xor_sync(0xffffffffu, sm, o);
+  }
+  const Real a = L > 0.0 ? (Real)(L / steps) : Real(0);
+#pragma unroll
+  for (int ch = 0; ch < 3; ch++) tau[ch] = a * (Bulk<Real>::ray_ext(P, ch) * sr + Bulk<Real>::mie_ext(P, ch) * sm);
+}
+
 template <class Real>
 __device__ __forceinline__ Real exp_neg(Real tau) {
   return Bulk<Real>::exp2(tau * Real(-1.4426950408889634));

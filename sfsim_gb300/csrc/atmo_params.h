@@ -70,6 +70,7 @@ struct BuildDims {
   int S;                   // ray steps
   int sphere_steps;        // point-scatter sphere steps
   int P;                   // directions of integral-sphere(sphere_steps)
+  int T;                   // their rings
   int Ph;                  // directions of integral-half-sphere(ray_steps)
   int iterations;
   double inv_S;            // 1 / S, the view rays' step in their parameter
@@ -147,6 +148,7 @@ template <class Real>
 struct PointRow {
   double ss;  // sin of the sun elevation of index k (index-to-sin-sun-elevation)
   double cs;  // sqrt(max(0, 1 - ss^2)), the bound of index-to-sun-direction's second component
+  Real lz;    // third component of the light direction where the second is at that bound
   int u0, u2;
   Real s0, s2;
   Real bR[3], bM[3];
@@ -186,7 +188,23 @@ struct RowSample {
   Real pad;
 };
 
-// Per height row i and sphere direction of point scatter.
+// Per height row i and ring of point scatter's sphere quadrature: what the
+// ring's directions share (x is on the first axis, so they differ in their
+// azimuth about it alone).
+template <class Real>
+struct alignas(16) SphereRing {
+  Real x0;             // first component of the directions omega
+  Real weight;         // quadrature weight (ring factor * 2 pi / ring steps)
+  Real tR;             // ground distance / R (rings ending on the ground): the ground point's sin of the
+                       // sun elevation is gA + tR (omega . l), gA of the (height, sun elevation) row
+  Real s1;             // elevation coordinate of (x, omega, !surface): fraction
+  Real ground[3];      // T(x, g) * brightness / pi (rings ending on the ground)
+  int u1;              // and lower index
+  int surface;         // 1: the ring's rays end on the ground
+  int w0, n;           // its directions: w0 .. w0 + n - 1
+};
+
+// Per height row i and sphere direction, for the work census.
 template <class Real>
 struct SphereDir {
   Real w[3];           // direction omega in world coordinates

@@ -1,0 +1,491 @@
+// k_point_scatter.cu -- point scatter J of the multiple-scattering iterations
+// (atmosphere.clj:203-222), for the nodes of one (height i, sun elevation k)
+// pair at a time.
+//
+// The sphere quadrature (sphere.clj:62-93) is a set of rings about x, which
+// lies on the first axis.  All directions of a ring share everything but
+// their azimuth: where they end, the ground's transmittance, and the height,
+// elevation and sun-elevation coordinates of the dS lookup (x.l = r sin(k) for
+// every node of the pair).  So dS collapses to one row along the sun-angle
+// axis per ring, and a direction's lookup is linear in that row at its own
+// omega.l.  The ground term is a linear lookup in the lowest row of the
+// surface-radiance table (a ray that ends on the ground ends at height 0).
+//
+// One thread holds one elevation j and kHP pairs of headings; the two FP32
+// lanes of every packed operation are two headings.  It walks the
+// directions ring by ring, forms the direction's two phase weights (they
+// depend on j and the direction only) once, and adds the interpolated rows of
+// all its headings.  The first and last headings ask for v.l = -1 and 1, which
+// clamps the light to the plane of x and v for every view
+// (index-to-sun-direction, atmosphere.clj:375-384): their l is the same for
+// all j, so the block interpolates their rows once per direction into shared
+// memory and every thread adds them from there.
+//
+// What bounds it: shared-memory wavefronts, six 4-byte gathers (three
+// channels, value and step to the next texel) per heading and direction and
+// six more on the ground.  Production tables (32x255x32x8, 336 directions, 5
+// iterations): 160M wavefronts a launch, 0.51 ms at one per clock and SM;
+// measured 0.63 ms, 3.49 ms for the build's five launches.  With a row per
+// direction instead of per ring (gathered to HBM by a kernel of its own), the
+// phases exchanged by shuffles and every heading walked, it was 7.08 ms; the
+// 16 atmospheres of a sweep (16x128x16x8) went from 11.8 to 5.5 ms, the
+// reference's tables (32x127x32x8, 71 directions) from 0.96 to 0.50 ms.
+#include <type_traits>
+
+#include "atmo_device.cuh"
+#include "kernels.h"
+
+namespace sfsim {
+
+// floor(c) of both lanes for |c| < 2^22: adding 1.5 2^23 rounding down leaves
+// floor(c) in the low bits, without the conversions of floor() and (int).
+constexpr float kFloorMagic = 12582912.0f;
+constexpr unsigned kFloorBits = 0x4B400000u;  // the bits of kFloorMagic
+
+// Lookups along a table of records of `stride` bytes: the byte offsets of
+// both lanes' records (from the start of shared memory) and their fractions.
+// For float the table's offset is lowered by stride * kFloorBits once
+// (lookup_base), so that a record's offset is one multiply-add of the sum's
+// bits.
+template <class Real>
+__device__ __forceinline__ unsigned lookup_base(unsigned origin, unsigned stride) {
+  return std::is_same<Real, float>::value ? origin - stride * kFloorBits : origin;
+}
+__device__ __forceinline__ float2 lookup(float2 c, unsigned base, unsigned stride, unsigned& oa, unsigned& ob) {
+  const float2 t = __fadd2_rd(c, make_float2(kFloorMagic, kFloorMagic));
+  oa = __float_as_uint(t.x) * stride + base;
+  ob = __float_as_uint(t.y) * stride + base;
+  return sub2(c, __fadd2_rn(t, make_float2(-kFloorMagic, -kFloorMagic)));
+}
+__device__ __forceinline__ double2 lookup(double2 c, unsigned base, unsigned stride, unsigned& oa, unsigned& ob) {
+  const double fa = floor(c.x), fb = floor(c.y);
+  oa = (unsigned)(int)fa * stride + base;
+  ob = (unsigned)(int)fb * stride + base;
+  return make_double2(c.x - fa, c.y - fb);
+}
+
+// Two 16-byte-aligned pairs in one load (two for double).
+__device__ __forceinline__ void ld_pairs(const float* p, float2& a, float2& b) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  a = make_float2(v.x, v.y);
+  b = make_float2(v.z, v.w);
+}
+__device__ __forceinline__ void ld_pairs(const double* p, double2& a, double2& b) {
+  a = reinterpret_cast<const double2*>(p)[0];
+  b = reinterpret_cast<const double2*>(p)[1];
+}
+
+template <class Real>
+__device__ __forceinline__ V2<Real> dup(Real a) {
+  return mk2(a, a);
+}
+
+// Values per record of a ring row: three channels' (value, step to the next
+// texel), in the first iteration those of the Mie strength too; an odd
+// stride spreads the texels over the banks.
+template <bool FIRST>
+__host__ __device__ constexpr int row_stride() {
+  return FIRST ? 13 : 7;
+}
+
+// Records of a ring row: a copy of texel 0, then the n3 texels, so that a
+// coordinate that rounding pushed just below 0 reads texel 0; the last
+// texel's step is 0.
+__host__ __device__ constexpr int row_records(int n3) { return n3 + 1; }
+
+// Shared-memory layout, in this order, each part 16-byte aligned.
+struct PointLayout {
+  unsigned dirs;    // [P][4] x1, x1, x2, x2
+  unsigned edge;    // [P][8] three channels at the first and last heading's l, in pairs
+  unsigned rings;   // [T] SphereRing
+  unsigned rows;    // [T][n3 + 1][row_stride]
+  unsigned etab;    // [nE1][estride]
+  unsigned bytes;
+  int estride;      // 7, or 6 where 7 would not fit
+};
+template <class Real>
+__host__ __device__ inline PointLayout point_layout(const BuildDims& d, bool first, int estride) {
+  auto up = [](size_t x) { return (x + 15) & ~size_t(15); };
+  PointLayout l;
+  size_t o = 0;
+  l.dirs = 0;
+  o = up(o + sizeof(Real) * 4 * d.P);
+  l.edge = (unsigned)o;
+  o = up(o + sizeof(Real) * 8 * d.P);
+  l.rings = (unsigned)o;
+  o = up(o + sizeof(SphereRing<Real>) * d.T);
+  l.rows = (unsigned)o;
+  o = up(o + sizeof(Real) * d.T * row_records(d.n3) * (first ? row_stride<true>() : row_stride<false>()));
+  l.etab = (unsigned)o;
+  o = up(o + sizeof(Real) * estride * d.nE1);
+  l.bytes = (unsigned)o;
+  l.estride = estride;
+  return l;
+}
+
+// dS (or the Mie strength) at texel a of a ring's row: height and sun
+// elevation of the pair, elevation of the ring; a corner whose weight is
+// exactly 0 is not loaded (mix3(x, y, 0) = x exactly).
+template <class Real>
+__device__ __forceinline__ void gather_row_texel(const Vec4<Real>* t, const BuildDims& d, int u0, Real s0, int u1,
+                                                 Real s1, int u2, Real s2, int a, Real* dst) {
+  const int v0 = upper_index(u0, d.n0), v1 = upper_index(u1, d.n1), v2 = upper_index(u2, d.n2);
+  auto pair = [&](int h, int e, Real* out) {  // mixed over the sun elevation
+    Real A[3], B[3];
+    ld3(t, idx4(d, h, e, u2, a), A);
+    if (s2 != Real(0)) {
+      ld3(t, idx4(d, h, e, v2, a), B);
+      mix3(A, B, s2, out);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; c++) out[c] = A[c];
+    }
+  };
+  auto row = [&](int e, Real* out) {  // mixed over the height
+    Real lo[3], hi[3];
+    pair(u0, e, lo);
+    if (s0 != Real(0)) {
+      pair(v0, e, hi);
+      mix3(lo, hi, s0, out);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; c++) out[c] = lo[c];
+    }
+  };
+  Real e0[3], e1[3];
+  row(u1, e0);
+  row(v1, e1);
+  mix3(e0, e1, s1, dst);
+}
+
+constexpr int kPointThreads = 128;
+
+// Blocks per SM the registers are limited for.  Three heading pairs measured
+// 3.49 / 3.57 / 3.70 ms of a production build (5 launches) at 3 / 4 / 5
+// blocks: the gathers, not the warps in flight, are the limit.
+template <class Real, int HP>
+constexpr int point_min_blocks() {
+  return sizeof(Real) == 8 ? 2 : HP == 3 ? 3 : HP == 2 ? 4 : 5;
+}
+
+template <class Real, int HP, bool FIRST>
+__global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
+    k_point_scatter(const AtmoParams* params, BuildDims d, PointLayout lay, const RowInfo* rowinfo,
+                    const SphereRing<Real>* rings, const Real* dirs4, const Real* offsets,
+                    const PointRow<Real>* prow, const CellGeom<Real>* geom, const Vec4<Real>* dS, const Vec4<Real>* Mt, const Vec4<Real>* dE,
+                    Real* J, int groups, int chunks) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  using R2 = V2<Real>;
+  constexpr int KS = row_stride<FIRST>();
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int b = blockIdx.y;
+  const int ik = blockIdx.x / chunks, chunk = blockIdx.x - ik * chunks;
+  const int i = ik / d.n2, k = ik - i * d.n2;
+  const AtmoParams& P = params[b];
+  const PointRow<Real> pk = prow[((long long)b * d.n0 + i) * d.n2 + k];
+  Real* sdirs = reinterpret_cast<Real*>(smem_raw + lay.dirs);
+  Real* sedge = reinterpret_cast<Real*>(smem_raw + lay.edge);
+  SphereRing<Real>* sring = reinterpret_cast<SphereRing<Real>*>(smem_raw + lay.rings);
+  Real* srows = reinterpret_cast<Real*>(smem_raw + lay.rows);
+  Real* setab = reinterpret_cast<Real*>(smem_raw + lay.etab);
+  const unsigned es = (unsigned)lay.estride;
+  const int nrec = row_records(d.n3);
+  const long long base4 = (long long)b * d.n4();
+
+  // ring records, directions, the rows' texels and the dE row
+  {
+    const SphereRing<Real>* src = rings + ((long long)b * d.n0 + i) * d.T;
+    for (int t = tid; t < (int)(sizeof(SphereRing<Real>) / 16) * d.T; t += nt)
+      reinterpret_cast<int4*>(sring)[t] = reinterpret_cast<const int4*>(src)[t];
+    for (int t = tid; t < (int)(sizeof(Real) * 4 / 16) * d.P; t += nt)
+      reinterpret_cast<int4*>(sdirs)[t] = reinterpret_cast<const int4*>(dirs4)[t];
+    for (int t = tid; t < d.T * d.n3; t += nt) {
+      const int r = t / d.n3, a = t - r * d.n3;
+      const int u1 = src[r].u1;
+      const Real s1 = src[r].s1;
+      Real v[3], vm[3];
+      gather_row_texel(dS + base4, d, pk.u0, pk.s0, u1, s1, pk.u2, pk.s2, a, v);
+      if (FIRST) gather_row_texel(Mt + base4, d, pk.u0, pk.s0, u1, s1, pk.u2, pk.s2, a, vm);
+      Real* o = srows + (r * nrec + a + 1) * KS;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        o[2 * c] = v[c];
+        if (FIRST) o[6 + 2 * c] = vm[c];
+        if (a == 0) {
+          o[2 * c - KS] = v[c];
+          o[2 * c + 1 - KS] = Real(0);
+          if (FIRST) {
+            o[6 + 2 * c - KS] = vm[c];
+            o[6 + 2 * c + 1 - KS] = Real(0);
+          }
+        }
+      }
+    }
+    const Vec4<Real>* e = dE + b * d.nE();
+    for (int t = tid; t < d.nE1; t += nt) {
+      Real A[3], B[3];
+      ld3(e, t, A);
+      ld3(e, upper_index(t, d.nE1), B);
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        setab[t * es + 2 * c] = A[c];
+        setab[t * es + 2 * c + 1] = B[c] - A[c];
+      }
+    }
+  }
+  __syncthreads();
+  for (int t = tid; t < d.T * d.n3; t += nt) {
+    const int r = t / d.n3, a = t - r * d.n3;
+    Real* o = srows + (r * nrec + a + 1) * KS;
+    constexpr int nc = FIRST ? 6 : 3;
+#pragma unroll
+    for (int c = 0; c < nc; c++) o[2 * c + 1] = a < d.n3 - 1 ? o[KS + 2 * c] - o[2 * c] : Real(0);
+  }
+  __syncthreads();
+
+  const PhaseCS<Real> phR(Bulk<Real>::phase_ray(P)), phM(Bulk<Real>::phase_mie(P));
+  const Real scale3 = Real(0.5) * Real(d.n3 - 1);
+  const Real scaleE = Bulk<Real>::sun_scale_E(d);
+  const unsigned kstride = KS * sizeof(Real), estride = es * sizeof(Real);
+  const unsigned ebase = lookup_base<Real>(lay.etab, estride);
+  const Real log2e = Real(1.4426950408889634);
+  const Real zA = -log2e * fma(Real(3), pk.gA, Real(0.6));
+  const Real lx = (Real)pk.ss;
+  // the light reaching x from direction (x0, x1, x2) of a ring, for the two
+  // light directions (lx, ly, lz) of a pair: dS along the ring's row and, for
+  // rings that end on the ground, the ground's radiance
+  auto incoming = [&](auto ground, const SphereRing<Real>& rc, unsigned rbase, R2 c0, R2 x1, R2 x2, R2 ly, R2 lz,
+                      Real off, R2 (&X)[3]) {
+    const R2 mu = fma2(x1, ly, fma2(x2, lz, c0));  // omega . l
+    // the sun-angle coordinate; |mu| <= 1 up to rounding, so its floor lies in
+    // [-1, n3 - 1], whose records give the clamped interpolation
+    unsigned oa, ob;
+    const R2 s = lookup(fma2(dup(scale3), mu, dup(scale3)), rbase, kstride, oa, ob);
+    const Real* ra = reinterpret_cast<const Real*>(smem_raw + oa);
+    const Real* rb = reinterpret_cast<const Real*>(smem_raw + ob);
+#pragma unroll
+    for (int c = 0; c < 3; c++) X[c] = fma2(mk2(ra[2 * c + 1], rb[2 * c + 1]), s, mk2(ra[2 * c], rb[2 * c]));
+    if (FIRST) {
+      const R2 ph = phM.pair(mu);
+#pragma unroll
+      for (int c = 3; c < 6; c++)
+        X[c - 3] = fma2(fma2(mk2(ra[2 * c + 1], rb[2 * c + 1]), s, mk2(ra[2 * c], rb[2 * c])), ph, X[c - 3]);
+    }
+    if (decltype(ground)::value) {
+      // the ground point's sin of the sun elevation, g.l / |g| = gA + tR (omega . l)
+      // and its coordinate (1 - exp(-3 sin - 0.6)) / (1 - exp(-3.6)) (nE1 - 1),
+      // at least 0; the sine is at most 1 (k_sphere_rings keeps tR finite)
+      const R2 z = fma2(dup(Real(-3) * log2e * rc.tR), mu, dup(zA));
+      const R2 ex = mk2(Bulk<Real>::exp2(z.x), Bulk<Real>::exp2(z.y));
+      R2 ie = fma2(dup(-scaleE), ex, dup(scaleE));
+      ie = mk2(fmax(ie.x, Real(0)), fmax(ie.y, Real(0)));
+      const R2 se = lookup(ie, ebase, estride, oa, ob);
+      const Real* ea = reinterpret_cast<const Real*>(smem_raw + oa);
+      const Real* eb = reinterpret_cast<const Real*>(smem_raw + ob);
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const R2 y = fma2(mk2(ea[2 * c + 1], eb[2 * c + 1]), se, mk2(ea[2 * c], eb[2 * c]));
+        X[c] = fma2(dup(rc.ground[c]), y, X[c]);
+      }
+      if constexpr (std::is_same<Real, double>::value) {
+        // the FP64 build's ground point is off height 0 by its rounding, as
+        // the reference's is: the next height's row has that weight
+        if (off != 0.0) {
+          const Vec4<double>* e0 = dE + b * d.nE();
+          const Vec4<double>* e1 = e0 + d.nE1;
+          const int ia = (int)ie.x, ib = (int)ie.y;
+          double A[3], B[3], C[3], D[3];
+          auto above = [&](int u, double s, double (&o)[3]) {  // row 1 less row 0
+            const int v = upper_index(u, d.nE1);
+            ld3(e1, u, A), ld3(e1, v, B), ld3(e0, u, C), ld3(e0, v, D);
+#pragma unroll
+            for (int c = 0; c < 3; c++) o[c] = (A[c] - C[c]) * (1.0 - s) + (B[c] - D[c]) * s;
+          };
+          double ya[3], yb[3];
+          above(ia, se.x, ya);
+          above(ib, se.y, yb);
+#pragma unroll
+          for (int c = 0; c < 3; c++) X[c] = fma2(dup(rc.ground[c] * off), mk2(ya[c], yb[c]), X[c]);
+        }
+      }
+    }
+  };
+  // the height coordinate of direction w's ground point (FP64 builds; 0 but for rounding)
+  auto offset = [&](int w) -> Real {
+    if constexpr (std::is_same<Real, double>::value)
+      return offsets[((long long)b * d.n0 + i) * d.P + w];
+    else
+      return 0;
+  };
+  auto ring_base = [&](int r) { return lookup_base<Real>(lay.rows + (unsigned)(r * nrec + 1) * kstride, kstride); };
+
+  // the first and last headings' rows at every direction
+  {
+    const R2 ly = mk2((Real)-pk.cs, (Real)pk.cs), lz = dup(pk.lz);
+    for (int r = 0; r < d.T; r++) {
+      const SphereRing<Real>& rc = sring[r];
+      const unsigned rbase = ring_base(r);
+      for (int m = tid; m < rc.n; m += nt) {
+        const Real* x = sdirs + 4 * (rc.w0 + m);
+        R2 X[3];
+        if (rc.surface)
+          incoming(std::true_type{}, rc, rbase, dup(rc.x0 * lx), dup(x[0]), dup(x[2]), ly, lz, offset(rc.w0 + m), X);
+        else
+          incoming(std::false_type{}, rc, rbase, dup(rc.x0 * lx), dup(x[0]), dup(x[2]), ly, lz, offset(rc.w0 + m), X);
+        R2* o = reinterpret_cast<R2*>(sedge + 8 * (rc.w0 + m));
+#pragma unroll
+        for (int c = 0; c < 3; c++) o[c] = X[c];
+      }
+    }
+  }
+  __syncthreads();
+
+  // this thread's elevation and headings; a thread past the last item repeats it and stores nothing
+  const int items = d.n1 * groups;
+  const int item_raw = chunk * nt + tid;
+  const bool valid = item_raw < items;
+  const int item = valid ? item_raw : items - 1;
+  const int grp = item / d.n1, j = item - grp * d.n1;
+  const int a0 = 1 + grp * 2 * HP;  // its headings a0 .. a0 + 2 HP - 1, those below n3 - 1
+  const long long node0 = base4 + idx4(d, i, j, k, 0);
+  Real sv, cv;
+  {
+    const RowR<Real> rw = row_r<Real>(rowinfo[(long long)b * d.rows() + (long long)i * d.n1 + j]);
+    sv = rw.sv, cv = rw.cv;
+  }
+  R2 ly[HP], lz[HP];
+#pragma unroll
+  for (int h = 0; h < HP; h++) {
+    const CellGeom<Real> ga = geom[node0 + min(a0 + 2 * h, d.n3 - 1)];
+    const CellGeom<Real> gb = geom[node0 + min(a0 + 2 * h + 1, d.n3 - 1)];
+    ly[h] = mk2(ga.ly, gb.ly);
+    lz[h] = mk2(ga.lz, gb.lz);
+  }
+  // sums over the directions so far, and over the ring being walked (pair HP: the first and last heading)
+  R2 tot[HP + 1][3];
+#pragma unroll
+  for (int h = 0; h <= HP; h++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) tot[h][c] = dup(Real(0));
+
+  for (int r = 0; r < d.T; r++) {
+    const SphereRing<Real>& rc = sring[r];
+    const unsigned rbase = ring_base(r);
+    const R2 c0 = dup(rc.x0 * lx);
+    const Real mv0 = sv * rc.x0;
+    const int n = rc.n;
+    const Real* x = sdirs + 4 * rc.w0;
+    const Real* e = sedge + 8 * rc.w0;
+    // beta_c(x) (atmosphere.clj:42-47, 140-151) times the ring's weight
+    Real bR[3], bM[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) bR[c] = rc.weight * pk.bR[c], bM[c] = rc.weight * pk.bM[c];
+    R2 sum[HP + 1][3];
+#pragma unroll
+    for (int h = 0; h <= HP; h++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) sum[h][c] = dup(Real(0));
+    auto walk = [&](auto ground) {
+      for (int m = 0; m < n; m++, x += 4, e += 8) {
+        R2 x1, x2;
+        ld_pairs(x, x1, x2);
+        const Real mv = fma(cv, x1.x, mv0);
+        const Real fR = phR(mv), fM = phM(mv);
+        R2 w[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) w[c] = dup(fma(bM[c], fM, bR[c] * fR));
+#pragma unroll
+        for (int h = 0; h < HP; h++) {
+          R2 X[3];
+          incoming(ground, rc, rbase, c0, x1, x2, ly[h], lz[h], offset(rc.w0 + m), X);
+#pragma unroll
+          for (int c = 0; c < 3; c++) sum[h][c] = fma2(w[c], X[c], sum[h][c]);
+        }
+        R2 X[3];
+        ld_pairs(e, X[0], X[1]);
+        X[2] = *reinterpret_cast<const R2*>(e + 4);
+#pragma unroll
+        for (int c = 0; c < 3; c++) sum[HP][c] = fma2(w[c], X[c], sum[HP][c]);
+      }
+    };
+    if (rc.surface)
+      walk(std::true_type{});
+    else
+      walk(std::false_type{});
+#pragma unroll
+    for (int h = 0; h <= HP; h++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) tot[h][c] = add2(tot[h][c], sum[h][c]);
+  }
+  if (!valid) return;
+  // J planar, [atmosphere][channel][node], for the ray-scatter gathers
+  const long long n4 = d.n4();
+  Real* Jn = J + (long long)b * 3 * n4 + (node0 - base4);
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    Real* o = Jn + c * n4;
+#pragma unroll
+    for (int h = 0; h < HP; h++) {
+      const int a = a0 + 2 * h;
+      if (a < d.n3 - 1) o[a] = tot[h][c].x;
+      if (a + 1 < d.n3 - 1) o[a + 1] = tot[h][c].y;
+    }
+    if (grp == 0) {
+      o[0] = tot[HP][c].x;
+      o[d.n3 - 1] = tot[HP][c].y;
+    }
+  }
+}
+
+// 40 bytes a direction (FP32; 76 in FP64), two rows of n3 + 2 RGB texels
+// each, and the surface-radiance table, with room for 16 directions more.
+// The tables above are smaller (a row per ring, not per direction), so a
+// configuration within this limit always fits.
+template <class Real>
+size_t point_scatter_capacity(const BuildDims& d) {
+  const size_t n = (size_t)d.P + 16;
+  return ((n * (9 * sizeof(Real) + sizeof(int)) + 15) & ~size_t(15)) +
+         sizeof(Real) * 3 * (n * (d.n3 + 2) * 2 + d.nE());
+}
+template size_t point_scatter_capacity<float>(const BuildDims&);
+template size_t point_scatter_capacity<double>(const BuildDims&);
+
+template <class Real>
+int launch_point_scatter(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
+                         const SphereRing<Real>* rings, const Real* dirs4, const Real* offsets,
+                         const PointRow<Real>* prow, const CellGeom<Real>* geom, const Vec4<Real>* dS, const Vec4<Real>* mie, const Vec4<Real>* dE,
+                         Real* J, cudaStream_t st) {
+  const bool first = mie != nullptr;
+  PointLayout lay = point_layout<Real>(d, first, 7);
+  if (lay.bytes > 227 * 1024) lay = point_layout<Real>(d, first, 6);
+  const int inner = d.n3 - 2;
+  int hp = sizeof(Real) == 8 ? 1 : inner > 4 ? 3 : inner > 2 ? 2 : 1;
+  const int groups = inner > 0 ? (inner + 2 * hp - 1) / (2 * hp) : 1;
+  const int items = d.n1 * groups;
+  const int chunks = (items + kPointThreads - 1) / kPointThreads;
+  const int block = ((items + chunks - 1) / chunks + 31) / 32 * 32;
+  const dim3 grid((unsigned)(d.n0 * d.n2 * chunks), d.B);
+  auto go = [&](auto kernel) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.bytes) != cudaSuccess)
+      return -1;
+    kernel<<<grid, block, lay.bytes, st>>>(params, d, lay, rowinfo, rings, dirs4, offsets, prow, geom, dS, mie,
+                                           dE, J, groups, chunks);
+    return 0;
+  };
+  if constexpr (std::is_same<Real, float>::value) {
+    if (hp == 3) return first ? go(k_point_scatter<Real, 3, true>) : go(k_point_scatter<Real, 3, false>);
+    if (hp == 2) return first ? go(k_point_scatter<Real, 2, true>) : go(k_point_scatter<Real, 2, false>);
+  }
+  return first ? go(k_point_scatter<Real, 1, true>) : go(k_point_scatter<Real, 1, false>);
+}
+
+template int launch_point_scatter<float>(const AtmoParams*, const BuildDims&, const RowInfo*, const SphereRing<float>*,
+                                         const float*, const float*, const PointRow<float>*, const CellGeom<float>*,
+                                         const Vec4<float>*, const Vec4<float>*, const Vec4<float>*, float*,
+                                         cudaStream_t);
+template int launch_point_scatter<double>(const AtmoParams*, const BuildDims&, const RowInfo*,
+                                          const SphereRing<double>*, const double*, const double*, const PointRow<double>*,
+                                          const CellGeom<double>*, const Vec4<double>*, const Vec4<double>*,
+                                          const Vec4<double>*, double*, cudaStream_t);
+
+}  // namespace sfsim

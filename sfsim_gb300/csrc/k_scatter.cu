@@ -1,6 +1,6 @@
 // k_scatter.cu -- multiple-scattering passes of the atmosphere LUT build
-// (atmosphere_lut.clj:86-97): point scatter J, surface radiance dE, ray
-// scatter dS, and the re-interpolating accumulation of E and S.
+// (atmosphere_lut.clj:86-97): surface radiance dE, ray scatter dS, and the
+// re-interpolating accumulation of E and S.
 #include <cstddef>
 #include <type_traits>
 
@@ -9,424 +9,9 @@
 
 namespace sfsim {
 
-// ---------------------------------------------------------------------------
-// Point scatter J (atmosphere.clj:203-222) for all nodes of one (height i,
-// sun elevation k) pair.  For such a pair every dS lookup shares the height
-// coordinate (x is fixed) and the sun-elevation coordinate (x.l/|x| is the
-// sin of the sun elevation), and a direction's elevation coordinate depends
-// on the direction alone.  So the block first gathers, per direction, dS
-// along the heading axis (8 corners per heading) into a row in shared
-// memory; a node then reads two texels of its direction's row at its own
-// sun-angle coordinate (omega.l).  The ground term reads the dE table, also
-// staged in shared memory.  One thread per node (elevation j, heading a);
-// directions, ground ends and T(x, ground) come from k_sphere_setup.
-// ---------------------------------------------------------------------------
-
-template <class Real>
-__device__ __forceinline__ void gather_heading_row(const Vec4<Real>* t, const BuildDims& d, int u0, int v0, Real s0,
-                                                   int u1, int v1, Real s1, int u2, int v2, Real s2, int a,
-                                                   Real* dst) {
-  // height and sun elevation first, then elevation; a corner whose weight
-  // is exactly 0 is not loaded (mix3(x, y, 0) = x exactly)
-  auto pair = [&](int h, int e, Real* out) {  // mixed over the sun elevation
-    Real A[3], B[3];
-    ld3(t, idx4(d, h, e, u2, a), A);
-    if (s2 != Real(0)) {
-      ld3(t, idx4(d, h, e, v2, a), B);
-      mix3(A, B, s2, out);
-    } else {
-#pragma unroll
-      for (int c = 0; c < 3; c++) out[c] = A[c];
-    }
-  };
-  auto row = [&](int e, Real* out) {  // mixed over the height
-    Real lo[3], hi[3];
-    pair(u0, e, lo);
-    if (s0 != Real(0)) {
-      pair(v0, e, hi);
-      mix3(lo, hi, s0, out);
-    } else {
-#pragma unroll
-      for (int c = 0; c < 3; c++) out[c] = lo[c];
-    }
-  };
-  Real e0[3], e1[3];
-  row(u1, e0);
-  row(v1, e1);
-  mix3(e0, e1, s1, dst);
-}
-
-// Shared-memory rows of RGB texels, three values per texel.  (16-byte texels
-// were measured slower: a warp's lanes read few distinct texels of a row,
-// which scalar loads serve as broadcasts in one wavefront each, while 16-byte
-// loads take four.)
-template <class Real>
-struct TexelRow {
-  static constexpr int kStride = 3;
-  static __device__ __forceinline__ void load(const Real* base, int idx, Real* out) {
-    out[0] = base[3 * idx];
-    out[1] = base[3 * idx + 1];
-    out[2] = base[3 * idx + 2];
-  }
-  static __device__ __forceinline__ void store(Real* base, int idx, const Real* v) {
-    base[3 * idx] = v[0];
-    base[3 * idx + 1] = v[1];
-    base[3 * idx + 2] = v[2];
-  }
-};
-
-// The heading rows of one (height i, sun elevation k) pair: for each of the
-// `used` partitioned directions, dS (and in the first iteration the Mie
-// strength) gathered along the heading axis at the pair's height and
-// sun-elevation coordinates and the direction's elevation coordinate, n3
-// texels between copies of the first and last (rows, then rowsM).
-template <class Real, bool FIRST>
-__device__ __forceinline__ void heading_rows(const BuildDims& d, const SphereDir<Real>* src, int used,
-                                             const Vec4<Real>* dS, const Vec4<Real>* Mt, const PointRow<Real>& pk,
-                                             Real* rows, int t0, int nt) {
-  using TR = TexelRow<Real>;
-  const int rlen = d.n3 + 2;
-  Real* rowsM = rows + TR::kStride * used * rlen;
-  const int u0 = pk.u0, u2 = pk.u2;
-  const Real s0 = pk.s0, s2 = pk.s2;
-  const int v0 = upper_index(u0, d.n0), v2 = upper_index(u2, d.n2);
-  for (int t = t0; t < used * d.n3; t += nt) {
-    const int w = t / d.n3, a = t - w * d.n3;
-    Real v[3] = {0, 0, 0}, vm[3] = {0, 0, 0};
-    if (!src[w].pad) {
-      const int u1 = src[w].u1, v1 = upper_index(u1, d.n1);
-      const Real s1 = src[w].s1;
-      gather_heading_row(dS, d, u0, v0, s0, u1, v1, s1, u2, v2, s2, a, v);
-      if (FIRST) gather_heading_row(Mt, d, u0, v0, s0, u1, v1, s1, u2, v2, s2, a, vm);
-    }
-    const int o = w * rlen + 1 + a;
-    TR::store(rows, o, v);
-    if (FIRST) TR::store(rowsM, o, vm);
-    if (a == 0) {
-      TR::store(rows, o - 1, v);
-      if (FIRST) TR::store(rowsM, o - 1, vm);
-    }
-    if (a == d.n3 - 1) {
-      TR::store(rows, o + 1, v);
-      if (FIRST) TR::store(rowsM, o + 1, vm);
-    }
-  }
-}
-
-// The rows of every (i, k) pair into the global row table, once per
-// iteration, so that the point-scatter blocks of a pair copy them instead
-// of each gathering them.
-template <class Real, bool FIRST>
-__global__ void __launch_bounds__(256) k_heading_rows(BuildDims d, const SphereDir<Real>* pdirs, const int2* pcount,
-                                                      const PointRow<Real>* prow, const Vec4<Real>* dS,
-                                                      const Vec4<Real>* Mt, Real* hrows) {
-  const int b = blockIdx.y;
-  const int i = blockIdx.x / d.n2, k = blockIdx.x % d.n2;
-  const long long pair = ((long long)b * d.n0 + i) * d.n2 + k;
-  const SphereDir<Real>* src = pdirs + ((long long)b * d.n0 + i) * dir_row(d.P);
-  const long long base4 = (long long)b * d.n4();
-  heading_rows<Real, FIRST>(d, src, pcount[(long long)b * d.n0 + i].y, dS + base4, FIRST ? Mt + base4 : nullptr,
-                            prow[pair], hrows + pair * heading_rows_stride(d), threadIdx.x, blockDim.x);
-}
-
-// Shared-memory layout of point scatter for one (height i, sun elevation k)
-// pair, `used` directions (a multiple of kDirBlock):
-//   dirs  [kDirFields][used] Real: x0, x1, x2, weight, tR, ground0..2, sE0
-//         of each direction (structure of arrays, so that two consecutive
-//         directions' components load as one pair);
-//   uE0   [used] int;
-//   rows  [used][n3 + 2][3] dS gathered along the heading axis between
-//         copies of its first and last texel (and the Mie rows in the first
-//         iteration);
-//   etab  [nE0][nE1][3] the dE table.
-
 template <class Real>
 __device__ __forceinline__ V2<Real> ld2(const Real* p) {
   return *reinterpret_cast<const V2<Real>*>(p);
-}
-
-static_assert(kDirBlock % 2 == 0, "direction pairs start at even indices (8-byte loads of pair fields)");
-
-// Blocks per (height, sun elevation) pair when each evaluates `cpb` of the
-// pair's `nchunks` chunks of 256 nodes; the launch and the kernel share it.
-__host__ __device__ __forceinline__ int point_scatter_blocks_per_pair(int nchunks, int cpb) {
-  return (nchunks + cpb - 1) / cpb;
-}
-
-// Three FP32 blocks of 256 share an SM (80 registers a thread); FP64 blocks
-// are register-bound anyway.
-constexpr int point_scatter_min_blocks(size_t real_size) { return real_size == 4 ? 3 : 1; }
-
-template <class Real, bool FIRST>
-__global__ void __launch_bounds__(256, point_scatter_min_blocks(sizeof(Real))) k_point_scatter(const AtmoParams* params, BuildDims d,
-                                                          const RowInfo* rowinfo, const SphereDir<Real>* pdirs,
-                                                          const unsigned char* dimage, const int2* pcount,
-                                                          const PointRow<Real>* prow,
-                                                          const CellGeom<Real>* geom,
-                                                          const Real* hrows, const Vec4<Real>* dE, Real* J,
-                                                          int nchunks, int chunks_per_block) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  using TR = TexelRow<Real>;
-  using R2 = V2<Real>;
-  constexpr int RS = TR::kStride;
-  constexpr int DB = kDirBlock;
-  const int b = blockIdx.y;
-  // one (height i, sun elevation k) pair, chunks_per_block chunks of 256 of
-  // its (elevation, heading) nodes: the rows are gathered once for them all
-  const int nblk = point_scatter_blocks_per_pair(nchunks, chunks_per_block);
-  const int chunk0 = (blockIdx.x % nblk) * chunks_per_block;
-  const int ik = blockIdx.x / nblk;
-  if (ik >= d.n0 * d.n2) return;  // the grid is n0 * n2 * nblk blocks; nothing beyond
-  const int i = ik / d.n2, k = ik % d.n2;
-  const AtmoParams& P = params[b];
-  const PointRow<Real>* prk = prow + ((long long)b * d.n0 + i) * d.n2 + k;
-  const int2 pc = pcount[(long long)b * d.n0 + i];
-  const int sky_end = pc.x, used = pc.y;
-  // texels of a heading row: a copy of texel 0, the n3 texels, a copy of
-  // texel n3 - 1, so that a sun-angle coordinate that rounding pushed just
-  // outside [0, n3 - 1] reads the edge texel without a clamp
-  const int rlen = d.n3 + 2;
-  Real* dirs = reinterpret_cast<Real*>(smem_raw);
-  int* uE0s = reinterpret_cast<int*>(dirs + kDirFields * used);
-  const size_t dir_bytes = dir_image_bytes(used, sizeof(Real));
-  Real* rows = reinterpret_cast<Real*>(smem_raw + dir_bytes);
-  Real* rowsM = rows + RS * used * rlen;
-  Real* etab = rowsM + (FIRST ? RS * used * rlen : 0);
-
-  const long long base4 = (long long)b * d.n4();
-  {
-    // the height's direction arrays, prepared by k_sphere_partition
-    const int4* ds = reinterpret_cast<const int4*>(dimage + ((long long)b * d.n0 + i) *
-                                                                dir_image_stride(d, sizeof(Real)));
-    int4* dd = reinterpret_cast<int4*>(smem_raw);
-    for (int t = threadIdx.x; t < (int)(dir_bytes / 16); t += blockDim.x) dd[t] = ds[t];
-  }
-  {
-    // the pair's heading rows from the row table (k_heading_rows), 16 bytes
-    // a thread at a time: a multiple of 24 values, both ends 16-byte aligned
-    const int4* hs = reinterpret_cast<const int4*>(hrows + (((long long)b * d.n0 + i) * d.n2 + k) *
-                                                                heading_rows_stride(d));
-    int4* hd = reinterpret_cast<int4*>(rows);
-    const int n16 = (int)((FIRST ? 2 : 1) * (size_t)RS * used * rlen * sizeof(Real) / 16);
-    for (int t = threadIdx.x; t < n16; t += blockDim.x) hd[t] = hs[t];
-  }
-  const long long nE = d.nE();
-  for (int t = threadIdx.x; t < nE; t += blockDim.x) {
-    Real A[3];
-    ld3(dE, b * nE + t, A);
-    TR::store(etab, t, A);
-  }
-  __syncthreads();
-
-  for (int chunk = chunk0; chunk < min(chunk0 + chunks_per_block, nchunks); chunk++) {
-    // a lane past the last node keeps running (it feeds the warp's shuffles) but stores nothing
-    const int nslab = d.n1 * d.n3;
-    const int cell_raw = chunk * blockDim.x + threadIdx.x;
-    const bool valid = cell_raw < nslab;
-    const int cell = valid ? cell_raw : nslab - 1;
-    const int j = cell / d.n3, a = cell % d.n3;
-    const RowR<Real> rw = row_r<Real>(rowinfo[(long long)b * d.rows() + (long long)i * d.n1 + j]);
-    const Real sv = rw.sv, cv = rw.cv;
-    const long long node = base4 + idx4(d, i, j, k, a);
-    const CellGeom<Real> g = geom[node];
-    const PhaseCS<Real> phR(Bulk<Real>::phase_ray(P)), phM(Bulk<Real>::phase_mie(P));
-    const Real scale3 = Real(0.5) * Real(d.n3 - 1);
-    const Real scaleE = Bulk<Real>::sun_scale_E(d);
-    // The weighted phases depend on (j, direction) only.  When the n3 headings
-    // of one j fill aligned lane groups of at least DB lanes, lane p of a group
-    // evaluates them for direction p of a block of DB and the group exchanges
-    // them by shuffles.
-    const int G = d.n3;
-    const bool share = G >= DB && (32 % G == 0) && (blockDim.x % G == 0);
-    const int lane = threadIdx.x & 31;
-    const int gbase = share ? (lane & ~(G - 1)) : lane;
-    const int gpos = lane - gbase;
-    const int row_len = RS * rlen;
-    const R2 lx2 = mk2(g.lx, g.lx), ly2 = mk2(g.ly, g.ly), lz2 = mk2(g.lz, g.lz);
-    const R2 sv2 = mk2(sv, sv), cv2 = mk2(cv, cv), sc3 = mk2(scale3, scale3);
-    const Real gA = prk->gA;
-    const R2 gA2 = mk2(gA, gA);
-
-    // compensated totals (x: Rayleigh, y: Mie) per channel, and the plain
-    // partial sums of the current directions (x: even, y: odd direction)
-    R2 acc[3], cmp[3], ringR[3], ringM[3];
-  #pragma unroll
-    for (int c = 0; c < 3; c++) acc[c] = cmp[c] = ringR[c] = ringM[c] = mk2(Real(0), Real(0));
-    // One block of DB directions starting at w0 (all sky or all ground), two
-    // directions per step.
-    auto dir_block = [&](int w0, auto ground) {
-      Real wRb = 0, wMb = 0;
-      if (share && gpos < DB) {
-        const int wb = w0 + gpos;
-        const Real mu_v = fma(sv, dirs[wb], cv * dirs[used + wb]);
-        wRb = dirs[3 * used + wb] * phR(mu_v);
-        wMb = dirs[3 * used + wb] * phM(mu_v);
-      }
-  #pragma unroll
-      for (int q = 0; q < DB; q += 2) {
-        const int wa = w0 + q;
-        const R2 X0 = ld2(dirs + wa), X1 = ld2(dirs + used + wa), X2 = ld2(dirs + 2 * used + wa);
-        R2 wR, wM;
-        if (share) {
-          wR = mk2(__shfl_sync(0xffffffffu, wRb, gbase + q), __shfl_sync(0xffffffffu, wRb, gbase + q + 1));
-          wM = mk2(__shfl_sync(0xffffffffu, wMb, gbase + q), __shfl_sync(0xffffffffu, wMb, gbase + q + 1));
-        } else {
-          const R2 wt = ld2(dirs + 3 * used + wa);
-          const R2 mu_v = fma2(sv2, X0, mul2(cv2, X1));
-          wR = mul2(wt, phR.pair(mu_v));
-          wM = mul2(wt, phM.pair(mu_v));
-        }
-        const R2 mu_l = fma2(X0, lx2, fma2(X1, ly2, mul2(X2, lz2)));
-        // sun-angle coordinates of (omega, l) along the two directions' heading rows
-        const R2 c3 = fma2(sc3, mu_l, sc3);
-        // |mu| <= 1 up to rounding, so floor(c) lies in [-1, n3 - 1]: texels u
-        // and u + 1 of the padded row give the clamped interpolation exactly
-        // (at u = -1 both are texel 0, at u = n3 - 1 the weight s of the copy
-        // is rounding-small and both are texel n3 - 1)
-        const Real fa = floor(c3.x), fb = floor(c3.y);
-        const int ua = (int)fa, ub = (int)fb;
-        const R2 s3 = sub2(c3, mk2(fa, fb));
-        const Real* ra = rows + wa * row_len + 3 * (ua + 1);
-        const Real* rb = rows + (wa + 1) * row_len + 3 * (ub + 1);
-        R2 X[3];
-  #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          const R2 lo = mk2(ra[c], rb[c]), hi = mk2(ra[3 + c], rb[3 + c]);
-          X[c] = fma2(sub2(hi, lo), s3, lo);
-        }
-        if (FIRST) {
-          const R2 ph = phM.pair(mu_l);
-          const Real* ma = rowsM + wa * row_len + 3 * (ua + 1);
-          const Real* mb = rowsM + (wa + 1) * row_len + 3 * (ub + 1);
-  #pragma unroll
-          for (int c = 0; c < 3; c++) {
-            const R2 lo = mk2(ma[c], mb[c]), hi = mk2(ma[3 + c], mb[3 + c]);
-            X[c] = fma2(fma2(sub2(hi, lo), s3, lo), ph, X[c]);
-          }
-        }
-        if (decltype(ground)::value) {
-          // the ground point's sin of the sun elevation, g.l / |g| = gA + tR (omega . l)
-          const R2 sg = fma2(ld2(dirs + 4 * used + wa), mu_l, gA2);
-          int ea, eb;
-          Real ta, tb;
-          split_coord_r<Real>(sun_elevation_index_r<Real>(sg.x, scaleE), d.nE1, &ea, &ta);
-          split_coord_r<Real>(sun_elevation_index_r<Real>(sg.y, scaleE), d.nE1, &eb, &tb);
-          const int fa = upper_index(ea, d.nE1), fb = upper_index(eb, d.nE1);
-          // both directions' height rows in one 8-byte load (wa is even and
-          // the int array starts 8-byte aligned: kDirFields * used floats, used
-          // a multiple of kDirBlock)
-          const int2 hab = *reinterpret_cast<const int2*>(uE0s + wa);
-          const int ha = hab.x, hb = hab.y;
-          const int ka = upper_index(ha, d.nE0), kb = upper_index(hb, d.nE0);
-          const R2 sE1 = mk2(ta, tb), sE0 = ld2(dirs + 8 * used + wa);
-          const R2 one = mk2(Real(1), Real(1));
-          const R2 oi = sub2(one, sE1);
-          const Real* e0a = etab + 3 * ha * d.nE1;
-          const Real* e0b = etab + 3 * hb * d.nE1;
-          if (sE0.x == Real(0) && sE0.y == Real(0)) {
-            // the vE0 row has weight 0: the bilinear mix is its uE0 row exactly
-            // (the same for every lane: both directions are the warp's)
-  #pragma unroll
-            for (int c = 0; c < 3; c++) {
-              const R2 Y = fma2(mk2(e0a[3 * fa + c], e0b[3 * fb + c]), sE1, mul2(mk2(e0a[3 * ea + c], e0b[3 * eb + c]), oi));
-              X[c] = fma2(ld2(dirs + (5 + c) * used + wa), Y, X[c]);
-            }
-          } else {
-            const R2 oo = sub2(one, sE0);
-            const Real* e1a = etab + 3 * ka * d.nE1;
-            const Real* e1b = etab + 3 * kb * d.nE1;
-  #pragma unroll
-            for (int c = 0; c < 3; c++) {
-              // bilinear in height rows (uE0, vE0) and sun-elevation columns (uE1, vE1)
-              const R2 lo =
-                  fma2(mk2(e0a[3 * fa + c], e0b[3 * fb + c]), sE1, mul2(mk2(e0a[3 * ea + c], e0b[3 * eb + c]), oi));
-              const R2 hi =
-                  fma2(mk2(e1a[3 * fa + c], e1b[3 * fb + c]), sE1, mul2(mk2(e1a[3 * ea + c], e1b[3 * eb + c]), oi));
-              const R2 Y = fma2(hi, sE0, mul2(lo, oo));
-              X[c] = fma2(ld2(dirs + (5 + c) * used + wa), Y, X[c]);
-            }
-          }
-        }
-  #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          ringR[c] = fma2(wR, X[c], ringR[c]);
-          ringM[c] = fma2(wM, X[c], ringM[c]);
-        }
-      }
-    };
-    // the partial sums of up to two blocks go to the compensated totals
-    auto flush = [&]() {
-  #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const R2 x = mk2(ringR[c].x + ringR[c].y, ringM[c].x + ringM[c].y);
-        const R2 y = sub2(x, cmp[c]);
-        const R2 t = add2(acc[c], y);
-        cmp[c] = sub2(sub2(t, acc[c]), y);
-        acc[c] = t;
-        ringR[c] = ringM[c] = mk2(Real(0), Real(0));
-      }
-    };
-    for (int w0 = 0; w0 < sky_end; w0 += DB) {
-      dir_block(w0, std::false_type{});
-      if (w0 & DB) flush();
-    }
-    flush();
-    for (int w0 = sky_end; w0 < used; w0 += DB) {
-      dir_block(w0, std::true_type{});
-      if ((w0 - sky_end) & DB) flush();
-    }
-    flush();
-    if (valid) {
-      // beta_c(x) (atmosphere.clj:42-47, 140-151)
-      const PointRow<Real> pr = *prk;
-      Vec4<Real> o;
-      o.x = pr.bR[0] * acc[0].x + pr.bM[0] * acc[0].y;
-      o.y = pr.bR[1] * acc[1].x + pr.bM[1] * acc[1].y;
-      o.z = pr.bR[2] * acc[2].x + pr.bM[2] * acc[2].y;
-      // J planar, [atmosphere][channel][node], for the ray-scatter gathers
-      Real* Jb = J + (long long)b * 3 * d.n4() + (node - base4);
-      Jb[0] = o.x;
-      Jb[d.n4()] = o.y;
-      Jb[2 * d.n4()] = o.z;
-    }
-  }
-}
-
-template <class Real>
-size_t point_scatter_smem(const BuildDims& d, bool first) {
-  const size_t n = dir_row(d.P);
-  return ((n * (kDirFields * sizeof(Real) + sizeof(int)) + 15) & ~size_t(15)) +
-         sizeof(Real) * 3 * (n * (d.n3 + 2) * (first ? 2 : 1) + d.nE());
-}
-
-template <class Real>
-int launch_point_scatter(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
-                         const SphereDir<Real>* pdirs, const unsigned char* dimage, const int2* pcount,
-                         const PointRow<Real>* prow, const CellGeom<Real>* geom, const Vec4<Real>* dS,
-                         const Vec4<Real>* mie, const Vec4<Real>* dE, Real* hrows, Real* J, cudaStream_t st) {
-  const int block = 256;
-  const int nchunks = (d.n1 * d.n3 + block - 1) / block;
-  const int cpb = 2;
-  const bool first = mie != nullptr;
-  size_t smem = point_scatter_smem<Real>(d, first);
-  const dim3 rgrid((unsigned)(d.n0 * d.n2), d.B);
-  dim3 grid((unsigned)(d.n0 * d.n2 * point_scatter_blocks_per_pair(nchunks, cpb)), d.B);
-  if (first) {
-    if (cudaFuncSetAttribute(k_point_scatter<Real, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return -1;
-    k_heading_rows<Real, true><<<rgrid, block, 0, st>>>(d, pdirs, pcount, prow, dS, mie, hrows);
-    k_point_scatter<Real, true><<<grid, block, smem, st>>>(params, d, rowinfo, pdirs, dimage, pcount, prow, geom,
-                                                           hrows, dE, J, nchunks, cpb);
-  } else {
-    if (cudaFuncSetAttribute(k_point_scatter<Real, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-      return -1;
-    k_heading_rows<Real, false><<<rgrid, block, 0, st>>>(d, pdirs, pcount, prow, dS, nullptr, hrows);
-    k_point_scatter<Real, false><<<grid, block, smem, st>>>(params, d, rowinfo, pdirs, dimage, pcount, prow, geom,
-                                                            hrows, dE, J, nchunks, cpb);
-  }
-  return 0;
 }
 
 // Threads per surface-radiance node: 128 lets about seven blocks share an
@@ -1046,10 +631,6 @@ void launch_export(long long n, const Vec4<Real>* tab, float* out, cudaStream_t 
 }
 
 #define SFSIM_INSTANTIATE(Real)                                                                                     \
-  template int launch_point_scatter<Real>(const AtmoParams*, const BuildDims&, const RowInfo*,                     \
-                                          const SphereDir<Real>*, const unsigned char*, const int2*,               \
-                                          const PointRow<Real>*, const CellGeom<Real>*, const Vec4<Real>*,         \
-                                          const Vec4<Real>*, const Vec4<Real>*, Real*, Real*, cudaStream_t);       \
   template void launch_surface_radiance<Real>(const AtmoParams*, const BuildDims&, const SurfRow<Real>*,          \
                                               const HalfDir<Real>*, const Vec4<Real>*, const Vec4<Real>*,          \
                                               Vec4<Real>*, cudaStream_t);                                          \
@@ -1066,7 +647,6 @@ void launch_export(long long n, const Vec4<Real>* tab, float* out, cudaStream_t 
   template void launch_export<Real>(long long, const Vec4<Real>*, float*, cudaStream_t);                           \
   template void launch_add_to_sum<Real>(long long, int, const Real*, Vec4<float>*, bool, cudaStream_t);           \
   template void launch_export_planar<Real>(long long, int, const Real*, float*, cudaStream_t);                      \
-  template size_t point_scatter_smem<Real>(const BuildDims&, bool);                                                 \
   template size_t ray_scatter_smem<Real>(const BuildDims&);
 
 SFSIM_INSTANTIATE(float)

@@ -356,13 +356,84 @@ __global__ void k_view_rows_scan(const AtmoParams* params, BuildDims d, const Ro
 }
 
 // ---------------------------------------------------------------------------
-// Sphere directions of point scatter per height row (atmosphere.clj:203-222,
-// sphere.clj:62-105): the direction in world space, where it ends, whether
-// that end is on the ground, the elevation coordinate of the dS lookup and,
-// for ground ends, T(x, g) * brightness / pi and the ground point's height
-// coordinate in the surface-radiance space.
+// Sphere rings of point scatter per height row (atmosphere.clj:203-222,
+// sphere.clj:62-105): where the ring's directions end, whether that end is on
+// the ground, the elevation coordinate of the dS lookup and, for ground ends,
+// T(x, g) * brightness / pi.  x = (r, 0, 0), so the ring's directions have
+// the same first component and with it the same end; the ring's first
+// direction stands for all.  One block per height: a warp finds the rings in
+// the direction list (the directions of a ring follow one another and share
+// their polar cosine), then each warp takes a ring, its lanes the samples of
+// the ground's optical depth.
 // ---------------------------------------------------------------------------
 
+template <class Real>
+__global__ void __launch_bounds__(256) k_sphere_rings(const AtmoParams* params, BuildDims d, const DirLocal* dirs,
+                                                      SphereRing<Real>* out, Real* dirs4, Real* offsets) {
+  extern __shared__ int start[];  // first direction of each ring, and P
+  const int i = blockIdx.x, b = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 0) {
+    int found = 0;
+    for (int t0 = 0; t0 < d.P; t0 += 32) {
+      const int t = t0 + lane;
+      const bool first = t < d.P && (t == 0 || dirs[t].x != dirs[t - 1].x);
+      const unsigned ballot = __ballot_sync(0xffffffffu, first);
+      const int pos = found + __popc(ballot & ((1u << lane) - 1u));
+      if (first && pos < d.T) start[pos] = t;
+      found += __popc(ballot);
+    }
+    if (lane == 0) start[d.T] = d.P;
+  }
+  __syncthreads();
+  const AtmoParams& P = params[b];
+  const double r = index_to_radius(P, d.n0, (double)i);
+  const d3 x = mk3(r, 0, 0);
+  const d3 n = mul3(x, 1.0 / mag3(x));
+  const d3 o1 = orthogonal(n);
+  const d3 o2 = cross3(n, o1);
+  if (i == 0 && b == 0) {
+    for (int t = threadIdx.x; t < d.P; t += blockDim.x) {
+      const d3 omega = to_world(n, o1, o2, dirs[t]);
+      dirs4[4 * t] = dirs4[4 * t + 1] = (Real)omega.y;
+      dirs4[4 * t + 2] = dirs4[4 * t + 3] = (Real)omega.z;
+    }
+  }
+  if (std::is_same<Real, double>::value) {
+    // per direction: the ground point is on the ground up to its rounding
+    for (int t = threadIdx.x; t < d.P; t += blockDim.x) {
+      const d3 g = ray_extremity(P, x, to_world(n, o1, o2, dirs[t]));
+      int u = 0;
+      Real s = 0;
+      if (surface_point(P, g)) split_coord<Real>(height_to_index(P, d.nE0, mag3(g)), d.nE0, &u, &s);
+      offsets[((long long)b * d.n0 + i) * d.P + t] = s;
+    }
+  }
+  for (int k = warp; k < d.T; k += blockDim.x >> 5) {
+    const int w = start[k];
+    const d3 omega = to_world(n, o1, o2, dirs[w]);
+    const d3 g = ray_extremity(P, x, omega);
+    const int surface = surface_point(P, g);
+    SphereRing<Real> o;
+    o.x0 = (Real)omega.x;
+    o.weight = (Real)dirs[w].w;
+    o.surface = surface;
+    o.w0 = w;
+    o.n = start[k + 1] - w;
+    split_coord<Real>(elevation_to_index(P, d.n1, x, omega, !surface), d.n1, &o.u1, &o.s1);
+    o.tR = o.ground[0] = o.ground[1] = o.ground[2] = 0;
+    if (surface) {
+      Real tau[3];
+      segment_depth_warp<Real>(P, x, sub3(g, x), d.S, lane, tau);
+      for (int c = 0; c < 3; c++) o.ground[c] = exp_neg(tau[c]) * (Real)(P.brightness[c] / M_PI);
+      const double tR = mag3(sub3(g, x)) / P.R;
+      o.tR = tR < 1.0e30 ? (Real)tR : Real(0);  // point scatter forms table indices from it
+    }
+    if (lane == 0) out[((long long)b * d.n0 + i) * d.T + k] = o;
+  }
+}
+
+// The same per direction, for the work census (one thread per height and direction).
 template <class Real>
 __global__ void k_sphere_setup(const AtmoParams* params, BuildDims d, const DirLocal* dirs,
                                SphereDir<Real>* out) {
@@ -403,81 +474,6 @@ __global__ void k_sphere_setup(const AtmoParams* params, BuildDims d, const DirL
   out[((long long)b * d.n0 + i) * d.P + w] = o;
 }
 
-// The sphere directions of one height row split into those that end in the
-// sky and those that end on the ground (the latter with an exactly-zero
-// ground height coordinate first), order kept within each part, and
-// each part filled to a multiple of kDirBlock with zero-weight entries, so
-// that point scatter runs both parts in whole blocks of directions without
-// a branch per direction.  One warp per row.
-template <class Real>
-__global__ void k_sphere_partition(BuildDims d, const SphereDir<Real>* sdirs, SphereDir<Real>* pdirs,
-                                   int2* pcount, unsigned char* dimage) {
-  const int i = blockIdx.x, b = blockIdx.y, lane = threadIdx.x;
-  const long long row = (long long)b * d.n0 + i;
-  const SphereDir<Real>* src = sdirs + row * d.P;
-  SphereDir<Real>* dst = pdirs + row * dir_row(d.P);
-  // three groups, order kept within each: sky, ground with the ground
-  // point's height coordinate exactly 0 (most of them: only its lower E row
-  // has weight), other ground
-  int nsky = 0, nflat = 0;
-  for (int t0 = 0; t0 < d.P; t0 += 32) {
-    const int t = t0 + lane;
-    const bool in = t < d.P;
-    nsky += __popc(__ballot_sync(0xffffffffu, in && !src[t].surface));
-    nflat += __popc(__ballot_sync(0xffffffffu, in && src[t].surface && src[t].sE0 == Real(0)));
-  }
-  const int sky_end = (nsky + kDirBlock - 1) / kDirBlock * kDirBlock;
-  const int nground = d.P - nsky;
-  const int used = sky_end + (nground + kDirBlock - 1) / kDirBlock * kDirBlock;
-  const unsigned below = (1u << lane) - 1u;
-  int s = 0, f = 0, g = 0;
-  for (int t0 = 0; t0 < d.P; t0 += 32) {
-    const int t = t0 + lane;
-    const bool in = t < d.P;
-    const bool sky = in && !src[t].surface;
-    const bool flat = in && !sky && src[t].sE0 == Real(0);
-    const unsigned bs = __ballot_sync(0xffffffffu, sky), bf = __ballot_sync(0xffffffffu, flat);
-    const unsigned bg = __ballot_sync(0xffffffffu, in && !sky && !flat);
-    if (in) {
-      SphereDir<Real> e = src[t];
-      e.pad = 0;
-      const int pos = sky ? s + __popc(bs & below)
-                          : (flat ? sky_end + f + __popc(bf & below) : sky_end + nflat + g + __popc(bg & below));
-      dst[pos] = e;
-    }
-    s += __popc(bs);
-    f += __popc(bf);
-    g += __popc(bg);
-  }
-  SphereDir<Real> z;
-  for (int c = 0; c < 3; c++) z.w[c] = z.ground[c] = 0;
-  z.tR = 0;
-  z.weight = z.s1 = z.sE0 = 0;
-  z.u1 = z.uE0 = 0;
-  z.pad = 1;
-  for (int t = nsky + lane; t < sky_end; t += 32) {
-    z.surface = 0;
-    dst[t] = z;
-  }
-  for (int t = sky_end + nground + lane; t < used; t += 32) {
-    z.surface = 1;
-    dst[t] = z;
-  }
-  if (lane == 0) pcount[row] = make_int2(sky_end, used);
-  // point scatter's shared-memory image of the list: each field as an array
-  __syncwarp();
-  Real* img = reinterpret_cast<Real*>(dimage + row * dir_image_stride(d, sizeof(Real)));
-  int* img_u = reinterpret_cast<int*>(img + kDirFields * used);
-  for (int t = lane; t < used; t += 32) {
-    const SphereDir<Real> e = dst[t];
-    const Real f[kDirFields] = {e.w[0],      e.w[1],      e.w[2],      e.weight, e.tR,
-                                e.ground[0], e.ground[1], e.ground[2], e.sE0};
-#pragma unroll
-    for (int c = 0; c < kDirFields; c++) img[c * used + t] = f[c];
-    img_u[t] = e.uE0;
-  }
-}
-
 // Point-scatter constants per (height i, sun elevation k): the coordinates
 // of ray-scatter-forward (atmosphere.clj:203-222) at x = (r_i, 0, 0) with the
 // sun at elevation k, and beta_c(x) (atmosphere.clj:42-47, 140-151), in FP64
@@ -499,7 +495,9 @@ __global__ void k_point_rows(const AtmoParams* params, BuildDims d, PointRow<Rea
   PointRow<Real> o;
   o.ss = ss;
   o.cs = sqrt(dmax(0.0, dsub(1.0, sqr(ss))));
-  o.gA = (Real)(r * ss / P.R);
+  o.lz = (Real)sqrt(dmax(0.0, dsub(dsub(1.0, sqr(o.cs)), sqr(ss))));
+  const double gA = r * ss / P.R;
+  o.gA = fabs(gA) < 1.0e30 ? (Real)gA : Real(0);  // point scatter forms table indices from it
   split_coord<Real>(height_to_index(P, d.n0, r), d.n0, &o.u0, &o.s0);
   split_coord<Real>(sun_elevation_to_index(d.n2, mk3(r, 0, 0), mk3(ss, 0, 0)), d.n2, &o.u2, &o.s2);
   const double h = r - P.R;
@@ -597,12 +595,12 @@ int launch_setup_aux(const AtmoParams* params, const BuildDims& d, const DirLoca
   // a build without iterations may ask for no sphere directions (sphere
   // steps below 2) or no half-sphere ones (ray steps below 4): nothing to launch
   if (d.P > 0)
-    k_sphere_setup<Real><<<grid1((long long)d.n0 * d.P, blk, d.B), blk, 0, st>>>(params, d, dirs, o.sdirs);
-  k_sphere_partition<Real><<<dim3(d.n0, d.B), 32, 0, st>>>(d, o.sdirs, o.pdirs, o.pcount, o.dimage);
+    k_sphere_rings<Real><<<dim3(d.n0, d.B), 256, sizeof(int) * (d.T + 1), st>>>(params, d, dirs, o.rings, o.dirs4,
+                                                                                   o.offsets);
   k_surface_rows<Real><<<grid1(d.nE(), blk, d.B), blk, 0, st>>>(params, d, o.erow);
   if (d.Ph > 0)
     k_half_dirs<Real><<<grid1((long long)d.nE0 * d.Ph, blk, d.B), blk, 0, st>>>(params, d, half_dirs, o.hdir);
-  return 4 + (d.P > 0) + (d.Ph > 0);
+  return 3 + (d.P > 0) + (d.Ph > 0);
 }
 
 template <class Real>
@@ -612,6 +610,13 @@ void launch_setup(const AtmoParams* params, const BuildDims& d, const DirLocal* 
   launch_node_maps<Real>(params, d, o, st);
   launch_view_rows<Real>(params, d, o, st);
   launch_setup_aux<Real>(params, d, dirs, half_dirs, o, st);
+}
+
+template <class Real>
+void launch_sphere_dirs(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs, SphereDir<Real>* out,
+                        cudaStream_t st) {
+  const int blk = 128;
+  if (d.P > 0) k_sphere_setup<Real><<<grid1((long long)d.n0 * d.P, blk, d.B), blk, 0, st>>>(params, d, dirs, out);
 }
 
 template <class Real>
@@ -646,6 +651,10 @@ template void launch_setup<float>(const AtmoParams*, const BuildDims&, const Dir
                                   const SetupBuffers<float>&, cudaStream_t);
 template void launch_setup<double>(const AtmoParams*, const BuildDims&, const DirLocal*, const DirLocal*,
                                    const SetupBuffers<double>&, cudaStream_t);
+template void launch_sphere_dirs<float>(const AtmoParams*, const BuildDims&, const DirLocal*, SphereDir<float>*,
+                                        cudaStream_t);
+template void launch_sphere_dirs<double>(const AtmoParams*, const BuildDims&, const DirLocal*, SphereDir<double>*,
+                                         cudaStream_t);
 template void launch_transmittance<float>(const AtmoParams*, const BuildDims&, Vec4<float>*, cudaStream_t);
 template void launch_transmittance<double>(const AtmoParams*, const BuildDims&, Vec4<double>*, cudaStream_t);
 template void launch_surface_base<float>(const AtmoParams*, const BuildDims&, Vec4<float>*, cudaStream_t);

@@ -17,49 +17,25 @@ struct SetupBuffers {
   RowInfo* rowinfo;
   Remap2<Real>* rowmap;  // [B][rows]: height and elevation coordinates of each view row
   RowSample<Real>* rows;
-  SphereDir<Real>* sdirs;
-  // sdirs partitioned per height row: the directions that end in the sky,
-  // then those that end on the ground, each part filled to a multiple of
-  // kDirBlock with zero-weight entries (pad = 1); kDirRow entries per row,
-  // pcount = {first ground entry, entries used}
-  SphereDir<Real>* pdirs;
-  int2* pcount;
-  // point scatter's shared-memory image of each height's partitioned
-  // directions (dir_image_bytes per height): the fields as arrays, then uE0
-  unsigned char* dimage;
+  SphereRing<Real>* rings;  // [B][n0][T]: point scatter's rings per height
+  Real* dirs4;              // [P][4]: x1, x1, x2, x2 of its directions (the same at every height)
+  Real* offsets;            // [B][n0][P]: surface-radiance height coordinate of the ground points (FP64 builds)
   PointRow<Real>* prow;  // [B][n0][n2]
   double* hdvs;          // [n3]: 2 a / (n3 - 1) - 1, index-to-sun-direction's v.l of heading a
   SurfRow<Real>* erow;   // [B][nE0][nE1]
   HalfDir<Real>* hdir;   // [B][nE0][Ph]
 };
 
-constexpr int kDirBlock = 8;
-__host__ __device__ constexpr int dir_row(int P) { return P + 2 * kDirBlock; }
-
-// Fields per direction in point scatter's shared direction arrays: x0, x1,
-// x2, weight, tR, ground0..2, sE0 (then uE0 as ints).
-constexpr int kDirFields = 9;
-// Bytes of the direction image of `used` directions, a multiple of 16.
-__host__ __device__ inline size_t dir_image_bytes(int used, size_t real_size) {
-  return ((size_t)used * (kDirFields * real_size + sizeof(int)) + 15) & ~size_t(15);
-}
-// Room per height in the global images: the most partitioned directions.
-__host__ __device__ inline size_t dir_image_stride(const BuildDims& d, size_t real_size) {
-  return dir_image_bytes((dir_row(d.P) + 7) / 8 * 8, real_size);
-}
-
-// Reals of one (height, sun elevation) pair's heading rows in point
-// scatter's global row table: the dS and Mie rows of every partitioned
-// direction, n3 + 2 RGB texels each; a multiple of 48.
-__host__ __device__ inline long long heading_rows_stride(const BuildDims& d) {
-  return 2LL * ((dir_row(d.P) + 7) / 8 * 8) * (d.n3 + 2) * 3;
-}
+// Bytes of shared memory that point scatter's tables are allowed: the limit
+// on a configuration's directions, headings and surface-radiance table, the
+// same for every build that runs.
+template <class Real>
+size_t point_scatter_capacity(const BuildDims& d);
 
 // The set-up tables in parts: the rows (row info and point rows), then the
 // 4-D node maps with each node's light direction (remap4) and the view-row
 // samples, which both read the rows but not each other, and the rest
-// (remapT, remapE, sphere directions and their partition, surface rows, half
-// directions).  launch_setup runs them all on one stream.
+// (remapT, remapE, sphere rings, surface rows, half directions).  launch_setup runs them all on one stream.
 template <class Real>
 void launch_setup_rows(const AtmoParams* params, const BuildDims& d, const SetupBuffers<Real>& o, cudaStream_t st);
 template <class Real>
@@ -126,12 +102,16 @@ int launch_smem_probe(int blocks, int iters, float* sink, cudaStream_t st);
 
 // J = point scatter of (dS, dE), planar [atmosphere][channel][node]; when
 // `mie` is non-NULL dS is the first iteration's rayleigh + mie * phase(mie, v.l).
-// hrows: scratch for the heading rows, B * n0 * n2 * heading_rows_stride(d) Reals.
 template <class Real>
 int launch_point_scatter(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
-                         const SphereDir<Real>* pdirs, const unsigned char* dimage, const int2* pcount,
-                         const PointRow<Real>* prow, const CellGeom<Real>* geom, const Vec4<Real>* dS,
-                         const Vec4<Real>* mie, const Vec4<Real>* dE, Real* hrows, Real* J, cudaStream_t st);
+                         const SphereRing<Real>* rings, const Real* dirs4, const Real* offsets,
+                         const PointRow<Real>* prow, const CellGeom<Real>* geom, const Vec4<Real>* dS, const Vec4<Real>* mie, const Vec4<Real>* dE,
+                         Real* J, cudaStream_t st);
+
+// The ends of every sphere direction at every height, for the work census.
+template <class Real>
+void launch_sphere_dirs(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs, SphereDir<Real>* out,
+                        cudaStream_t st);
 
 // dE = surface radiance of dS (same first-iteration convention).
 template <class Real>
