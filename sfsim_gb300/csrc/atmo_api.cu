@@ -17,11 +17,6 @@
 #include "atmo_device.cuh"
 #include "kernels.h"
 
-namespace sfsim {
-template <class Real>
-size_t ray_scatter_smem(const BuildDims& d);
-}
-
 using namespace sfsim;
 
 namespace {
@@ -329,7 +324,7 @@ template <class Real>
 int check_smem(const BuildDims& d) {
   if (point_scatter_capacity<Real>(d) > kMaxSmem)
     return fail(SFSIM_ATMO_ESHAPE, "elevation x heading slab of point scatter exceeds shared memory");
-  if (ray_scatter_smem<Real>(d) > kMaxSmem)
+  if (ray_scatter_capacity<Real>(d) > kMaxSmem)
     return fail(SFSIM_ATMO_ESHAPE, "sun elevation x heading plane of ray scatter exceeds shared memory");
   if (first_order_smem<Real>(d, false) > kMaxSmem)
     return fail(SFSIM_ATMO_ESHAPE, "the view rows' samples of the first order exceed shared memory");
@@ -378,8 +373,7 @@ struct Work {
   DirLocal* hdirs;
   SetupBuffers<Real> setup;
   Vec4<Real>*T, *E0, *dE[2], *Eacc[2];
-  Vec4<Real>*S1R, *M, *dS[2], *Sacc[2];
-  Real* J;
+  Vec4<Real>*S1R, *M, *J, *dS[2], *Sacc[2];
   float *oT, *oE, *oS, *oM;  // device outputs when the caller passes host buffers
   unsigned char* sun;        // sun-ray optical-depth tables, kSunTableBytes per atmosphere (FP32 builds), or NULL
 };
@@ -398,7 +392,7 @@ size_t carve(Work<Real>& w, char* base, const BuildDims& d, bool outputs, bool s
   w.params = c.take<AtmoParams>(B);
   w.dirs = c.take<DirLocal>(d.P + 1);
   w.hdirs = c.take<DirLocal>(d.Ph + 1);
-  w.setup.remapS = c.take<Remap4<Real>>(B * d.n4());
+  w.setup.angle = c.take<Coord<Real>>(B * d.n4());
   w.setup.geom = c.take<CellGeom<Real>>(B * d.n4());
   w.setup.remapT = c.take<Remap2<Real>>(B * d.nT());
   w.setup.remapE = c.take<Remap2<Real>>(B * d.nE());
@@ -420,7 +414,7 @@ size_t carve(Work<Real>& w, char* base, const BuildDims& d, bool outputs, bool s
   }
   w.S1R = c.take<Vec4<Real>>(B * d.n4());
   w.M = c.take<Vec4<Real>>(B * d.n4());
-  w.J = c.take<Real>(3 * B * d.n4());  // planar [atmosphere][channel][node]
+  w.J = c.take<Vec4<Real>>(B * d.n4());
   for (int i = 0; i < 2; i++) {
     w.dS[i] = c.take<Vec4<Real>>(B * d.n4());
     w.Sacc[i] = c.take<Vec4<Real>>(B * d.n4());
@@ -594,7 +588,7 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
   // (and, for host outputs, their copies) need not wait for the iterations
   tm.mark_begin(9);
   launch_output2<Real>(d.B, d.nT0, d.nT1, w.setup.remapT, w.T, oT, st);
-  launch_output4<Real>(d, w.setup.remapS, w.M, oM, st);
+  launch_output4<Real>(d, w.setup, w.M, oM, st);
   launches += 2;
   tm.mark_end();
   if (early_done) CUDA_TRY(cudaEventRecord(early_done, st));
@@ -672,14 +666,13 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
     launches++;
     tm.mark_end();
     if (jsum) {
-      launch_add_to_sum<Real>(d.n4(), d.B, w.J, jsum, it == 0, st);
+      launch_add_to_sum<Real>(d.B * d.n4(), w.J, jsum, it == 0, st);
       launches++;
     }
 
     if (fork && it > it0) CUDA_TRY(cudaStreamWaitEvent(st, g_side_acc[tm.dev], 0));  // its dS buffer read
     tm.mark_begin(7);
-    if (launch_ray_scatter<Real>(w.params, d, w.setup.rowinfo, w.setup.rows, w.setup.geom, w.setup.remapS, w.J,
-                                 dS_new, st))
+    if (launch_ray_scatter<Real>(d, w.setup.rowinfo, w.setup.rows, w.setup.geom, w.setup.angle, w.J, dS_new, st))
       return fail(SFSIM_ATMO_ECUDA, "ray scatter launch configuration failed");
     launches++;
     tm.mark_end();
@@ -689,14 +682,14 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
     }
     tm.mark_begin(8, ss);
     launch_accumulate2<Real>(d.B, d.nE0, d.nE1, w.setup.remapE, E_prev, dE_new, E_new, ss);
-    launch_accumulate4<Real>(d, w.setup.remapS, S_prev, dS_new, S_new, ss);
+    launch_accumulate4<Real>(d, w.setup, S_prev, dS_new, S_new, ss);
     launches += 2;
     tm.mark_end(ss);
     if (fork) CUDA_TRY(cudaEventRecord(g_side_acc[tm.dev], ss));
     CUDA_TRY(cudaGetLastError());
     if (inter) {
       if (inter->point_scatter)
-        launch_export_planar<Real>(d.n4(), d.B, w.J, inter->point_scatter + (size_t)3 * d.B * d.n4() * it, st);
+        launch_export<Real>(d.B * d.n4(), w.J, inter->point_scatter + (size_t)3 * d.B * d.n4() * it, st);
       if (inter->surface_delta)
         launch_export<Real>(d.B * d.nE(), dE_new, inter->surface_delta + (size_t)3 * d.B * d.nE() * it, st);
       if (inter->ray_scatter_delta)
@@ -724,7 +717,7 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
   if (fork && d.iterations > it0) CUDA_TRY(cudaStreamWaitEvent(st, g_side_acc[tm.dev], 0));  // the final S and E
   tm.mark_begin(9);
   launch_output2<Real>(d.B, d.nE0, d.nE1, w.setup.remapE, E_prev, oE, st);
-  launch_output4<Real>(d, w.setup.remapS, S_prev, oS, st);
+  launch_output4<Real>(d, w.setup, S_prev, oS, st);
   launches += 2;
   tm.mark_end();
   CUDA_TRY(cudaGetLastError());
@@ -1571,20 +1564,23 @@ int static_scratch_base(int dev, void** base) {
   return 0;
 }
 
-// What the static array's limit counts beside the scratch tables: the row
-// tables and direction lists per (height, sun elevation) pair that point
-// scatter no longer keeps.  They stay in the count so that the configurations
-// the entry point accepts stay the same.
+// What the static array's limit counts beside the scratch tables: tables that
+// the build no longer keeps (point scatter's rows per (height, sun elevation)
+// pair and its direction lists, four coordinates per node) less those that
+// took their place.  They stay in the count so that the configurations the
+// entry point accepts stay the same.
 template <class Real>
 size_t static_margin(const BuildDims& d) {
-  auto up = [](long long x) { return (size_t)((x + 255) & ~255LL); };
-  const long long n = d.P + 16, n8 = (n + 7) / 8 * 8, R = sizeof(Real);
-  const size_t lists = up(sizeof(SphereDir<Real>) * d.n0 * (d.P + 1LL)) + up(sizeof(SphereDir<Real>) * d.n0 * n) +
-                       up(d.n0 * ((n8 * (9 * R + 4) + 15) & ~15LL)) + up(sizeof(int2) * d.n0);
-  const size_t rows = up(R * d.n0 * d.n2 * 2 * n8 * (d.n3 + 2) * 3);
-  const size_t kept = up(sizeof(SphereRing<Real>) * d.n0 * (d.T + 1LL)) + up(R * 4 * (d.P + 1LL)) +
-                      up(R == 8 ? R * d.n0 * d.P : 0);
-  return lists + rows > kept ? lists + rows - kept : 0;
+  auto up = [](long long x) { return (long long)((x + 255) & ~255LL); };
+  const long long n = d.P + 16, n8 = (n + 7) / 8 * 8, R = sizeof(Real), n4 = d.n4(), pairs = (long long)d.n0 * d.n2;
+  const long long gone = up(sizeof(SphereDir<Real>) * d.n0 * (d.P + 1LL)) + up(sizeof(SphereDir<Real>) * d.n0 * n) +
+                         up(d.n0 * ((n8 * (9 * R + 4) + 15) & ~15LL)) + up(sizeof(int2) * d.n0) +
+                         up(R * pairs * 2 * n8 * (d.n3 + 2) * 3) + up(4 * (sizeof(int) + R) * n4) + up(3 * R * n4) +
+                         up((R == 8 ? 96 : 64) * pairs);
+  const long long kept = up(sizeof(SphereRing<Real>) * d.n0 * (d.T + 1LL)) + up(R * 4 * (d.P + 1LL)) +
+                         up(R == 8 ? R * d.n0 * d.P : 0) + up(sizeof(Coord<Real>) * n4) + up(sizeof(Vec4<Real>) * n4) +
+                         up(sizeof(PointRow<Real>) * pairs);
+  return gone > kept ? (size_t)(gone - kept) : 0;
 }
 
 template <class Real>

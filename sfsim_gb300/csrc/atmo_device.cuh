@@ -423,6 +423,51 @@ __device__ __forceinline__ V sub2(V b, V a) {
   return fma2(a, mk2(decltype(a.x)(-1), decltype(a.x)(-1)), b);
 }
 
+// floor(c) of both lanes for |c| < 2^22: adding 1.5 2^23 rounding down leaves
+// floor(c) in the low bits, without the conversions of floor() and (int).
+constexpr float kFloorMagic = 12582912.0f;
+constexpr unsigned kFloorBits = 0x4B400000u;  // the bits of kFloorMagic
+
+// Lookups along a table of records of `stride` bytes: the byte offsets of
+// both lanes' records (from the start of shared memory) and their fractions.
+// For float the table's offset is lowered by stride * kFloorBits once
+// (lookup_base), so that a record's offset is one multiply-add of the sum's
+// bits.
+template <class Real>
+__device__ __forceinline__ unsigned lookup_base(unsigned origin, unsigned stride) {
+  return std::is_same<Real, float>::value ? origin - stride * kFloorBits : origin;
+}
+__device__ __forceinline__ float2 lookup(float2 c, unsigned base_a, unsigned base_b, unsigned stride, unsigned& oa,
+                                         unsigned& ob) {
+  const float2 t = __fadd2_rd(c, make_float2(kFloorMagic, kFloorMagic));
+  oa = __float_as_uint(t.x) * stride + base_a;
+  ob = __float_as_uint(t.y) * stride + base_b;
+  return sub2(c, __fadd2_rn(t, make_float2(-kFloorMagic, -kFloorMagic)));
+}
+__device__ __forceinline__ double2 lookup(double2 c, unsigned base_a, unsigned base_b, unsigned stride, unsigned& oa,
+                                          unsigned& ob) {
+  const double fa = floor(c.x), fb = floor(c.y);
+  oa = (unsigned)(int)fa * stride + base_a;
+  ob = (unsigned)(int)fb * stride + base_b;
+  return make_double2(c.x - fa, c.y - fb);
+}
+
+// Two 16-byte-aligned pairs in one load (two for double).
+__device__ __forceinline__ void ld_pairs(const float* p, float2& a, float2& b) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  a = make_float2(v.x, v.y);
+  b = make_float2(v.z, v.w);
+}
+__device__ __forceinline__ void ld_pairs(const double* p, double2& a, double2& b) {
+  a = reinterpret_cast<const double2*>(p)[0];
+  b = reinterpret_cast<const double2*>(p)[1];
+}
+
+template <class Real>
+__device__ __forceinline__ V2<Real> dup(Real a) {
+  return mk2(a, a);
+}
+
 // Cornette-Shanks phase k (1 + mu^2) (a + b mu)^-3/2 from the host-computed
 // coefficients {k, a, b} of AtmoParams.
 template <class Real>

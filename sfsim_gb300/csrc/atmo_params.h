@@ -98,13 +98,6 @@ struct alignas(2 * sizeof(Real) >= 8 ? 2 * sizeof(Real) : 8) Coord {
   Real s;
 };
 
-// Re-interpolation coordinates of a 4-D node (forward of backward of the node).
-template <class Real>
-struct Remap4 {
-  int u[4];
-  Real s[4];
-};
-
 template <class Real>
 struct Remap2 {
   int u[2];

@@ -37,49 +37,6 @@
 
 namespace sfsim {
 
-// floor(c) of both lanes for |c| < 2^22: adding 1.5 2^23 rounding down leaves
-// floor(c) in the low bits, without the conversions of floor() and (int).
-constexpr float kFloorMagic = 12582912.0f;
-constexpr unsigned kFloorBits = 0x4B400000u;  // the bits of kFloorMagic
-
-// Lookups along a table of records of `stride` bytes: the byte offsets of
-// both lanes' records (from the start of shared memory) and their fractions.
-// For float the table's offset is lowered by stride * kFloorBits once
-// (lookup_base), so that a record's offset is one multiply-add of the sum's
-// bits.
-template <class Real>
-__device__ __forceinline__ unsigned lookup_base(unsigned origin, unsigned stride) {
-  return std::is_same<Real, float>::value ? origin - stride * kFloorBits : origin;
-}
-__device__ __forceinline__ float2 lookup(float2 c, unsigned base, unsigned stride, unsigned& oa, unsigned& ob) {
-  const float2 t = __fadd2_rd(c, make_float2(kFloorMagic, kFloorMagic));
-  oa = __float_as_uint(t.x) * stride + base;
-  ob = __float_as_uint(t.y) * stride + base;
-  return sub2(c, __fadd2_rn(t, make_float2(-kFloorMagic, -kFloorMagic)));
-}
-__device__ __forceinline__ double2 lookup(double2 c, unsigned base, unsigned stride, unsigned& oa, unsigned& ob) {
-  const double fa = floor(c.x), fb = floor(c.y);
-  oa = (unsigned)(int)fa * stride + base;
-  ob = (unsigned)(int)fb * stride + base;
-  return make_double2(c.x - fa, c.y - fb);
-}
-
-// Two 16-byte-aligned pairs in one load (two for double).
-__device__ __forceinline__ void ld_pairs(const float* p, float2& a, float2& b) {
-  const float4 v = *reinterpret_cast<const float4*>(p);
-  a = make_float2(v.x, v.y);
-  b = make_float2(v.z, v.w);
-}
-__device__ __forceinline__ void ld_pairs(const double* p, double2& a, double2& b) {
-  a = reinterpret_cast<const double2*>(p)[0];
-  b = reinterpret_cast<const double2*>(p)[1];
-}
-
-template <class Real>
-__device__ __forceinline__ V2<Real> dup(Real a) {
-  return mk2(a, a);
-}
-
 // Values per record of a ring row: three channels' (value, step to the next
 // texel), in the first iteration those of the Mie strength too; an odd
 // stride spreads the texels over the banks.
@@ -173,7 +130,7 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     k_point_scatter(const AtmoParams* params, BuildDims d, PointLayout lay, const RowInfo* rowinfo,
                     const SphereRing<Real>* rings, const Real* dirs4, const Real* offsets,
                     const PointRow<Real>* prow, const CellGeom<Real>* geom, const Vec4<Real>* dS, const Vec4<Real>* Mt, const Vec4<Real>* dE,
-                    Real* J, int groups, int chunks) {
+                    Vec4<Real>* J, int groups, int chunks) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using R2 = V2<Real>;
   constexpr int KS = row_stride<FIRST>();
@@ -260,7 +217,7 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     // the sun-angle coordinate; |mu| <= 1 up to rounding, so its floor lies in
     // [-1, n3 - 1], whose records give the clamped interpolation
     unsigned oa, ob;
-    const R2 s = lookup(fma2(dup(scale3), mu, dup(scale3)), rbase, kstride, oa, ob);
+    const R2 s = lookup(fma2(dup(scale3), mu, dup(scale3)), rbase, rbase, kstride, oa, ob);
     const Real* ra = reinterpret_cast<const Real*>(smem_raw + oa);
     const Real* rb = reinterpret_cast<const Real*>(smem_raw + ob);
 #pragma unroll
@@ -279,7 +236,7 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
       const R2 ex = mk2(Bulk<Real>::exp2(z.x), Bulk<Real>::exp2(z.y));
       R2 ie = fma2(dup(-scaleE), ex, dup(scaleE));
       ie = mk2(fmax(ie.x, Real(0)), fmax(ie.y, Real(0)));
-      const R2 se = lookup(ie, ebase, estride, oa, ob);
+      const R2 se = lookup(ie, ebase, ebase, estride, oa, ob);
       const Real* ea = reinterpret_cast<const Real*>(smem_raw + oa);
       const Real* eb = reinterpret_cast<const Real*>(smem_raw + ob);
 #pragma unroll
@@ -418,22 +375,23 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
       for (int c = 0; c < 3; c++) tot[h][c] = add2(tot[h][c], sum[h][c]);
   }
   if (!valid) return;
-  // J planar, [atmosphere][channel][node], for the ray-scatter gathers
-  const long long n4 = d.n4();
-  Real* Jn = J + (long long)b * 3 * n4 + (node0 - base4);
+  auto put = [&](int at, Real x, Real y, Real z) {
+    Vec4<Real> o;
+    o.x = x;
+    o.y = y;
+    o.z = z;
+    o.w = 0;
+    J[node0 + at] = o;
+  };
 #pragma unroll
-  for (int c = 0; c < 3; c++) {
-    Real* o = Jn + c * n4;
-#pragma unroll
-    for (int h = 0; h < HP; h++) {
-      const int a = a0 + 2 * h;
-      if (a < d.n3 - 1) o[a] = tot[h][c].x;
-      if (a + 1 < d.n3 - 1) o[a + 1] = tot[h][c].y;
-    }
-    if (grp == 0) {
-      o[0] = tot[HP][c].x;
-      o[d.n3 - 1] = tot[HP][c].y;
-    }
+  for (int h = 0; h < HP; h++) {
+    const int a = a0 + 2 * h;
+    if (a < d.n3 - 1) put(a, tot[h][0].x, tot[h][1].x, tot[h][2].x);
+    if (a + 1 < d.n3 - 1) put(a + 1, tot[h][0].y, tot[h][1].y, tot[h][2].y);
+  }
+  if (grp == 0) {
+    put(0, tot[HP][0].x, tot[HP][1].x, tot[HP][2].x);
+    put(d.n3 - 1, tot[HP][0].y, tot[HP][1].y, tot[HP][2].y);
   }
 }
 
@@ -454,7 +412,7 @@ template <class Real>
 int launch_point_scatter(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
                          const SphereRing<Real>* rings, const Real* dirs4, const Real* offsets,
                          const PointRow<Real>* prow, const CellGeom<Real>* geom, const Vec4<Real>* dS, const Vec4<Real>* mie, const Vec4<Real>* dE,
-                         Real* J, cudaStream_t st) {
+                         Vec4<Real>* J, cudaStream_t st) {
   const bool first = mie != nullptr;
   PointLayout lay = point_layout<Real>(d, first, 7);
   if (lay.bytes > 227 * 1024) lay = point_layout<Real>(d, first, 6);
@@ -481,11 +439,11 @@ int launch_point_scatter(const AtmoParams* params, const BuildDims& d, const Row
 
 template int launch_point_scatter<float>(const AtmoParams*, const BuildDims&, const RowInfo*, const SphereRing<float>*,
                                          const float*, const float*, const PointRow<float>*, const CellGeom<float>*,
-                                         const Vec4<float>*, const Vec4<float>*, const Vec4<float>*, float*,
+                                         const Vec4<float>*, const Vec4<float>*, const Vec4<float>*, Vec4<float>*,
                                          cudaStream_t);
 template int launch_point_scatter<double>(const AtmoParams*, const BuildDims&, const RowInfo*,
                                           const SphereRing<double>*, const double*, const double*, const PointRow<double>*,
                                           const CellGeom<double>*, const Vec4<double>*, const Vec4<double>*,
-                                          const Vec4<double>*, double*, cudaStream_t);
+                                          const Vec4<double>*, Vec4<double>*, cudaStream_t);
 
 }  // namespace sfsim

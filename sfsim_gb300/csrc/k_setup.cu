@@ -62,11 +62,11 @@ __global__ void k_row_info(const AtmoParams* params, BuildDims d, RowInfo* info,
 // The height and elevation coordinates of a node are its row's (k_row_info);
 // its light direction l = index-to-sun-direction(v, sin(k), a) has
 // x.l = r sin(k) with x = (r, 0, 0), so its sun-elevation coordinate is the
-// (i, k) one of k_point_rows, which also holds sin(k).
+// (i, k) one of k_point_rows, which also holds sin(k).  Left per node are the
+// sun-angle coordinate and l itself.
 template <class Real>
-__global__ void k_remap4(const AtmoParams* params, BuildDims d, const RowInfo* info, const Remap2<Real>* rowmap,
-                         const PointRow<Real>* prow, const double* __restrict__ hdvs, Remap4<Real>* out,
-                         CellGeom<Real>* geom) {
+__global__ void k_remap4(BuildDims d, const RowInfo* info, const PointRow<Real>* prow,
+                         const double* __restrict__ hdvs, Coord<Real>* angle, CellGeom<Real>* geom) {
   const long long n4 = d.n4();
   const long long node = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
@@ -76,20 +76,13 @@ __global__ void k_remap4(const AtmoParams* params, BuildDims d, const RowInfo* i
   const long long row = node / ((long long)d.n3 * d.n2);
   const int i = (int)(row / d.n1);
   const RowInfo& ri = info[b * d.rows() + row];
-  const Remap2<Real> rm = rowmap[b * d.rows() + row];
   const PointRow<Real>& pk = prow[((long long)b * d.n0 + i) * d.n2 + k];
   const double sv = ri.sv, cv = ri.cv;
   const d3 v = mk3(sv, cv, 0);
   const d3 l = node_light(sv, cv, pk.ss, pk.cs, hdvs[a]);
-  Remap4<Real> m;
-  m.u[0] = rm.u[0];
-  m.s[0] = rm.s[0];
-  m.u[1] = rm.u[1];
-  m.s[1] = rm.s[1];
-  m.u[2] = pk.u2;
-  m.s[2] = pk.s2;
-  split_coord<Real>(sun_angle_to_index(d.n3, v, l), d.n3, &m.u[3], &m.s[3]);
-  out[b * n4 + node] = m;
+  Coord<Real> m;
+  split_coord<Real>(sun_angle_to_index(d.n3, v, l), d.n3, &m.u, &m.s);
+  angle[b * n4 + node] = m;
   geom[b * n4 + node] = cell_geom<Real>(sv, cv, l);
 }
 
@@ -573,8 +566,7 @@ void launch_setup_rows(const AtmoParams* params, const BuildDims& d, const Setup
 template <class Real>
 void launch_node_maps(const AtmoParams* params, const BuildDims& d, const SetupBuffers<Real>& o, cudaStream_t st) {
   const int blk = 128;
-  k_remap4<Real><<<grid1(d.n4(), blk, d.B), blk, 0, st>>>(params, d, o.rowinfo, o.rowmap, o.prow, o.hdvs,
-                                                            o.remapS, o.geom);
+  k_remap4<Real><<<grid1(d.n4(), blk, d.B), blk, 0, st>>>(d, o.rowinfo, o.prow, o.hdvs, o.angle, o.geom);
 }
 
 template <class Real>

@@ -10,7 +10,7 @@ namespace sfsim {
 
 template <class Real>
 struct SetupBuffers {
-  Remap4<Real>* remapS;
+  Coord<Real>* angle;    // [B][n4]: sun-angle coordinate of each node's (v, l); its others are its row's and k's
   CellGeom<Real>* geom;
   Remap2<Real>* remapT;
   Remap2<Real>* remapE;
@@ -31,6 +31,9 @@ struct SetupBuffers {
 // same for every build that runs.
 template <class Real>
 size_t point_scatter_capacity(const BuildDims& d);
+// The same for ray scatter's planes of sun elevations x sun headings.
+template <class Real>
+size_t ray_scatter_capacity(const BuildDims& d);
 
 // The set-up tables in parts: the rows (row info and point rows), then the
 // 4-D node maps with each node's light direction (remap4) and the view-row
@@ -100,13 +103,13 @@ void launch_sfu_probe(int blocks, int threads, int iters, float* sink, cudaStrea
 // reading `iters` x 8 16-byte words.
 int launch_smem_probe(int blocks, int iters, float* sink, cudaStream_t st);
 
-// J = point scatter of (dS, dE), planar [atmosphere][channel][node]; when
+// J = point scatter of (dS, dE) at every node; when
 // `mie` is non-NULL dS is the first iteration's rayleigh + mie * phase(mie, v.l).
 template <class Real>
 int launch_point_scatter(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
                          const SphereRing<Real>* rings, const Real* dirs4, const Real* offsets,
                          const PointRow<Real>* prow, const CellGeom<Real>* geom, const Vec4<Real>* dS, const Vec4<Real>* mie, const Vec4<Real>* dE,
-                         Real* J, cudaStream_t st);
+                         Vec4<Real>* J, cudaStream_t st);
 
 // The ends of every sphere direction at every height, for the work census.
 template <class Real>
@@ -119,16 +122,16 @@ void launch_surface_radiance(const AtmoParams* params, const BuildDims& d, const
                              const HalfDir<Real>* hdir, const Vec4<Real>* dS, const Vec4<Real>* mie,
                              Vec4<Real>* dE, cudaStream_t st);
 
-// dS = ray scatter of J (planar [atmosphere][channel][node]).
+// dS = ray scatter of J.
 template <class Real>
-int launch_ray_scatter(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
-                       const RowSample<Real>* rows, const CellGeom<Real>* geom, const Remap4<Real>* remap,
-                       const Real* J, Vec4<Real>* dS, cudaStream_t st);
+int launch_ray_scatter(const BuildDims& d, const RowInfo* rowinfo, const RowSample<Real>* rows,
+                       const CellGeom<Real>* geom, const Coord<Real>* angle, const Vec4<Real>* J, Vec4<Real>* dS,
+                       cudaStream_t st);
 
 // out = re-interpolation of (a + b) at the node maps; b may be NULL and, for
 // the 2-D variant, a may be NULL.
 template <class Real>
-void launch_accumulate4(const BuildDims& d, const Remap4<Real>* remap, const Vec4<Real>* a, const Vec4<Real>* b,
+void launch_accumulate4(const BuildDims& d, const SetupBuffers<Real>& maps, const Vec4<Real>* a, const Vec4<Real>* b,
                         Vec4<Real>* out, cudaStream_t st);
 
 template <class Real>
@@ -137,7 +140,7 @@ void launch_accumulate2(int B, int n0, int n1, const Remap2<Real>* remap, const 
 
 // Final tables in the .scatter layout (float RGB, 4-D tables tiled 2-D).
 template <class Real>
-void launch_output4(const BuildDims& d, const Remap4<Real>* remap, const Vec4<Real>* tab, float* out,
+void launch_output4(const BuildDims& d, const SetupBuffers<Real>& maps, const Vec4<Real>* tab, float* out,
                     cudaStream_t st);
 
 template <class Real>
@@ -191,14 +194,9 @@ void launch_pack_infer(const __nv_bfloat16* const* W, unsigned char* packed, cud
 // Bytes of the packed weight chunks the inference kernel streams.
 size_t infer_packed_bytes();
 
-// jsum = (first ? 0 : jsum) + J, converted to float; J planar
-// [atmosphere][channel][node] with n4 nodes per atmosphere.
+// jsum = (first ? 0 : jsum) + J, converted to float; n nodes.
 template <class Real>
-void launch_add_to_sum(long long n4, int B, const Real* J, Vec4<float>* jsum, bool first, cudaStream_t st);
-
-// Float [atmosphere][node][channel] copy of a planar table.
-template <class Real>
-void launch_export_planar(long long n4, int B, const Real* tab, float* out, cudaStream_t st);
+void launch_add_to_sum(long long n, const Vec4<Real>* J, Vec4<float>* jsum, bool first, cudaStream_t st);
 
 // Plain-order float copy of an internal table (debug intermediates).
 template <class Real>
