@@ -3,8 +3,11 @@
 // generate-atmosphere-luts (src/clj/sfsim/atmosphere_lut.clj:43-105).
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <atomic>
+#include <cerrno>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -738,6 +741,26 @@ void collect_timings(Timer& tm) {
   g_have_timings = kStages;
 }
 
+// Makes the pages of a host output present and writable, its contents
+// unchanged, while the GPU works on the build.  A copy into pages that are
+// not there yet faults them in one by one: 100 MB of a fresh array took 4.6 ms
+// (and at times, depending on the address, 40 ms of GPU page faults) against
+// 0.56 ms into present pages, and the populating call 3.4 ms, which the build
+// hides.  Below a megabyte the call is not worth its entry.  Best effort: a
+// kernel without MADV_POPULATE_WRITE (before Linux 5.14) or a mapping that
+// refuses it is copied into as it is.
+void populate_host(void* p, size_t bytes) {
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+  if (bytes < (1u << 20)) return;
+  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  const size_t lo = (size_t)p / page * page, hi = ((size_t)p + bytes + page - 1) / page * page;
+  const int saved = errno;
+  (void)madvise((void*)lo, hi - lo, MADV_POPULATE_WRITE);
+  errno = saved;
+}
+
 // Shared driver of all build entry points.  `host_out`: the four output
 // pointers are host memory (copied back and synchronised); otherwise device
 // memory on `user_stream`.
@@ -815,6 +838,9 @@ int build_impl(const sfsim_atmo_config* cfgs, int B, float* T, float* E, float* 
     // whole build is queued first, so a copy into pageable memory, which
     // blocks the host, cannot hold back the launches)
     cudaStream_t cs = g_copy_stream[dev];
+    populate_host(M, sizeof(float) * 3 * B * d.n4());
+    populate_host(T, sizeof(float) * 3 * B * d.nT());
+    populate_host(S, sizeof(float) * 3 * B * d.n4());
     CUDA_TRY(cudaStreamWaitEvent(cs, g_early_done[dev], 0));
     CUDA_TRY(cudaMemcpyAsync(T, w.oT, sizeof(float) * 3 * B * d.nT(), cudaMemcpyDeviceToHost, cs));
     CUDA_TRY(cudaMemcpyAsync(M, w.oM, sizeof(float) * 3 * B * d.n4(), cudaMemcpyDeviceToHost, cs));
