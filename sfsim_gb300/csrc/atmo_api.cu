@@ -257,24 +257,6 @@ int make_params(const sfsim_atmo_config& c, AtmoParams& P) {
   P.f_mie_g = (float)P.mie_g;
   P.f_top = (float)P.top;
   P.f_Hh = (float)P.Hh;
-  P.f_H = (float)P.H;
-  // the descending sun rays' distance to their perigee is tabulated in
-  // asinh(d / s): about linear within s of the perigee, where the Mie density
-  // peak lies (it spans sqrt(2 R H_mie)), logarithmic beyond
-  P.f_desc_s = (float)(1.2 * std::sqrt(2.0 * P.R * P.mie_scale));
-  P.f_desc_inv_s = 1.0f / P.f_desc_s;
-  // Near the top of the climbing sun-ray table the sums fall to zero like
-  // sqrt(q_top - q), which bilinear interpolation follows badly: a numpy model
-  // put the optical-depth error of the last row at about 0.18 times the
-  // Rayleigh density at the top relative to the ground (2.2e-3 in a 35 km
-  // atmosphere), 1e-5 eight rows down.  Where that density exceeds 2e-5 the
-  // rays starting in the top eight rows are integrated directly; elsewhere
-  // (the 100 km atmospheres) the whole table is read.
-  {
-    const double top_density = std::exp(-P.H / P.ray_scale);
-    const double x = (double)(kSunNR - 9) / (double)(kSunNR - 1);
-    P.f_sun_qlim = top_density > 2e-5 ? (float)(P.Hh2 * x * x) : 3.0e38f;
-  }
   const double gs[2] = {P.ray_g, P.mie_g};
   for (int m = 0; m < 2; m++) {
     const double g = gs[m];
@@ -308,6 +290,7 @@ BuildDims make_dims(const sfsim_atmo_config& c, int B) {
   d.S = c.ray_steps;
   d.sphere_steps = c.sphere_steps;
   d.iterations = c.iterations;
+  d.sun_segs = 0;
   d.scan_rays = (c.flags & SFSIM_ATMO_SCAN_RAYS) ? 1 : 0;
   d.inv_S = 1.0 / c.ray_steps;
   std::vector<DirLocal> v;
@@ -378,18 +361,42 @@ struct Work {
   Vec4<Real>*T, *E0, *dE[2], *Eacc[2];
   Vec4<Real>*S1R, *M, *J, *dS[2], *Sacc[2];
   float *oT, *oE, *oS, *oM;  // device outputs when the caller passes host buffers
-  unsigned char* sun;        // sun-ray optical-depth tables, kSunTableBytes per atmosphere (FP32 builds), or NULL
+  unsigned char* sun;        // the first order's fitted sun rays (BuildDims::sun_segs > 0), or NULL
 };
 
-// The sun-ray tables cost kSunTableLen nodes of S samples per atmosphere;
-// integrating the lit sun rays directly costs S samples for each lit
-// (node, ray sample) pair, about a third of all pairs.  Small builds (the
-// 8x16x8x4 case) integrate directly, larger ones (the production and sweep
-// tables) read the tables.
-inline bool sun_tables_pay(const BuildDims& d) { return (double)d.n4() * d.S / 3.0 > (double)kSunTableLen; }
+// Segments of the FP32 first order's fitted sun rays, or 0 for integrating
+// every sun ray.
+//  * The log of a ray's mean density varies over sqrt(2 R h) of its length near
+//    the perigee (h the smaller scale height) and the longest ray is
+//    2 sqrt(2 R H); a segment of at most 2.85 of those widths keeps the quintics
+//    within 1e-5 of the optical depth at depth 15 and 1e-8 of the
+//    transmittance (numpy model).
+//  * The sums must resolve the density peak themselves: with fewer than about
+//    2.4 sqrt(H / h) steps they ripple with the samples' positions, which no
+//    smooth fit follows; 3 sqrt(H / h) keeps the ripple below 1e-6.
+//  * The fits cost 6 rays per segment at 8192 heights of each atmosphere and
+//    about 20 us of their own latency, the direct integration one ray for each
+//    lit (node, ray sample) pair, about a third of all pairs.  Measured, whole
+//    builds at 8 segments, fitted / direct: 2.9M pairs 351 / 344 us, 4.9M 400 /
+//    438, 11M 532 / 638, 26M 807 / 1428.
+constexpr double kSunFitPays = 18.0;  // direct rays per segment and height above which the fits are taken
+int sun_fit_segments(const sfsim_atmo_config* cfgs, int B, const BuildDims& d) {
+  if (cfgs[0].precision != SFSIM_ATMO_FP32) return 0;
+  double ratio = 1.0;
+  for (int b = 0; b < B; b++)
+    ratio = std::fmax(ratio, cfgs[b].height / std::fmin(cfgs[b].mie.scatter_scale, cfgs[b].rayleigh.scatter_scale));
+  if (d.S < 3.0 * std::sqrt(ratio)) return 0;
+  int segs = 8;
+  while (segs < 128 && 2.0 * std::sqrt(ratio) > 2.85 * segs) segs *= 2;
+  if (2.0 * std::sqrt(ratio) > 2.85 * segs) return 0;
+  BuildDims f = d;
+  f.sun_segs = segs;
+  if (first_order_fit_smem(f) > kMaxSmem) return 0;
+  return (double)d.n4() * d.S / 3.0 > kSunFitPays * segs * 8192.0 ? segs : 0;
+}
 
 template <class Real>
-size_t carve(Work<Real>& w, char* base, const BuildDims& d, bool outputs, bool sun_table = true) {
+size_t carve(Work<Real>& w, char* base, const BuildDims& d, bool outputs) {
   Carver c{base};
   const long long B = d.B;
   w.params = c.take<AtmoParams>(B);
@@ -430,8 +437,7 @@ size_t carve(Work<Real>& w, char* base, const BuildDims& d, bool outputs, bool s
   } else {
     w.oT = w.oE = w.oS = w.oM = nullptr;
   }
-  w.sun = (sun_table && sizeof(Real) == sizeof(float) && sun_tables_pay(d)) ? c.take<unsigned char>(B * kSunTableBytes)
-                                                                             : nullptr;
+  w.sun = d.sun_segs > 0 ? c.take<unsigned char>(B * sun_fit_bytes(d.sun_segs)) : nullptr;
   return c.off + 256;
 }
 
@@ -541,14 +547,14 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
   // in shared memory keep the node maps before the first order.
   cudaStream_t ss = tm.side ? g_side_stream[tm.dev] : nullptr;
   const bool setup_fork = ss != nullptr && !g_timing;
-  const bool cells = setup_fork && first_order_smem<Real>(d, true) <= kMaxSmem;
+  const bool cells = setup_fork && (w.sun || first_order_smem<Real>(d, true) <= kMaxSmem);
   cudaStream_t sa = setup_fork ? ss : st;
   if (setup_fork) {
     CUDA_TRY(cudaEventRecord(g_side_fork[tm.dev], st));
     CUDA_TRY(cudaStreamWaitEvent(ss, g_side_fork[tm.dev], 0));
     if (w.sun) {
       tm.mark_begin(3, ss);
-      launch_sun_table(w.params, d, w.sun, ss);
+      launch_sun_fit(w.params, d, w.sun, ss);
       launches++;
       tm.mark_end(ss);
     }
@@ -578,11 +584,19 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
   }
   tm.mark_begin(3);
   if (w.sun && !setup_fork) {
-    launch_sun_table(w.params, d, w.sun, st);
+    launch_sun_fit(w.params, d, w.sun, st);
     launches++;
   }
-  if (launch_first_order<Real>(w.params, d, w.setup.rowinfo, w.setup.rows, cells ? nullptr : w.setup.geom,
-                               w.setup.prow, w.setup.hdvs, w.sun, w.S1R, w.M, st))
+  int first = 0;
+  if constexpr (sizeof(Real) == sizeof(float)) {
+    if (w.sun)
+      first = launch_first_order_fit(w.params, d, w.setup.rowinfo, w.setup.rows, w.setup.prow, w.setup.hdvs, w.sun,
+                                     w.S1R, w.M, st);
+  }
+  if (!w.sun)
+    first = launch_first_order<Real>(w.params, d, w.setup.rowinfo, w.setup.rows, cells ? nullptr : w.setup.geom,
+                                     w.setup.prow, w.setup.hdvs, w.S1R, w.M, st);
+  if (first)
     return fail(SFSIM_ATMO_ECUDA, "first order launch configuration failed");
   launches++;
   tm.mark_end();
@@ -780,6 +794,7 @@ int build_impl(const sfsim_atmo_config* cfgs, int B, float* T, float* E, float* 
   sphere_directions(cfgs[0].sphere_steps >> 1, cfgs[0].sphere_steps, M_PI, dirs);
   sphere_directions(cfgs[0].ray_steps >> 2, cfgs[0].ray_steps, M_PI / 2, hdirs);
 
+  d.sun_segs = sun_fit_segments(cfgs, B, d);
   Work<Real> w;
   size_t bytes = carve<Real>(w, nullptr, d, host_out);
   if ((rc = ensure_arena(dev, bytes))) return rc;
@@ -887,11 +902,11 @@ int census_impl(const sfsim_atmo_config& cfg, unsigned long long* out, int n) {
   std::vector<DirLocal> dirs;
   sphere_directions(cfg.sphere_steps >> 1, cfg.sphere_steps, M_PI, dirs);
   Work<Real> w;
-  size_t bytes = carve<Real>(w, nullptr, d, false, false);
+  size_t bytes = carve<Real>(w, nullptr, d, false);
   const size_t sdirs_at = (bytes + 255) & ~size_t(255), nsd = (size_t)d.n0 * (d.P + 1);
   const size_t count_at = (sdirs_at + sizeof(SphereDir<Real>) * nsd + 255) & ~size_t(255);
   if ((rc = ensure_arena(dev, count_at + 256))) return rc;
-  carve<Real>(w, (char*)g_arena[dev].base, d, false, false);
+  carve<Real>(w, (char*)g_arena[dev].base, d, false);
   SphereDir<Real>* dsd = reinterpret_cast<SphereDir<Real>*>((char*)g_arena[dev].base + sdirs_at);
   unsigned long long* dcount = reinterpret_cast<unsigned long long*>((char*)g_arena[dev].base + count_at);
   cudaStream_t st = g_stream[dev];
@@ -1204,6 +1219,7 @@ int context_build(sfsim_atmo_context* c) {
   std::vector<DirLocal> dirs, hdirs;
   sphere_directions(cfg.sphere_steps >> 1, cfg.sphere_steps, M_PI, dirs);
   sphere_directions(cfg.ray_steps >> 2, cfg.ray_steps, M_PI / 2, hdirs);
+  d.sun_segs = sun_fit_segments(&cfg, 1, d);
   Work<Real> w;
   const size_t wbytes = carve<Real>(w, nullptr, d, true);
   const size_t total = wbytes + sizeof(Vec4<float>) * (size_t)d.n4() + 256;
@@ -1617,7 +1633,7 @@ int build_static_impl(const sfsim_atmo_config& cfg, float* T, float* E, float* S
   BuildDims d = make_dims(cfg, 1);
   if ((rc = check_smem<Real>(d))) return rc;
   Work<Real> w;
-  const size_t bytes = carve<Real>(w, nullptr, d, false, false);
+  const size_t bytes = carve<Real>(w, nullptr, d, false);
   const size_t counted = bytes + static_margin<Real>(d);
   if (counted > kStaticScratchBytes)
     return fail(SFSIM_ATMO_ETOOBIG, "the build needs " + std::to_string(counted) +
@@ -1629,7 +1645,10 @@ int build_static_impl(const sfsim_atmo_config& cfg, float* T, float* E, float* S
   sphere_directions(cfg.ray_steps >> 2, cfg.ray_steps, M_PI / 2, hdirs);
   void* base = nullptr;
   if ((rc = static_scratch_base(dev, &base))) return rc;
-  carve<Real>(w, (char*)base, d, false, false);
+  // the fitted sun rays where they fit as well, else every sun ray is integrated
+  d.sun_segs = sun_fit_segments(&cfg, 1, d);
+  if (carve<Real>(w, nullptr, d, false) > kStaticScratchBytes) d.sun_segs = 0;
+  carve<Real>(w, (char*)base, d, false);
   // every scratch table is written before it is read, so nothing is cleared;
   // parameters and quadrature directions are copied in on the caller's stream
   g_h2d_bytes = sizeof(AtmoParams) + sizeof(DirLocal) * (dirs.size() + hdirs.size());
@@ -1679,6 +1698,7 @@ int plan_prepare(sfsim_atmo_plan* p, Work<Real>& w) {
   std::vector<DirLocal> dirs, hdirs;
   sphere_directions(cfg.sphere_steps >> 1, cfg.sphere_steps, M_PI, dirs);
   sphere_directions(cfg.ray_steps >> 2, cfg.ray_steps, M_PI / 2, hdirs);
+  d.sun_segs = sun_fit_segments(&cfg, 1, d);
   const size_t bytes = carve<Real>(w, nullptr, d, false);
   cudaError_t e = cudaMalloc(&p->mem, bytes);
   if (e != cudaSuccess) {

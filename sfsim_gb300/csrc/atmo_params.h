@@ -52,12 +52,6 @@ struct AtmoParams {
   double d_srcR[3], d_srcM[3];
   float f_srcR[3], f_srcM[3];
   float f_top, f_Hh;
-  // descending sun-ray table of the FP32 first order: atmosphere height and
-  // the distance scale s of its asinh coordinate (and 1 / s)
-  float f_H, f_desc_s, f_desc_inv_s;
-  // climbing sun rays from q >= f_sun_qlim are integrated directly (the top
-  // rows of the climbing table where the density at the top matters)
-  float f_sun_qlim;
   int hpoly_n;                        // number of coefficients
 };
 
@@ -73,6 +67,7 @@ struct BuildDims {
   int T;                   // their rings
   int Ph;                  // directions of integral-half-sphere(ray_steps)
   int iterations;
+  int sun_segs;            // segments of the fitted sun rays (FP32 first order), 0: integrated directly
   double inv_S;            // 1 / S, the view rays' step in their parameter
   int scan_rays;           // view-ray transmittances by prefix scan (SFSIM_ATMO_SCAN_RAYS)
   // (size - 1) / (1 - exp(-3.6)) of the sun-elevation axes of the ray-scatter

@@ -70,27 +70,19 @@ size_t first_order_smem(const BuildDims& d, bool cells);
 template <class Real>
 int launch_first_order(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
                        const RowSample<Real>* rows, const CellGeom<Real>* geom, const PointRow<Real>* prow,
-                       const double* hdvs, const unsigned char* sun_table, Vec4<Real>* rayleigh, Vec4<Real>* mie,
-                       cudaStream_t st);
+                       const double* hdvs, Vec4<Real>* rayleigh, Vec4<Real>* mie, cudaStream_t st);
 
-// Sun-ray optical-depth tables of the FP32 first order, per atmosphere: the
-// climbing rays' kSunNR x kSunNM float2, then the descending rays' kDescNX x
-// kDescNY float2 (see k_first_order.cu).
-constexpr int kSunNR = 2048;
-constexpr int kSunNM = 2048;
-constexpr int kDescNX = 1024;
-constexpr int kDescNY = 2048;
-constexpr long long kSunTableLen = (long long)kSunNR * kSunNM + (long long)kDescNX * kDescNY;
-// Bytes of the tables per atmosphere: the climbing table's rows, then the
-// descending table's.  A table of paired texels holds (v(j), v(j + 1)) per
-// entry, 16 bytes; otherwise v(j), 8 bytes.  Pairing the climbing table
-// (most lookups) halves its L1 sectors; pairing the descending one too made
-// the tables (96 MB) spill from L2 and gained nothing.
-constexpr bool kSunPairClimb = true, kSunPairDesc = false;
-constexpr size_t kSunClimbBytes = (size_t)kSunNR * kSunNM * (kSunPairClimb ? 16 : 8);
-constexpr size_t kSunDescBytes = (size_t)kDescNX * kDescNY * (kSunPairDesc ? 16 : 8);
-constexpr size_t kSunTableBytes = kSunClimbBytes + kSunDescBytes;
-void launch_sun_table(const AtmoParams* params, const BuildDims& d, unsigned char* table, cudaStream_t st);
+// The FP32 first order with fitted sun rays (k_first_order_fit.cu): bytes of
+// the fits of one atmosphere with `segs` segments, the fits, and the first
+// order that reads them (its blocks form their cells' light directions
+// themselves).  BuildDims::sun_segs says how many segments, 0 for the direct
+// integration of launch_first_order.
+size_t sun_fit_bytes(int segs);
+void launch_sun_fit(const AtmoParams* params, const BuildDims& d, unsigned char* table, cudaStream_t st);
+size_t first_order_fit_smem(const BuildDims& d);
+int launch_first_order_fit(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
+                           const RowSample<float>* rows, const PointRow<float>* prow, const double* hdvs,
+                           const unsigned char* table, Vec4<float>* rayleigh, Vec4<float>* mie, cudaStream_t st);
 
 template <class Real>
 void launch_first_order_census(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
