@@ -299,6 +299,8 @@ BuildDims make_dims(const sfsim_atmo_config& c, int B) {
   d.T = d.P > 0 ? c.sphere_steps >> 1 : 0;
   sphere_directions(c.ray_steps >> 2, c.ray_steps, M_PI / 2, v);
   d.Ph = (int)v.size();
+  d.Th = d.Ph > 0 ? c.ray_steps >> 2 : 0;
+  d.half_slab = d.nE1;
   d.sun_scale = (d.n2 - 1) / (1 - std::exp(-3.6));
   d.sun_scale_E = (d.nE1 - 1) / (1 - std::exp(-3.6));
   d.f_sun_scale = (float)d.sun_scale;
@@ -415,7 +417,10 @@ size_t carve(Work<Real>& w, char* base, const BuildDims& d, bool outputs) {
   w.setup.prow = c.take<PointRow<Real>>(B * d.n0 * d.n2);
   w.setup.hdvs = c.take<double>(d.n3);
   w.setup.erow = c.take<SurfRow<Real>>(B * d.nE());
-  w.setup.hdir = c.take<HalfDir<Real>>(B * d.nE0 * (long long)d.Ph);
+  w.setup.half_rings = c.take<HalfRing<Real>>(d.Th + 1);
+  w.setup.half_y = c.take<Real>(d.Ph);
+  w.setup.half_rows = c.take<Coord<Real>>(B * d.nE0 * (long long)d.Th);
+  w.setup.half_weights = c.take<HalfWeight<Real>>(B * d.half_slab * (long long)d.Th * d.n3);
   w.T = c.take<Vec4<Real>>(B * d.nT());
   w.E0 = c.take<Vec4<Real>>(B * d.nE());
   for (int i = 0; i < 2; i++) {
@@ -672,8 +677,7 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
       CUDA_TRY(cudaStreamWaitEvent(ss, g_side_fork[tm.dev], 0));
     }
     tm.mark_begin(6, ss);
-    launch_surface_radiance<Real>(w.params, d, w.setup.erow, w.setup.hdir, dS_prev, M_first, dE_new, ss);
-    launches++;
+    launches += launch_surface_radiance<Real>(w.params, d, w.setup, dS_prev, M_first, dE_new, ss);
     tm.mark_end(ss);
     if (fork) CUDA_TRY(cudaEventRecord(g_side_sr[tm.dev], ss));
     tm.mark_begin(5);
@@ -1608,21 +1612,25 @@ int static_scratch_base(int dev, void** base) {
 
 // What the static array's limit counts beside the scratch tables: tables that
 // the build no longer keeps (point scatter's rows per (height, sun elevation)
-// pair and its direction lists, four coordinates per node) less those that
-// took their place.  They stay in the count so that the configurations the
+// pair and its direction lists, four coordinates per node, surface radiance's
+// directions per height; 1024 bytes of parameters) less those that took their
+// place.  They stay in the count so that the configurations the
 // entry point accepts stay the same.
 template <class Real>
-size_t static_margin(const BuildDims& d) {
+long long static_margin(const BuildDims& d) {
   auto up = [](long long x) { return (long long)((x + 255) & ~255LL); };
   const long long n = d.P + 16, n8 = (n + 7) / 8 * 8, R = sizeof(Real), n4 = d.n4(), pairs = (long long)d.n0 * d.n2;
-  const long long gone = up(sizeof(SphereDir<Real>) * d.n0 * (d.P + 1LL)) + up(sizeof(SphereDir<Real>) * d.n0 * n) +
+  const long long gone = 1024 + up(sizeof(SphereDir<Real>) * d.n0 * (d.P + 1LL)) + up(sizeof(SphereDir<Real>) * d.n0 * n) +
                          up(d.n0 * ((n8 * (9 * R + 4) + 15) & ~15LL)) + up(sizeof(int2) * d.n0) +
                          up(R * pairs * 2 * n8 * (d.n3 + 2) * 3) + up(4 * (sizeof(int) + R) * n4) + up(3 * R * n4) +
-                         up((R == 8 ? 96 : 64) * pairs);
-  const long long kept = up(sizeof(SphereRing<Real>) * d.n0 * (d.T + 1LL)) + up(R * 4 * (d.P + 1LL)) +
+                         up((R == 8 ? 96 : 64) * pairs) + up(R * 3LL * d.nE0 * d.Ph) + up((8 + 7 * R) * d.nE());
+  const long long kept = up(sizeof(AtmoParams)) + up(sizeof(SphereRing<Real>) * d.n0 * (d.T + 1LL)) + up(R * 4 * (d.P + 1LL)) +
                          up(R == 8 ? R * d.n0 * d.P : 0) + up(sizeof(Coord<Real>) * n4) + up(sizeof(Vec4<Real>) * n4) +
-                         up(sizeof(PointRow<Real>) * pairs);
-  return gone > kept ? (size_t)(gone - kept) : 0;
+                         up(sizeof(PointRow<Real>) * pairs) + up(sizeof(HalfRing<Real>) * (d.Th + 1LL)) +
+                         up(R * (long long)d.Ph) + up(sizeof(Coord<Real>) * d.nE0 * d.Th) +
+                         up(sizeof(HalfWeight<Real>) * d.half_slab * d.Th * (long long)d.n3) +
+                         up(sizeof(SurfRow<Real>) * d.nE());
+  return gone - kept;
 }
 
 template <class Real>
@@ -1648,6 +1656,11 @@ int build_static_impl(const sfsim_atmo_config& cfg, float* T, float* E, float* S
   // the fitted sun rays where they fit as well, else every sun ray is integrated
   d.sun_segs = sun_fit_segments(&cfg, 1, d);
   if (carve<Real>(w, nullptr, d, false) > kStaticScratchBytes) d.sun_segs = 0;
+  // and the surface-radiance weights of as many lights at a time as fit: the
+  // count above has more room than one light's (directions per height, four
+  // coordinates per node)
+  while (d.half_slab > 1 && carve<Real>(w, nullptr, d, false) > kStaticScratchBytes)
+    d.half_slab = (d.half_slab + 1) / 2;
   carve<Real>(w, (char*)base, d, false);
   // every scratch table is written before it is read, so nothing is cleared;
   // parameters and quadrature directions are copied in on the caller's stream

@@ -787,6 +787,41 @@ __device__ inline void interp4(const Vec4<Real>* t, const BuildDims& d, const in
   mix3(rh[0], rh[1], s[0], out);
 }
 
+// Texel a of a 4-D table's row along the sun angle at height (u0, s0),
+// elevation (u1, s1) and sun elevation (u2, s2); a corner whose height or sun
+// elevation weight is exactly 0 is not loaded (mix3(x, y, 0) = x exactly).
+template <class Real>
+__device__ __forceinline__ void gather_row_texel(const Vec4<Real>* t, const BuildDims& d, int u0, Real s0, int u1,
+                                                 Real s1, int u2, Real s2, int a, Real* dst) {
+  const int v0 = upper_index(u0, d.n0), v1 = upper_index(u1, d.n1), v2 = upper_index(u2, d.n2);
+  auto pair = [&](int h, int e, Real* out) {  // mixed over the sun elevation
+    Real A[3], B[3];
+    ld3(t, idx4(d, h, e, u2, a), A);
+    if (s2 != Real(0)) {
+      ld3(t, idx4(d, h, e, v2, a), B);
+      mix3(A, B, s2, out);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; c++) out[c] = A[c];
+    }
+  };
+  auto row = [&](int e, Real* out) {  // mixed over the height
+    Real lo[3], hi[3];
+    pair(u0, e, lo);
+    if (s0 != Real(0)) {
+      pair(v0, e, hi);
+      mix3(lo, hi, s0, out);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; c++) out[c] = lo[c];
+    }
+  };
+  Real e0[3], e1[3];
+  row(u1, e0);
+  row(v1, e1);
+  mix3(e0, e1, s1, dst);
+}
+
 template <class Real>
 __device__ inline void interp2(const Vec4<Real>* t, int n0, int n1, const int* u, const Real* s, Real out[3]) {
   const int v0 = upper_index(u[0], n0), v1 = upper_index(u[1], n1);

@@ -66,6 +66,8 @@ struct BuildDims {
   int P;                   // directions of integral-sphere(sphere_steps)
   int T;                   // their rings
   int Ph;                  // directions of integral-half-sphere(ray_steps)
+  int Th;                  // their rings
+  int half_slab;           // lights (of nE1) whose surface-radiance weights are kept at a time
   int iterations;
   int sun_segs;            // segments of the fitted sun rays (FP32 first order), 0: integrated directly
   double inv_S;            // 1 / S, the view rays' step in their parameter
@@ -145,22 +147,30 @@ struct PointRow {
 };
 
 // Per node (height iE, sun elevation kE) of the surface-radiance space, from
-// FP64: the dS lookup's height and sun-elevation coordinates at x = (r, 0, 0)
-// and the terms of the elevation coordinate of (x, w) (atmosphere.clj:239-253):
-// H^2 - q, 2 rho + 2 H, r; and the light direction (lx, ly, 0).
+// FP64: the height and sun-elevation coordinates of its dS lookups at
+// x = (r, 0, 0), and its light direction (lx, ly, 0).
 template <class Real>
 struct SurfRow {
   int u0, u2;
   Real s0, s2;
-  Real Hh2mq, den, rr, lx, ly;
+  Real lx, ly;
 };
 
-// A direction of the surface-radiance half-sphere integral in world
-// coordinates at the height of row iE: its first two components and its
-// quadrature weight times w.n.
+// A ring of the surface-radiance half sphere: its first direction, the first
+// component of its directions (the normal is the first axis) and their
+// quadrature weight times that component (w.n).
 template <class Real>
-struct HalfDir {
-  Real wx, wy, wgt;
+struct HalfRing {
+  int w0;
+  Real x0, weight;
+};
+
+// What the directions of a ring add up to at one texel of the ring's row
+// along the sun angle, for one light: interpolation weight times quadrature
+// weight, and the same with the Mie phase of the direction.
+template <class Real>
+struct alignas(2 * sizeof(Real)) HalfWeight {
+  Real ray, mie;
 };
 
 // Per view row and ray sample s (p_s = x + D (s + 1/2)/S).

@@ -80,41 +80,6 @@ __host__ __device__ inline PointLayout point_layout(const BuildDims& d, bool fir
   return l;
 }
 
-// dS (or the Mie strength) at texel a of a ring's row: height and sun
-// elevation of the pair, elevation of the ring; a corner whose weight is
-// exactly 0 is not loaded (mix3(x, y, 0) = x exactly).
-template <class Real>
-__device__ __forceinline__ void gather_row_texel(const Vec4<Real>* t, const BuildDims& d, int u0, Real s0, int u1,
-                                                 Real s1, int u2, Real s2, int a, Real* dst) {
-  const int v0 = upper_index(u0, d.n0), v1 = upper_index(u1, d.n1), v2 = upper_index(u2, d.n2);
-  auto pair = [&](int h, int e, Real* out) {  // mixed over the sun elevation
-    Real A[3], B[3];
-    ld3(t, idx4(d, h, e, u2, a), A);
-    if (s2 != Real(0)) {
-      ld3(t, idx4(d, h, e, v2, a), B);
-      mix3(A, B, s2, out);
-    } else {
-#pragma unroll
-      for (int c = 0; c < 3; c++) out[c] = A[c];
-    }
-  };
-  auto row = [&](int e, Real* out) {  // mixed over the height
-    Real lo[3], hi[3];
-    pair(u0, e, lo);
-    if (s0 != Real(0)) {
-      pair(v0, e, hi);
-      mix3(lo, hi, s0, out);
-    } else {
-#pragma unroll
-      for (int c = 0; c < 3; c++) out[c] = lo[c];
-    }
-  };
-  Real e0[3], e1[3];
-  row(u1, e0);
-  row(v1, e1);
-  mix3(e0, e1, s1, dst);
-}
-
 constexpr int kPointThreads = 128;
 
 // Blocks per SM the registers are limited for.  Three heading pairs measured

@@ -1,130 +1,11 @@
-// k_scatter.cu -- multiple-scattering passes of the atmosphere LUT build
-// (atmosphere_lut.clj:86-97): surface radiance dE and the re-interpolating
-// accumulation of E and S.
+// k_scatter.cu -- the re-interpolating accumulation of E and S in the
+// multiple-scattering iterations (atmosphere_lut.clj:86-97) and the outputs.
 #include <cstddef>
-#include <type_traits>
 
 #include "atmo_device.cuh"
 #include "kernels.h"
 
 namespace sfsim {
-
-// Threads per surface-radiance node: 128 lets about seven blocks share an
-// SM, so the 1024 nodes of the production tables run in about one wave.
-constexpr int kSurfaceThreads = 128;
-
-// ---------------------------------------------------------------------------
-// Surface radiance dE (atmosphere.clj:225-230): integral over the upper half
-// sphere of dS(x, w, l, above) (w.n); the reference passes the ray steps as
-// the sphere steps (atmosphere_lut.clj:89).  One block per node, threads over
-// directions, block reduction.  The per-node coordinates and the world-space
-// directions come from FP64 setup tables, so no thread uses the FP64 pipe.
-// ---------------------------------------------------------------------------
-
-template <class Real, bool FIRST>
-__global__ void __launch_bounds__(kSurfaceThreads) k_surface_radiance(const AtmoParams* params, BuildDims d,
-                                                          const SurfRow<Real>* erow, const HalfDir<Real>* hdir,
-                                                          const Vec4<Real>* dS, const Vec4<Real>* Mt,
-                                                          Vec4<Real>* dE) {
-  __shared__ Real red[3][kSurfaceThreads];
-  const int b = blockIdx.y;
-  const long long node = blockIdx.x;
-  const AtmoParams& P = params[b];
-  const int iE = (int)(node / d.nE1);
-  // per node, from FP64 (k_surface_rows): x = (r, 0, 0), l = (lx, ly, 0) and
-  // the height and sun-elevation coordinates shared by every direction
-  const SurfRow<Real> er = erow[(long long)b * d.nE() + node];
-  int u[4] = {er.u0, 0, er.u2, 0};
-  Real s[4] = {er.s0, 0, er.s2, 0};
-  // elevation coordinate of (x, w, above) (atmosphere.clj:239-253) in Real:
-  // r sin_el = x.w, rho^2 = q, Delta + H^2 = (x.w)^2 + (H^2 - q) with both
-  // terms non-negative, and r sin_el - sqrt(Delta + H^2) rewritten without
-  // cancellation when x.w > 0
-  const Real Hh2mq = er.Hh2mq, den = er.den, rr = er.rr, lx = er.lx, ly = er.ly;
-  const Real scale1 = Real(d.n1 - 1), scale3 = Real(0.5) * Real(d.n3 - 1);
-  const Vec4<Real>* tS = dS + (long long)b * d.n4();
-  const Vec4<Real>* tM = FIRST ? Mt + (long long)b * d.n4() : nullptr;
-  const HalfDir<Real>* hd = hdir + ((long long)b * d.nE0 + iE) * d.Ph;
-  const PhaseCS<Real> phase_mie(Bulk<Real>::phase_mie(P));
-  Real acc[3] = {0, 0, 0}, cmp[3] = {0, 0, 0};
-  for (int w = threadIdx.x; w < d.Ph; w += blockDim.x) {
-    const HalfDir<Real> qd = hd[w];
-    const Real wx = qd.wx, wy = qd.wy;
-    const Real pv = rr * wx;
-    const Real root = Bulk<Real>::sqrt(fma(pv, pv, Hh2mq));
-    const Real a = pv > Real(0) ? -Hh2mq / (pv + root) : pv - root;
-    int uu[4] = {u[0], 0, u[2], 0};
-    Real sx[4] = {s[0], 0, s[2], 0};
-    Real lq;
-    {
-      // limit-quot (util.clj:403-420) with limits -0.5, 0
-      Real aa = a, bb = den;
-      if (aa == Real(0)) lq = Real(0);
-      else {
-        if (bb < Real(0)) { aa = -aa; bb = -bb; }
-        lq = aa < Real(0) ? (aa > bb * Real(-0.5) ? aa / bb : Real(-0.5)) : Real(0);
-      }
-    }
-    {
-      // (n1 - 1)(1/2 - lq) with the exact base (n1 - 1)/2 split off: the
-      // fraction keeps the precision of the part above it, -(n1 - 1) lq,
-      // which is small for the rays near the horizon that carry the most
-      // light (in FP32 the whole coordinate near n1/2 resolves only ~1e-5 of
-      // a texel there, and the table is steep)
-      const Real t = ((d.n1 - 1) & 1 ? Real(0.5) : Real(0)) - scale1 * lq;
-      const Real ft = floor(t);
-      uu[1] = ((d.n1 - 1) >> 1) + (int)ft;
-      sx[1] = t - ft;
-      if (uu[1] >= d.n1 - 1) {
-        uu[1] = d.n1 - 1;
-        sx[1] = Real(0);
-      }
-    }
-    const Real mu = fma(wx, lx, wy * ly);  // w.l, l.z = 0
-    split_coord_r<Real>(scale3 * (Real(1) + mu), d.n3, &uu[3], &sx[3]);
-    Real val[3];
-    interp4(tS, d, uu, sx, val);
-    if (FIRST) {
-      Real vm[3];
-      interp4(tM, d, uu, sx, vm);
-      const Real ph = phase_mie(mu);
-#pragma unroll
-      for (int c = 0; c < 3; c++) val[c] = fma(vm[c], ph, val[c]);
-    }
-    const Real wgt = qd.wgt;
-#pragma unroll
-    for (int c = 0; c < 3; c++) kahan_add(acc[c], cmp[c], val[c] * wgt);
-  }
-#pragma unroll
-  for (int c = 0; c < 3; c++) red[c][threadIdx.x] = acc[c];
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-#pragma unroll
-      for (int c = 0; c < 3; c++) red[c][threadIdx.x] += red[c][threadIdx.x + o];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    Vec4<Real> o;
-    o.x = red[0][0];
-    o.y = red[1][0];
-    o.z = red[2][0];
-    o.w = 0;
-    dE[(long long)b * d.nE() + node] = o;
-  }
-}
-
-template <class Real>
-void launch_surface_radiance(const AtmoParams* params, const BuildDims& d, const SurfRow<Real>* erow,
-                             const HalfDir<Real>* hdir, const Vec4<Real>* dS, const Vec4<Real>* mie,
-                             Vec4<Real>* dE, cudaStream_t st) {
-  dim3 grid((unsigned)d.nE(), d.B);
-  if (mie)
-    k_surface_radiance<Real, true><<<grid, kSurfaceThreads, 0, st>>>(params, d, erow, hdir, dS, mie, dE);
-  else
-    k_surface_radiance<Real, false><<<grid, kSurfaceThreads, 0, st>>>(params, d, erow, hdir, dS, mie, dE);
-}
 
 // ---------------------------------------------------------------------------
 // Re-interpolating accumulation and outputs
@@ -290,9 +171,6 @@ void launch_export(long long n, const Vec4<Real>* tab, float* out, cudaStream_t 
 }
 
 #define SFSIM_INSTANTIATE(Real)                                                                                     \
-  template void launch_surface_radiance<Real>(const AtmoParams*, const BuildDims&, const SurfRow<Real>*,          \
-                                              const HalfDir<Real>*, const Vec4<Real>*, const Vec4<Real>*,          \
-                                              Vec4<Real>*, cudaStream_t);                                          \
   template void launch_accumulate4<Real>(const BuildDims&, const SetupBuffers<Real>&, const Vec4<Real>*,           \
                                          const Vec4<Real>*, Vec4<Real>*, cudaStream_t);                            \
   template void launch_accumulate2<Real>(int, int, int, const Remap2<Real>*, const Vec4<Real>*, const Vec4<Real>*, \

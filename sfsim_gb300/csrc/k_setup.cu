@@ -502,54 +502,6 @@ __global__ void k_point_rows(const AtmoParams* params, BuildDims d, PointRow<Rea
   out[(long long)b * d.n0 * d.n2 + t] = o;
 }
 
-// Surface-radiance constants per node (iE, kE), in FP64 as the per-node part
-// of k_surface_radiance needs them (atmosphere.clj:225-230, 239-253).
-template <class Real>
-__global__ void k_surface_rows(const AtmoParams* params, BuildDims d, SurfRow<Real>* out) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const int b = blockIdx.y;
-  if (t >= d.nE()) return;
-  const AtmoParams& P = params[b];
-  const int iE = (int)(t / d.nE1), kE = (int)(t % d.nE1);
-  const double r = index_to_radius(P, d.nE0, (double)iE);
-  const double ss = index_to_sin_sun_elevation(d.nE1, (double)kE);
-  const d3 x = mk3(r, 0, 0), l = mk3(ss, sqrt(dmax(0.0, 1 - sqr(ss))), 0);
-  SurfRow<Real> o;
-  split_coord<Real>(height_to_index(P, d.n0, mag3(x)), d.n0, &o.u0, &o.s0);
-  split_coord<Real>(sun_elevation_to_index(d.n2, x, l), d.n2, &o.u2, &o.s2);
-  const double c0 = dmul(dsub(r, P.R), dadd(r, P.R));  // |x|^2 - R^2
-  const Real rho = (Real)sqrt(dmax(0.0, c0));
-  o.Hh2mq = (Real)dsub(P.Hh2, c0);
-  o.den = rho + rho + Real(2) * (Real)P.Hh;
-  o.rr = (Real)r;
-  o.lx = (Real)l.x;
-  o.ly = (Real)l.y;
-  out[(long long)b * d.nE() + t] = o;
-}
-
-// The half-sphere directions of surface radiance in world coordinates at
-// the height of row iE (x = (r, 0, 0), the frame of integral-half-sphere).
-template <class Real>
-__global__ void k_half_dirs(const AtmoParams* params, BuildDims d, const DirLocal* hdirs, HalfDir<Real>* out) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const int b = blockIdx.y;
-  if (t >= (long long)d.nE0 * d.Ph) return;
-  const AtmoParams& P = params[b];
-  const int iE = (int)(t / d.Ph), w = (int)(t % d.Ph);
-  const double r = index_to_radius(P, d.nE0, (double)iE);
-  const d3 x = mk3(r, 0, 0);
-  const d3 n = mul3(x, 1.0 / mag3(x));
-  const d3 o1 = orthogonal(n);
-  const d3 o2 = cross3(n, o1);
-  const DirLocal qd = hdirs[w];
-  const d3 omega = to_world(n, o1, o2, qd);
-  HalfDir<Real> o;
-  o.wx = (Real)omega.x;
-  o.wy = (Real)omega.y;
-  o.wgt = (Real)(qd.w * dot3(omega, n));
-  out[(long long)b * d.nE0 * d.Ph + t] = o;
-}
-
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
@@ -589,10 +541,7 @@ int launch_setup_aux(const AtmoParams* params, const BuildDims& d, const DirLoca
   if (d.P > 0)
     k_sphere_rings<Real><<<dim3(d.n0, d.B), 256, sizeof(int) * (d.T + 1), st>>>(params, d, dirs, o.rings, o.dirs4,
                                                                                    o.offsets);
-  k_surface_rows<Real><<<grid1(d.nE(), blk, d.B), blk, 0, st>>>(params, d, o.erow);
-  if (d.Ph > 0)
-    k_half_dirs<Real><<<grid1((long long)d.nE0 * d.Ph, blk, d.B), blk, 0, st>>>(params, d, half_dirs, o.hdir);
-  return 3 + (d.P > 0) + (d.Ph > 0);
+  return 2 + (d.P > 0) + launch_surface_rows<Real>(params, d, half_dirs, o, st);
 }
 
 template <class Real>

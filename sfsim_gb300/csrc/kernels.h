@@ -23,7 +23,10 @@ struct SetupBuffers {
   PointRow<Real>* prow;  // [B][n0][n2]
   double* hdvs;          // [n3]: 2 a / (n3 - 1) - 1, index-to-sun-direction's v.l of heading a
   SurfRow<Real>* erow;   // [B][nE0][nE1]
-  HalfDir<Real>* hdir;   // [B][nE0][Ph]
+  HalfRing<Real>* half_rings;      // [Th + 1]: surface radiance's rings, the same at every height; then where they end
+  Real* half_y;                    // [Ph]: second component of the half sphere's directions
+  Coord<Real>* half_rows;          // [B][nE0][Th]: elevation coordinate of the ring's dS lookups
+  HalfWeight<Real>* half_weights;  // [B][half_slab][Th][n3]: of that many lights at a time
 };
 
 // Bytes of shared memory that point scatter's tables are allowed: the limit
@@ -38,7 +41,7 @@ size_t ray_scatter_capacity(const BuildDims& d);
 // The set-up tables in parts: the rows (row info and point rows), then the
 // 4-D node maps with each node's light direction (remap4) and the view-row
 // samples, which both read the rows but not each other, and the rest
-// (remapT, remapE, sphere rings, surface rows, half directions).  launch_setup runs them all on one stream.
+// (remapT, remapE, sphere rings, surface radiance's tables).  launch_setup runs them all on one stream.
 template <class Real>
 void launch_setup_rows(const AtmoParams* params, const BuildDims& d, const SetupBuffers<Real>& o, cudaStream_t st);
 template <class Real>
@@ -108,11 +111,15 @@ template <class Real>
 void launch_sphere_dirs(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs, SphereDir<Real>* out,
                         cudaStream_t st);
 
-// dE = surface radiance of dS (same first-iteration convention).
+// Surface radiance's set-up tables; the number of kernels launched.
 template <class Real>
-void launch_surface_radiance(const AtmoParams* params, const BuildDims& d, const SurfRow<Real>* erow,
-                             const HalfDir<Real>* hdir, const Vec4<Real>* dS, const Vec4<Real>* mie,
-                             Vec4<Real>* dE, cudaStream_t st);
+int launch_surface_rows(const AtmoParams* params, const BuildDims& d, const DirLocal* half_dirs,
+                        const SetupBuffers<Real>& o, cudaStream_t st);
+// dE = surface radiance of dS (same first-iteration convention); the number
+// of kernels launched.
+template <class Real>
+int launch_surface_radiance(const AtmoParams* params, const BuildDims& d, const SetupBuffers<Real>& o,
+                            const Vec4<Real>* dS, const Vec4<Real>* mie, Vec4<Real>* dE, cudaStream_t st);
 
 // dS = ray scatter of J.
 template <class Real>
