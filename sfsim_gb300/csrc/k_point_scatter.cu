@@ -21,15 +21,17 @@
 // all j, so the block interpolates their rows once per direction into shared
 // memory and every thread adds them from there.
 //
-// What bounds it: shared-memory wavefronts, six 4-byte gathers (three
-// channels, value and step to the next texel) per heading and direction and
-// six more on the ground.  Production tables (32x255x32x8, 336 directions, 5
-// iterations): 160M wavefronts a launch, 0.51 ms at one per clock and SM;
-// measured 0.63 ms, 3.49 ms for the build's five launches.  With a row per
-// direction instead of per ring (gathered to HBM by a kernel of its own), the
-// phases exchanged by shuffles and every heading walked, it was 7.08 ms; the
-// 16 atmospheres of a sweep (16x128x16x8) went from 11.8 to 5.5 ms, the
-// reference's tables (32x127x32x8, 71 directions) from 0.96 to 0.50 ms.
+// What bounds it: the FMA pipe (packed operations take it for two cycles) and
+// the shared-memory wavefronts together, about 70 and 60 % of a launch.  A
+// heading and direction gathers 24 bytes of its ring's row (two channels'
+// values and steps in one load, the third's in another) and 24 more of the
+// ground's.  Production tables (32x255x32x8, 336 directions, 5 iterations):
+// 98M wavefronts and 0.55 ms a launch, 2.96 ms for the build's five; with
+// 4-byte loads it was 160M and 3.49 ms.  With a row per direction instead of
+// per ring (gathered to HBM by a kernel of its own), the phases exchanged by
+// shuffles and every heading walked, it was 7.08 ms.  The 16 atmospheres of a
+// sweep (16x128x16x8) went from 11.8 to 5.3 to 4.6 ms, the reference's tables
+// (32x127x32x8, 71 directions) from 0.96 to 0.47 to 0.41 ms.
 #include <type_traits>
 
 #include "atmo_device.cuh"
@@ -37,13 +39,18 @@
 
 namespace sfsim {
 
-// Values per record of a ring row: three channels' (value, step to the next
-// texel), in the first iteration those of the Mie strength too; an odd
-// stride spreads the texels over the banks.
+// A record of a row: the values of two channels and their steps to the next
+// texel, value and step of the third.  With the Mie strength (first
+// iteration) its two channels follow the first four, and its third the other
+// two.  All of it is read in 8- and 16-byte loads, which take half the
+// wavefronts of 4-byte ones where the lanes of each pair (2n, 2n + 1) read the
+// same record, as neighbouring elevations mostly do, and no more where they do
+// not.
 template <bool FIRST>
 __host__ __device__ constexpr int row_stride() {
-  return FIRST ? 13 : 7;
+  return FIRST ? 12 : 8;
 }
+constexpr int kGroundStride = 6;  // the same for the surface-radiance row
 
 // Records of a ring row: a copy of texel 0, then the n3 texels, so that a
 // coordinate that rounding pushed just below 0 reads texel 0; the last
@@ -53,15 +60,14 @@ __host__ __device__ constexpr int row_records(int n3) { return n3 + 1; }
 // Shared-memory layout, in this order, each part 16-byte aligned.
 struct PointLayout {
   unsigned dirs;    // [P][4] x1, x1, x2, x2
-  unsigned edge;    // [P][8] three channels at the first and last heading's l, in pairs
+  unsigned edge;    // [P][8] HeadingPair of the first and last heading
   unsigned rings;   // [T] SphereRing
   unsigned rows;    // [T][n3 + 1][row_stride]
-  unsigned etab;    // [nE1][estride]
+  unsigned etab;    // [nE1][kGroundStride]
   unsigned bytes;
-  int estride;      // 7, or 6 where 7 would not fit
 };
 template <class Real>
-__host__ __device__ inline PointLayout point_layout(const BuildDims& d, bool first, int estride) {
+__host__ __device__ inline PointLayout point_layout(const BuildDims& d, bool first) {
   auto up = [](size_t x) { return (x + 15) & ~size_t(15); };
   PointLayout l;
   size_t o = 0;
@@ -74,17 +80,34 @@ __host__ __device__ inline PointLayout point_layout(const BuildDims& d, bool fir
   l.rows = (unsigned)o;
   o = up(o + sizeof(Real) * d.T * row_records(d.n3) * (first ? row_stride<true>() : row_stride<false>()));
   l.etab = (unsigned)o;
-  o = up(o + sizeof(Real) * estride * d.nE1);
+  o = up(o + sizeof(Real) * kGroundStride * d.nE1);
   l.bytes = (unsigned)o;
-  l.estride = estride;
   return l;
 }
+
+// Where a record keeps channel c's value (c < 3: dS, c >= 3: the Mie
+// strength), and its step.
+template <bool FIRST>
+__device__ __forceinline__ constexpr int value_at(int c) {
+  return c < 2 ? c : c == 2 ? (FIRST ? 8 : 4) : c < 5 ? c + 1 : 10;
+}
+template <bool FIRST>
+__device__ __forceinline__ constexpr int step_at(int c) {
+  return value_at<FIRST>(c) + (c == 2 || c == 5 ? 1 : 2);
+}
+
+// Radiances of a pair of headings a and b: the first two channels of each,
+// and the third of both.
+template <class Real>
+struct HeadingPair {
+  V2<Real> a, b, z;
+};
 
 constexpr int kPointThreads = 128;
 
 // Blocks per SM the registers are limited for.  Three heading pairs measured
-// 3.49 / 3.57 / 3.70 ms of a production build (5 launches) at 3 / 4 / 5
-// blocks: the gathers, not the warps in flight, are the limit.
+// 3.11 / 2.96 / 3.04 / 3.25 ms of a production build (5 launches) at 2 / 3 /
+// 4 / 5 blocks.
 template <class Real, int HP>
 constexpr int point_min_blocks() {
   return sizeof(Real) == 8 ? 2 : HP == 3 ? 3 : HP == 2 ? 4 : 5;
@@ -110,7 +133,7 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
   SphereRing<Real>* sring = reinterpret_cast<SphereRing<Real>*>(smem_raw + lay.rings);
   Real* srows = reinterpret_cast<Real*>(smem_raw + lay.rows);
   Real* setab = reinterpret_cast<Real*>(smem_raw + lay.etab);
-  const unsigned es = (unsigned)lay.estride;
+  constexpr int ES = kGroundStride;
   const int nrec = row_records(d.n3);
   const long long base4 = (long long)b * d.n4();
 
@@ -130,16 +153,12 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
       if (FIRST) gather_row_texel(Mt + base4, d, pk.u0, pk.s0, u1, s1, pk.u2, pk.s2, a, vm);
       Real* o = srows + (r * nrec + a + 1) * KS;
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        o[2 * c] = v[c];
-        if (FIRST) o[6 + 2 * c] = vm[c];
+      for (int c = 0; c < (FIRST ? 6 : 3); c++) {
+        const Real x = c < 3 ? v[c % 3] : vm[c % 3];
+        o[value_at<FIRST>(c)] = x;
         if (a == 0) {
-          o[2 * c - KS] = v[c];
-          o[2 * c + 1 - KS] = Real(0);
-          if (FIRST) {
-            o[6 + 2 * c - KS] = vm[c];
-            o[6 + 2 * c + 1 - KS] = Real(0);
-          }
+          o[value_at<FIRST>(c) - KS] = x;
+          o[step_at<FIRST>(c) - KS] = Real(0);
         }
       }
     }
@@ -150,8 +169,8 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
       ld3(e, upper_index(t, d.nE1), B);
 #pragma unroll
       for (int c = 0; c < 3; c++) {
-        setab[t * es + 2 * c] = A[c];
-        setab[t * es + 2 * c + 1] = B[c] - A[c];
+        setab[t * ES + value_at<false>(c)] = A[c];
+        setab[t * ES + step_at<false>(c)] = B[c] - A[c];
       }
     }
   }
@@ -159,16 +178,16 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
   for (int t = tid; t < d.T * d.n3; t += nt) {
     const int r = t / d.n3, a = t - r * d.n3;
     Real* o = srows + (r * nrec + a + 1) * KS;
-    constexpr int nc = FIRST ? 6 : 3;
 #pragma unroll
-    for (int c = 0; c < nc; c++) o[2 * c + 1] = a < d.n3 - 1 ? o[KS + 2 * c] - o[2 * c] : Real(0);
+    for (int c = 0; c < (FIRST ? 6 : 3); c++)
+      o[step_at<FIRST>(c)] = a < d.n3 - 1 ? o[KS + value_at<FIRST>(c)] - o[value_at<FIRST>(c)] : Real(0);
   }
   __syncthreads();
 
   const PhaseCS<Real> phR(Bulk<Real>::phase_ray(P)), phM(Bulk<Real>::phase_mie(P));
   const Real scale3 = Real(0.5) * Real(d.n3 - 1);
   const Real scaleE = Bulk<Real>::sun_scale_E(d);
-  const unsigned kstride = KS * sizeof(Real), estride = es * sizeof(Real);
+  const unsigned kstride = KS * sizeof(Real), estride = ES * sizeof(Real);
   const unsigned ebase = lookup_base<Real>(lay.etab, estride);
   const Real log2e = Real(1.4426950408889634);
   const Real zA = -log2e * fma(Real(3), pk.gA, Real(0.6));
@@ -177,7 +196,7 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
   // light directions (lx, ly, lz) of a pair: dS along the ring's row and, for
   // rings that end on the ground, the ground's radiance
   auto incoming = [&](auto ground, const SphereRing<Real>& rc, unsigned rbase, R2 c0, R2 x1, R2 x2, R2 ly, R2 lz,
-                      Real off, R2 (&X)[3]) {
+                      Real off, HeadingPair<Real>& X) {
     const R2 mu = fma2(x1, ly, fma2(x2, lz, c0));  // omega . l
     // the sun-angle coordinate; |mu| <= 1 up to rounding, so its floor lies in
     // [-1, n3 - 1], whose records give the clamped interpolation
@@ -185,13 +204,27 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     const R2 s = lookup(fma2(dup(scale3), mu, dup(scale3)), rbase, rbase, kstride, oa, ob);
     const Real* ra = reinterpret_cast<const Real*>(smem_raw + oa);
     const Real* rb = reinterpret_cast<const Real*>(smem_raw + ob);
-#pragma unroll
-    for (int c = 0; c < 3; c++) X[c] = fma2(mk2(ra[2 * c + 1], rb[2 * c + 1]), s, mk2(ra[2 * c], rb[2 * c]));
+    R2 v, step, third;
+    ld_pairs(ra, v, step);
+    X.a = fma2(step, dup(s.x), v);
+    ld_pairs(rb, v, step);
+    X.b = fma2(step, dup(s.y), v);
     if (FIRST) {
       const R2 ph = phM.pair(mu);
-#pragma unroll
-      for (int c = 3; c < 6; c++)
-        X[c - 3] = fma2(fma2(mk2(ra[2 * c + 1], rb[2 * c + 1]), s, mk2(ra[2 * c], rb[2 * c])), ph, X[c - 3]);
+      R2 thirdm;
+      ld_pairs(ra + 4, v, step);
+      X.a = fma2(fma2(step, dup(s.x), v), dup(ph.x), X.a);
+      ld_pairs(rb + 4, v, step);
+      X.b = fma2(fma2(step, dup(s.y), v), dup(ph.y), X.b);
+      ld_pairs(ra + 8, third, thirdm);
+      X.z.x = fma(fma(thirdm.y, s.x, thirdm.x), ph.x, fma(third.y, s.x, third.x));
+      ld_pairs(rb + 8, third, thirdm);
+      X.z.y = fma(fma(thirdm.y, s.y, thirdm.x), ph.y, fma(third.y, s.y, third.x));
+    } else {
+      third = *reinterpret_cast<const R2*>(ra + 4);
+      X.z.x = fma(third.y, s.x, third.x);
+      third = *reinterpret_cast<const R2*>(rb + 4);
+      X.z.y = fma(third.y, s.y, third.x);
     }
     if (decltype(ground)::value) {
       // the ground point's sin of the sun elevation, g.l / |g| = gA + tR (omega . l)
@@ -202,13 +235,13 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
       R2 ie = fma2(dup(-scaleE), ex, dup(scaleE));
       ie = mk2(fmax(ie.x, Real(0)), fmax(ie.y, Real(0)));
       const R2 se = lookup(ie, ebase, ebase, estride, oa, ob);
-      const Real* ea = reinterpret_cast<const Real*>(smem_raw + oa);
-      const Real* eb = reinterpret_cast<const Real*>(smem_raw + ob);
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const R2 y = fma2(mk2(ea[2 * c + 1], eb[2 * c + 1]), se, mk2(ea[2 * c], eb[2 * c]));
-        X[c] = fma2(dup(rc.ground[c]), y, X[c]);
-      }
+      const R2* ea = reinterpret_cast<const R2*>(smem_raw + oa);
+      const R2* eb = reinterpret_cast<const R2*>(smem_raw + ob);
+      const R2 g = mk2(rc.ground[0], rc.ground[1]);
+      X.a = fma2(g, fma2(ea[1], dup(se.x), ea[0]), X.a);
+      X.b = fma2(g, fma2(eb[1], dup(se.y), eb[0]), X.b);
+      const R2 ta = ea[2], tb = eb[2];
+      X.z = fma2(dup(rc.ground[2]), mk2(fma(ta.y, se.x, ta.x), fma(tb.y, se.y, tb.x)), X.z);
       if constexpr (std::is_same<Real, double>::value) {
         // the FP64 build's ground point is off height 0 by its rounding, as
         // the reference's is: the next height's row has that weight
@@ -226,8 +259,10 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
           double ya[3], yb[3];
           above(ia, se.x, ya);
           above(ib, se.y, yb);
-#pragma unroll
-          for (int c = 0; c < 3; c++) X[c] = fma2(dup(rc.ground[c] * off), mk2(ya[c], yb[c]), X[c]);
+          const R2 go = mk2(rc.ground[0] * off, rc.ground[1] * off);
+          X.a = fma2(go, mk2(ya[0], ya[1]), X.a);
+          X.b = fma2(go, mk2(yb[0], yb[1]), X.b);
+          X.z = fma2(dup(rc.ground[2] * off), mk2(ya[2], yb[2]), X.z);
         }
       }
     }
@@ -249,14 +284,13 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
       const unsigned rbase = ring_base(r);
       for (int m = tid; m < rc.n; m += nt) {
         const Real* x = sdirs + 4 * (rc.w0 + m);
-        R2 X[3];
+        HeadingPair<Real> X;
         if (rc.surface)
           incoming(std::true_type{}, rc, rbase, dup(rc.x0 * lx), dup(x[0]), dup(x[2]), ly, lz, offset(rc.w0 + m), X);
         else
           incoming(std::false_type{}, rc, rbase, dup(rc.x0 * lx), dup(x[0]), dup(x[2]), ly, lz, offset(rc.w0 + m), X);
         R2* o = reinterpret_cast<R2*>(sedge + 8 * (rc.w0 + m));
-#pragma unroll
-        for (int c = 0; c < 3; c++) o[c] = X[c];
+        o[0] = X.a, o[1] = X.b, o[2] = X.z;
       }
     }
   }
@@ -284,11 +318,10 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     lz[h] = mk2(ga.lz, gb.lz);
   }
   // sums over the directions so far, and over the ring being walked (pair HP: the first and last heading)
-  R2 tot[HP + 1][3];
+  HeadingPair<Real> tot[HP + 1];
+  const HeadingPair<Real> none{dup(Real(0)), dup(Real(0)), dup(Real(0))};
 #pragma unroll
-  for (int h = 0; h <= HP; h++)
-#pragma unroll
-    for (int c = 0; c < 3; c++) tot[h][c] = dup(Real(0));
+  for (int h = 0; h <= HP; h++) tot[h] = none;
 
   for (int r = 0; r < d.T; r++) {
     const SphereRing<Real>& rc = sring[r];
@@ -302,32 +335,32 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     Real bR[3], bM[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) bR[c] = rc.weight * pk.bR[c], bM[c] = rc.weight * pk.bM[c];
-    R2 sum[HP + 1][3];
+    HeadingPair<Real> sum[HP + 1];
 #pragma unroll
-    for (int h = 0; h <= HP; h++)
-#pragma unroll
-      for (int c = 0; c < 3; c++) sum[h][c] = dup(Real(0));
+    for (int h = 0; h <= HP; h++) sum[h] = none;
+    auto add = [](HeadingPair<Real>& t, R2 w, Real wz, const HeadingPair<Real>& X) {
+      t.a = fma2(w, X.a, t.a);
+      t.b = fma2(w, X.b, t.b);
+      t.z = fma2(dup(wz), X.z, t.z);
+    };
     auto walk = [&](auto ground) {
       for (int m = 0; m < n; m++, x += 4, e += 8) {
         R2 x1, x2;
         ld_pairs(x, x1, x2);
         const Real mv = fma(cv, x1.x, mv0);
         const Real fR = phR(mv), fM = phM(mv);
-        R2 w[3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) w[c] = dup(fma(bM[c], fM, bR[c] * fR));
+        const R2 w = fma2(mk2(bM[0], bM[1]), dup(fM), mul2(mk2(bR[0], bR[1]), dup(fR)));
+        const Real wz = fma(bM[2], fM, bR[2] * fR);
 #pragma unroll
         for (int h = 0; h < HP; h++) {
-          R2 X[3];
+          HeadingPair<Real> X;
           incoming(ground, rc, rbase, c0, x1, x2, ly[h], lz[h], offset(rc.w0 + m), X);
-#pragma unroll
-          for (int c = 0; c < 3; c++) sum[h][c] = fma2(w[c], X[c], sum[h][c]);
+          add(sum[h], w, wz, X);
         }
-        R2 X[3];
-        ld_pairs(e, X[0], X[1]);
-        X[2] = *reinterpret_cast<const R2*>(e + 4);
-#pragma unroll
-        for (int c = 0; c < 3; c++) sum[HP][c] = fma2(w[c], X[c], sum[HP][c]);
+        HeadingPair<Real> X;
+        ld_pairs(e, X.a, X.b);
+        X.z = *reinterpret_cast<const R2*>(e + 4);
+        add(sum[HP], w, wz, X);
       }
     };
     if (rc.surface)
@@ -335,15 +368,17 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     else
       walk(std::false_type{});
 #pragma unroll
-    for (int h = 0; h <= HP; h++)
-#pragma unroll
-      for (int c = 0; c < 3; c++) tot[h][c] = add2(tot[h][c], sum[h][c]);
+    for (int h = 0; h <= HP; h++) {
+      tot[h].a = add2(tot[h].a, sum[h].a);
+      tot[h].b = add2(tot[h].b, sum[h].b);
+      tot[h].z = add2(tot[h].z, sum[h].z);
+    }
   }
   if (!valid) return;
-  auto put = [&](int at, Real x, Real y, Real z) {
+  auto put = [&](int at, R2 xy, Real z) {
     Vec4<Real> o;
-    o.x = x;
-    o.y = y;
+    o.x = xy.x;
+    o.y = xy.y;
     o.z = z;
     o.w = 0;
     J[node0 + at] = o;
@@ -351,12 +386,12 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
 #pragma unroll
   for (int h = 0; h < HP; h++) {
     const int a = a0 + 2 * h;
-    if (a < d.n3 - 1) put(a, tot[h][0].x, tot[h][1].x, tot[h][2].x);
-    if (a + 1 < d.n3 - 1) put(a + 1, tot[h][0].y, tot[h][1].y, tot[h][2].y);
+    if (a < d.n3 - 1) put(a, tot[h].a, tot[h].z.x);
+    if (a + 1 < d.n3 - 1) put(a + 1, tot[h].b, tot[h].z.y);
   }
   if (grp == 0) {
-    put(0, tot[HP][0].x, tot[HP][1].x, tot[HP][2].x);
-    put(d.n3 - 1, tot[HP][0].y, tot[HP][1].y, tot[HP][2].y);
+    put(0, tot[HP].a, tot[HP].z.x);
+    put(d.n3 - 1, tot[HP].b, tot[HP].z.y);
   }
 }
 
@@ -379,8 +414,7 @@ int launch_point_scatter(const AtmoParams* params, const BuildDims& d, const Row
                          const PointRow<Real>* prow, const CellGeom<Real>* geom, const Vec4<Real>* dS, const Vec4<Real>* mie, const Vec4<Real>* dE,
                          Vec4<Real>* J, cudaStream_t st) {
   const bool first = mie != nullptr;
-  PointLayout lay = point_layout<Real>(d, first, 7);
-  if (lay.bytes > 227 * 1024) lay = point_layout<Real>(d, first, 6);
+  const PointLayout lay = point_layout<Real>(d, first);
   const int inner = d.n3 - 2;
   int hp = sizeof(Real) == 8 ? 1 : inner > 4 ? 3 : inner > 2 ? 2 : 1;
   const int groups = inner > 0 ? (inner + 2 * hp - 1) / (2 * hp) : 1;
