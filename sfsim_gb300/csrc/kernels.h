@@ -334,6 +334,11 @@ void launch_perlin(int divisions, int size, const int* gradients, float* out, un
 // 2048 pixels that split evenly over 8 (or 16) CTAs run on a CTA cluster
 // (blue_noise_cluster_size); `error` (device int, zeroed by the caller) is
 // set when one of its bounded waits gave up.
+// Where blue_tiles_serve, the chains of steps run on one CTA each
+// (k_blue_noise.cu): stage 0 the seed pattern, 1 phases 1 and 2, 2 phase 3.
+bool blue_tiles_serve(int m, double sigma);
+int launch_blue_tiles(int stage, int m, int n, const double* table, double* density, double* density0,
+                      unsigned char* mask, unsigned char* work, int* dither, cudaStream_t st);
 size_t blue_noise_smem(int m, bool* use_smem);
 int blue_noise_cluster_size(int m);
 int launch_blue_noise(int m, int n, const int* seed, double sigma, const double* table, double* density,
