@@ -4,18 +4,25 @@
 // K contiguous).
 //
 // A persistent, warp-specialised kernel.  Work items are output tiles of
-// 128 x Nt (Nt = N rounded up to 16, at most 256) times split-K slices of the
-// K range, dealt round-robin to one CTA per SM.  Warp 0 is the producer: one thread loads K chunks of 64 of A
+// 128 x Nt (Nt = N rounded up to 16, at most 256, or 128 where the outputs are
+// row-major) times split-K slices of the K range, dealt round-robin to one CTA per SM.  Warp 0 is the producer: one thread loads K chunks of 64 of A
 // (128 x 64) and B (Nt x 64) with TMA tensor copies (128-byte swizzle) into a
 // ring of shared-memory stages.  Warp 1 issues the tcgen05.mma (K = 16 each,
 // 128-byte-swizzled K-major descriptors) into one of two tensor-memory
-// accumulators and releases each stage with tcgen05.commit.  Warps 2-9 are the
-// epilogue, two per group of 32 tensor-memory lanes (one per half of the
-// columns): they read the finished accumulator (tcgen05.ld, the next 32
-// columns in flight while the current ones are written) and apply the
+// accumulators and releases each stage with tcgen05.commit.  Warps 2-17 are the
+// epilogue, four per group of 32 tensor-memory lanes (one per quarter of the
+// columns): they read the finished accumulator (tcgen05.ld) and apply the
 // epilogue while the MMAs of the next tile run into the other accumulator;
 // full 32 x 32 blocks pass their row-major input and outputs through a
 // per-warp shared-memory tile so that global accesses are row-contiguous.
+//
+// What bounds it: for the surrogate's layers (65536 x 256 x 256, SiLU and its
+// derivative written, 167 MB moved) the epilogue, whose warps wait for their
+// loads and for the chain through the staging tile; the MMAs take a twentieth.
+// Measured, forward / activation-gradient layer: 50 / 33 us (24 at the memory's
+// rate); with 8 epilogue warps, tiles of all 256 columns, the SiLU' input
+// loaded when its block was due and the transposed output stored 2 bytes a
+// lane 100 / 100, with 16 such warps 72 / 53.
 // Every wait is bounded by a poll limit set at run time
 // (sfsim_atmo_set_wait_limit); on timeout the CTA records an error, tells its
 // other roles through a shared-memory flag (their waits give up when they see
@@ -36,9 +43,11 @@
 namespace sfsim {
 
 constexpr int kGemmBK = 64;                 // K per stage: one 128-byte swizzle atom of bf16
-constexpr int kGemmThreads = 320;  // producer, MMA, 8 epilogue warps
-constexpr int kGemmEpilogueThreads = 256;
-constexpr int kGemmSmemBudget = 192 * 1024;  // stages
+constexpr int kGemmEpilogueWarps = 16;
+constexpr int kGemmEpilogueThreads = 32 * kGemmEpilogueWarps;
+constexpr int kGemmThreads = 64 + kGemmEpilogueThreads;  // producer, MMA, epilogue
+constexpr int kGemmSmemBudget = 192 * 1024;        // stages
+constexpr int kGemmSmemBudgetStaged = 144 * 1024;  // beside the staging tiles
 constexpr int kGemmTileA = 128 * kGemmBK * 2;
 
 // K-major operand with 128-byte swizzle: rows of 128 B, 16-byte chunks XOR
@@ -70,39 +79,60 @@ __device__ __forceinline__ float dsilu(float z) {
 
 struct GemmKernelArgs {
   GemmArgs g;
-  int nt;          // N rounded up to 16: the MMA's N and the B box height
+  int nt;          // a tile's columns, a multiple of 16: the MMA's N and the B box height
   int stages;
-  int tiles_m, splits;
+  int tiles_m, tiles_n, splits;
   long long kper;  // K per split, a multiple of kGemmBK
   int wait_limit;  // polls per mbarrier wait
 };
 
-// Per epilogue warp: a 32 x 32 staging tile (row stride 33 words) that turns
-// the lane-per-row layout of the tensor-memory loads into row-contiguous
-// global accesses.
-constexpr int kGemmStageWords = 32 * 33;
+// Per epilogue warp: a 32 x 32 staging tile that turns the lane-per-row layout
+// of the tensor-memory loads into row-contiguous global accesses.  Rows of 36
+// words (20 for BF16): 16-byte accesses of 8 lanes, a row each, reach every
+// bank once.
+constexpr int kGemmStageRow = 36, kGemmStageRowH = 20;
+constexpr int kGemmStageWords = 32 * kGemmStageRow;
 
-// The 32 x 32 block of rows m0 .. m0 + 31 (lane = row), columns n0 .. n0 + 31,
-// with every row and column inside the output and 16-byte aligned rows: the
-// SiLU' input is read, and the SiLU' and BF16 row-major outputs written, a
-// whole row segment at a time through the warp's staging tile.  Returns
-// false (nothing done) when the block does not qualify.
+// Only the row-major outputs go through the staging tiles.
+__host__ __device__ inline bool gemm_staged(const GemmArgs& g) { return !g.Cacc && !g.Cf32; }
+
+// Whether the 32 x 32 block of rows m0 .. m0 + 31, columns n0 .. n0 + 31 goes
+// through a staging tile: every row and column inside the output, 16-byte
+// aligned rows.
+__device__ __forceinline__ bool gemm_block_fits(const GemmArgs& g, int m0, int n0) {
+  return gemm_staged(g) && m0 + 32 <= g.M && n0 + 32 <= g.N && (g.N % 4) == 0 &&
+         (!g.dact || (reinterpret_cast<uintptr_t>(g.dact) & 15) == 0) &&
+         (!g.Dsilu || (reinterpret_cast<uintptr_t>(g.Dsilu) & 15) == 0) &&
+         (!g.row_bias || (reinterpret_cast<uintptr_t>(g.row_bias) & 15) == 0) &&
+         (!g.Hbf16 || ((g.ldh % 8) == 0 && (reinterpret_cast<uintptr_t>(g.Hbf16) & 15) == 0));
+}
+
+// Such a block's SiLU' input on its way into the warp's staging tile, a whole
+// row segment at a time: lane l moves 16 bytes of row 4k + l / 8.
+__device__ __forceinline__ void gemm_fetch_dact(const GemmArgs& g, int m0, int n0, float* sg) {
+  const int rq = (threadIdx.x & 31) >> 3, c4 = 4 * (threadIdx.x & 7);
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     tc::smem_u32(sg + (4 * k + rq) * kGemmStageRow + c4)),
+                 "l"(g.dact + (long long)(m0 + 4 * k + rq) * g.N + n0 + c4)
+                 : "memory");
+}
+__device__ __forceinline__ void gemm_fetch_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The epilogue of a block that fits (lane = row): the SiLU' input comes out of
+// the staging tile, and the SiLU' and BF16 row-major outputs go through it, a
+// whole row segment at a time.  `bias` is g.bias in shared memory.
 template <bool ROWB>
-__device__ __forceinline__ bool gemm_epilogue32_staged(const GemmArgs& g, const uint32_t* r, int m0, int n0,
-                                                       float* sg) {
+__device__ __forceinline__ void gemm_epilogue32_staged(const GemmArgs& g, const uint32_t* r, int m0, int n0,
+                                                       const float* bias, float* sg) {
   const int lane = threadIdx.x & 31;
-  const bool fits = m0 + 32 <= g.M && n0 + 32 <= g.N && (g.N % 4) == 0 && !g.Cacc && !g.Cf32 &&
-                    (!g.dact || (reinterpret_cast<uintptr_t>(g.dact) & 15) == 0) &&
-                    (!g.Dsilu || (reinterpret_cast<uintptr_t>(g.Dsilu) & 15) == 0) &&
-                    (!g.row_bias || (reinterpret_cast<uintptr_t>(g.row_bias) & 15) == 0) &&
-                    (!g.Hbf16 || ((g.ldh % 8) == 0 && (reinterpret_cast<uintptr_t>(g.Hbf16) & 15) == 0));
-  if (!fits) return false;
   float z[32];
 #pragma unroll
   for (int i = 0; i < 32; i++) z[i] = __uint_as_float(r[i]) * g.alpha;
   if (g.bias) {
 #pragma unroll
-    for (int i = 0; i < 32; i++) z[i] += g.bias[n0 + i];
+    for (int i = 0; i < 32; i++) z[i] += bias[n0 + i];
   }
   if (ROWB) {
     const float4* rb = reinterpret_cast<const float4*>(g.row_bias + (long long)g.row_group[m0 + lane] * g.N + n0);
@@ -114,17 +144,15 @@ __device__ __forceinline__ bool gemm_epilogue32_staged(const GemmArgs& g, const 
   }
   // row segments of 32 floats: lane l moves 16 bytes of row 4k + l / 8
   const int rq = lane >> 3, c4 = 4 * (lane & 7);
+  float* own = sg + lane * kGemmStageRow;
   if (g.dact) {
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const int row = 4 * k + rq;
-      const float4 v = *reinterpret_cast<const float4*>(g.dact + (long long)(m0 + row) * g.N + n0 + c4);
-      float* d = sg + row * 33 + c4;
-      d[0] = v.x, d[1] = v.y, d[2] = v.z, d[3] = v.w;
-    }
+    gemm_fetch_wait();
     __syncwarp();
 #pragma unroll
-    for (int i = 0; i < 32; i++) z[i] *= sg[lane * 33 + i];
+    for (int i = 0; i < 32; i += 4) {
+      const float4 d = *reinterpret_cast<const float4*>(own + i);
+      z[i] *= d.x, z[i + 1] *= d.y, z[i + 2] *= d.z, z[i + 3] *= d.w;
+    }
     __syncwarp();
   }
   // with SiLU' requested, the logistic s of each z serves both SiLU' and
@@ -132,48 +160,68 @@ __device__ __forceinline__ bool gemm_epilogue32_staged(const GemmArgs& g, const 
   const bool silu_done = g.Dsilu && g.silu;
   if (g.Dsilu) {
 #pragma unroll
-    for (int i = 0; i < 32; i++) {
-      const float sgm = 1.0f / (1.0f + __expf(-z[i]));
-      sg[lane * 33 + i] = sgm * (1.0f + z[i] * (1.0f - sgm));
-      if (g.silu) z[i] *= sgm;
+    for (int i = 0; i < 32; i += 4) {
+      float d[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const float sgm = 1.0f / (1.0f + __expf(-z[i + e]));
+        d[e] = sgm * (1.0f + z[i + e] * (1.0f - sgm));
+        if (g.silu) z[i + e] *= sgm;
+      }
+      *reinterpret_cast<float4*>(own + i) = make_float4(d[0], d[1], d[2], d[3]);
     }
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       const int row = 4 * k + rq;
-      const float* d = sg + row * 33 + c4;
-      *reinterpret_cast<float4*>(g.Dsilu + (long long)(m0 + row) * g.N + n0 + c4) = make_float4(d[0], d[1], d[2], d[3]);
+      *reinterpret_cast<float4*>(g.Dsilu + (long long)(m0 + row) * g.N + n0 + c4) =
+          *reinterpret_cast<const float4*>(sg + row * kGemmStageRow + c4);
     }
     __syncwarp();
   }
   if (g.Hbf16 || g.HTbf16) {
-    __nv_bfloat16 h[32];
+    uint32_t h[16];  // pairs of columns
 #pragma unroll
-    for (int i = 0; i < 32; i++) h[i] = __float2bfloat16(g.silu && !silu_done ? silu(z[i]) : z[i]);
+    for (int i = 0; i < 16; i++) {
+      const bool act = g.silu && !silu_done;
+      const __nv_bfloat162 p = __floats2bfloat162_rn(act ? silu(z[2 * i]) : z[2 * i], act ? silu(z[2 * i + 1]) : z[2 * i + 1]);
+      h[i] = *reinterpret_cast<const uint32_t*>(&p);
+    }
     if (g.Hbf16) {
-      // 16 packed pairs per row; lane l moves 16 bytes of row 8k + l / 4
       uint32_t* s32 = reinterpret_cast<uint32_t*>(sg);
-      const uint32_t* hp = reinterpret_cast<const uint32_t*>(h);
 #pragma unroll
-      for (int i = 0; i < 16; i++) s32[lane * 17 + i] = hp[i];
+      for (int i = 0; i < 16; i += 4)
+        *reinterpret_cast<uint4*>(s32 + lane * kGemmStageRowH + i) = make_uint4(h[i], h[i + 1], h[i + 2], h[i + 3]);
       __syncwarp();
+      // lane l moves 16 bytes of row 8k + l / 4
       const int rr = lane >> 2, q4 = 4 * (lane & 3);
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         const int row = 8 * k + rr;
-        const uint32_t* d = s32 + row * 17 + q4;
         *reinterpret_cast<uint4*>(g.Hbf16 + (long long)(m0 + row) * g.ldh + n0 + 2 * q4) =
-            make_uint4(d[0], d[1], d[2], d[3]);
+            *reinterpret_cast<const uint4*>(s32 + row * kGemmStageRowH + q4);
       }
       __syncwarp();
     }
     if (g.HTbf16) {
-      const int m = m0 + lane;
+      if ((g.ldht % 2) == 0 && (reinterpret_cast<uintptr_t>(g.HTbf16) & 3) == 0) {
+        // lanes 2k and 2k + 1 (two rows) exchange halves: the first takes both rows of the even columns, the
+        // second of the odd ones, so a store moves 64 contiguous bytes of two transposed rows
+        const int odd = lane & 1;
+        __nv_bfloat16* dst = g.HTbf16 + (long long)(n0 + odd) * g.ldht + m0 + lane - odd;
 #pragma unroll
-      for (int i = 0; i < 32; i++) g.HTbf16[(long long)(n0 + i) * g.ldht + m] = h[i];
+        for (int i = 0; i < 16; i++) {
+          const uint32_t o = __shfl_xor_sync(0xffffffffu, h[i], 1);
+          const uint32_t w = odd ? __byte_perm(o, h[i], 0x7632) : __byte_perm(h[i], o, 0x5410);
+          *reinterpret_cast<uint32_t*>(dst + (long long)(2 * i) * g.ldht) = w;
+        }
+      } else {
+        const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(h);
+#pragma unroll
+        for (int i = 0; i < 32; i++) g.HTbf16[(long long)(n0 + i) * g.ldht + m0 + lane] = e[i];
+      }
     }
   }
-  return true;
 }
 
 // 32 columns of the epilogue for row m, columns n0 .. n0 + 31.
@@ -286,10 +334,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   uint64_t* stall = drain + 1;   // self-test: nothing arrives on it
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stall + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* staging = reinterpret_cast<float*>(smem + S * stage_bytes + 1024);  // [8 epilogue warps][32 * 33]
+  float* bias = reinterpret_cast<float*>(smem + S * stage_bytes + 1024);  // [256]
+  float* staging = bias + 256;  // [epilogue warps][kGemmStageWords], where gemm_staged
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t ncols = a.nt <= 32 ? 32 : a.nt <= 64 ? 64 : a.nt <= 128 ? 128 : 256;  // per accumulator
-  const long long ntiles = (long long)a.tiles_m * a.splits;
+  const long long ntiles = (long long)a.tiles_m * a.tiles_n * a.splits;
   const long long my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
   const int kchunks = (int)(a.kper / kGemmBK);
 
@@ -308,6 +357,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     *abort_flag = 0;
     tc::fence_mbar_init();
   }
+  if (a.g.bias)
+    for (int t = threadIdx.x; t < a.g.N; t += kGemmThreads) bias[t] = a.g.bias[t];
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
@@ -320,7 +371,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       bool ok = true;
       for (long long ti = 0; ti < my_tiles && ok; ti++) {
         const long long tile = blockIdx.x + ti * gridDim.x;
-        const int tm = (int)(tile % a.tiles_m), split = (int)(tile / a.tiles_m);
+        const int tn = (int)(tile % a.tiles_n);
+        const long long rest = tile / a.tiles_n;
+        const int tm = (int)(rest % a.tiles_m), split = (int)(rest / a.tiles_m);
         for (int kc = 0; kc < kchunks; kc++, issued++) {
           const int s = (int)(issued % S);
           if (*abort_flag ||
@@ -333,7 +386,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           tc::mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
           const int k = (int)(split * a.kper + (long long)kc * kGemmBK);
           tma_load_2d(st, &mapA, k, tm * 128, &full[s]);
-          tma_load_2d(st + kGemmTileA, &mapB, k, 0, &full[s]);
+          tma_load_2d(st + kGemmTileA, &mapB, k, tn * a.nt, &full[s]);
         }
       }
       if (!ok) {
@@ -386,8 +439,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     __syncwarp();
   } else {
     // epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. + 31, columns
-    // of its half
-    const int q = warp & 3, half = (warp - 2) >> 2;
+    // of its quarter
+    const int q = warp & 3, part = (warp - 2) >> 2;
     bool ok = true;
     if (a.g.stall_polls > 0) {
       // self-test of the timeout path: a wait that cannot succeed
@@ -396,42 +449,36 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     for (long long ti = 0; ti < my_tiles && ok; ti++) {
       const long long tile = blockIdx.x + ti * gridDim.x;
-      const int tm = (int)(tile % a.tiles_m);
+      const int tn = (int)(tile % a.tiles_n), tm = (int)(tile / a.tiles_n % a.tiles_m);
       const int b = (int)(ti & 1);
+      const int m0 = tm * 128 + q * 32, m = m0 + lane;
+      const int nall = (a.nt + 31) / 32, each = (nall + 3) / 4;
+      float* sg = staging + (warp - 2) * kGemmStageWords;
+      // staged tiles have at most a block a warp (launch_gemm_tn)
+      const int first = tn * a.nt + 32 * part * each;
+      const bool staged = gemm_block_fits(a.g, m0, first);
+      if (staged && a.g.dact) gemm_fetch_dact(a.g, m0, first, sg);  // while the MMAs run
       bool done = tc::mbar_wait_or_abort(&tfull[b], (uint32_t)((ti >> 1) & 1), a.wait_limit, abort_flag);
       if (!__all_sync(0xffffffffu, done) || *abort_flag) {
         ok = false;
         break;
       }
       tc::fence_after();
-      const int m = tm * 128 + q * 32 + lane;
-      const int m0 = tm * 128 + q * 32;
-      float* sg = staging + (warp - 2) * kGemmStageWords;
-      auto epilogue = [&](const uint32_t* r, int n0) {
-        if (!__all_sync(0xffffffffu, gemm_epilogue32_staged<ROWB>(a.g, r, m0, n0, sg)))
-          gemm_epilogue32<ROWB>(a.g, r, m, n0);
-      };
       const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * ncols);
-      const int nall = (a.nt + 31) / 32, nh = (nall + 1) / 2;
-      const int b0 = half * nh, b1 = min(nall, b0 + nh);
-      if (b0 < b1) {
-        uint32_t rb[2][32];
-        tc::tmem_ld32_async(trow + (uint32_t)(32 * b0), rb[0]);
-        tc::tmem_wait_ld(rb[0]);
-        for (int blk = b0; blk < b1; blk += 2) {
-          if (blk + 1 < b1) tc::tmem_ld32_async(trow + (uint32_t)(32 * (blk + 1)), rb[1]);
-          epilogue(rb[0], 32 * blk);
-          if (blk + 1 < b1) {
-            tc::tmem_wait_ld(rb[1]);
-            if (blk + 2 < b1) tc::tmem_ld32_async(trow + (uint32_t)(32 * (blk + 2)), rb[0]);
-            epilogue(rb[1], 32 * (blk + 1));
-            if (blk + 2 < b1) tc::tmem_wait_ld(rb[0]);
-          }
-        }
+      const int b1 = min(nall, (part + 1) * each);
+      for (int blk = part * each; blk < b1; blk++) {
+        uint32_t r[32];
+        tc::tmem_ld32_async(trow + (uint32_t)(32 * blk), r);
+        tc::tmem_wait_ld(r);
+        if (staged)
+          gemm_epilogue32_staged<ROWB>(a.g, r, m0, first, bias, sg);
+        else
+          gemm_epilogue32<ROWB>(a.g, r, m, tn * a.nt + 32 * blk);
       }
       tc::fence_before();
       tc::mbar_arrive(&tempty[b]);
     }
+    gemm_fetch_wait();
     if (!ok) {
       *abort_flag = 1;
       if (lane == 0 && a.g.error) atomicExch(a.g.error, 1);
@@ -486,16 +533,21 @@ int launch_gemm_tn(const GemmArgs& g, int splits, cudaStream_t st) {
     return -1;
   GemmKernelArgs a;
   a.g = g;
-  a.nt = (g.N + 15) / 16 * 16;
+  // staged outputs in tiles of 128 columns: a block of 32 columns for each
+  // epilogue warp, and twice the tiles, which leave a smaller last wave
+  a.nt = gemm_staged(g) && g.N > 128 ? 128 : (g.N + 15) / 16 * 16;
+  a.tiles_n = (g.N + a.nt - 1) / a.nt;
   a.splits = splits;
   a.tiles_m = (g.M + 127) / 128;
   a.kper = g.K / splits;
   a.wait_limit = g.wait_limit > 0 ? g.wait_limit : wait_limit();
   const int stage_bytes = kGemmTileA + a.nt * kGemmBK * 2;
   const long long kchunks = a.kper / kGemmBK;
-  a.stages = (int)std::min<long long>(std::min(kGemmSmemBudget / stage_bytes, 8), std::max<long long>(kchunks, 2));
-  // the epilogue warps' staging tiles after the stages and the barriers
-  const size_t staging = (size_t)(kGemmEpilogueThreads / 32) * kGemmStageWords * sizeof(float);
+  const int budget = gemm_staged(g) ? kGemmSmemBudgetStaged : kGemmSmemBudget;
+  a.stages = (int)std::min<long long>(std::min(budget / stage_bytes, 8), std::max<long long>(kchunks, 2));
+  // the bias and the epilogue warps' staging tiles after the stages and the barriers
+  const size_t staging =
+      256 * sizeof(float) + (gemm_staged(g) ? (size_t)kGemmEpilogueWarps * kGemmStageWords * sizeof(float) : 0);
   CUtensorMap mapA, mapB;
   if (!make_map(&mapA, g.A, g.M, g.K, g.lda, 128) || !make_map(&mapB, g.B, g.N, g.K, g.ldb, a.nt)) return -1;
   size_t smem = 1024 + (size_t)a.stages * stage_bytes + 1024 + staging;
@@ -508,7 +560,7 @@ int launch_gemm_tn(const GemmArgs& g, int splits, cudaStream_t st) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return -1;
-  const long long ntiles = (long long)a.tiles_m * splits;
+  const long long ntiles = (long long)a.tiles_m * a.tiles_n * splits;
   const unsigned grid = (unsigned)std::min<long long>(ntiles, sms);
   kernel<<<grid, kGemmThreads, smem, st>>>(mapA, mapB, a);
   return 0;
