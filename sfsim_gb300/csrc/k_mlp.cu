@@ -62,40 +62,62 @@ __global__ void k_features(long long n, const float* __restrict__ coords, __nv_b
   }
 }
 
-// out[i][c] = sum_j H[i][j] W5[c][j] + b5[c], c < kMlpOut; one warp per row,
-// each lane one 16-byte load of eight BF16 (kMlpHidden == 256), W5 staged in
-// shared memory.
-static_assert(kMlpHidden == 256, "k_head_forward reads a row as 32 lanes x 8 BF16");
-__global__ void k_head_forward(long long n, const __nv_bfloat16* __restrict__ H, const float* __restrict__ W5,
-                               const float* __restrict__ b5, float* __restrict__ out) {
-  __shared__ float sW[kMlpOut * kMlpHidden];
-  for (int t = threadIdx.x; t < kMlpOut * kMlpHidden; t += blockDim.x) sW[t] = W5[t];
-  __syncthreads();
-  const long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+// Head: out[i][c] = H4[i] . W5[c] + b5[c].  A lane keeps its 8 columns of W5 in
+// registers and the warp walks rows, two at a time; the eight sums are reduced
+// together, each exchange halving the values a lane still carries (9 shuffles
+// for two rows).  With the weights read from shared memory for every row and
+// 20 shuffles a row, 65536 rows took 27 us; now 17.
+static_assert(kMlpHidden == 256 && kMlpOut == 4, "k_head_forward reads a row as 32 lanes x 8 BF16, four sums a row");
+constexpr int kHeadRows = 2;
+__global__ void __launch_bounds__(256) k_head_forward(long long n, const __nv_bfloat16* __restrict__ H,
+                                                      const float* __restrict__ W5, const float* __restrict__ b5,
+                                                      float* __restrict__ out) {
   const int lane = threadIdx.x & 31;
-  if (row >= n) return;
-  const uint4 q = *reinterpret_cast<const uint4*>(H + row * kMlpHidden + 8 * lane);
-  const uint32_t wq[4] = {q.x, q.y, q.z, q.w};
-  float h[8];
+  float w[kMlpOut][8];
 #pragma unroll
-  for (int e = 0; e < 4; e++) {
-    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wq[e]));
-    h[2 * e] = f.x;
-    h[2 * e + 1] = f.y;
-  }
-  float acc[kMlpOut];
+  for (int c = 0; c < kMlpOut; c++)
 #pragma unroll
-  for (int c = 0; c < kMlpOut; c++) {
-    const float* w = sW + c * kMlpHidden + 8 * lane;
-    float a = 0;
+    for (int e = 0; e < 8; e++) w[c][e] = W5[c * kMlpHidden + 8 * lane + e];
+  const float bias = b5[lane >> 2 & 3];
+  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long row = kHeadRows * ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5); row < n;
+       row += kHeadRows * warps) {
+    float v[8];  // row 0's four sums, then row 1's
 #pragma unroll
-    for (int e = 0; e < 8; e++) a = fmaf(h[e], w[e], a);
-    acc[c] = a;
-  }
+    for (int r = 0; r < kHeadRows; r++) {
+      const long long i = row + r < n ? row + r : n - 1;
+      const uint4 q = *reinterpret_cast<const uint4*>(H + i * kMlpHidden + 8 * lane);
+      const uint32_t wq[4] = {q.x, q.y, q.z, q.w};
+      float h[8];
 #pragma unroll
-  for (int c = 0; c < kMlpOut; c++) {
-    for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-    if (lane == 0) out[row * kMlpOut + c] = acc[c] + b5[c];
+      for (int e = 0; e < 4; e++) {
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wq[e]));
+        h[2 * e] = f.x;
+        h[2 * e + 1] = f.y;
+      }
+#pragma unroll
+      for (int c = 0; c < kMlpOut; c++) {
+        float a = 0;
+#pragma unroll
+        for (int e = 0; e < 8; e++) a = fmaf(h[e], w[c][e], a);
+        v[4 * r + c] = a;
+      }
+    }
+    // lanes with bit 16, 8, 4 set keep the upper half of the values
+#pragma unroll
+    for (int o = 16, k = 4; k > 0; o >>= 1, k >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int e = 0; e < k; e++) {
+        const float keep = up ? v[e + k] : v[e], give = up ? v[e] : v[e + k];
+        v[e] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    // lane 4 k holds value k: row k / 4, output k % 4
+    const long long i = row + (lane >> 4);
+    if ((lane & 3) == 0 && i < n) out[i * kMlpOut + (lane >> 2 & 3)] = v[0] + bias;
   }
 }
 
@@ -131,66 +153,85 @@ __global__ void k_loss_grad(long long n, const float* __restrict__ out, const fl
 static_assert(kMlpOut == 4, "the head kernels read rows of dout as float4");
 
 // Backward of the head: dZ4[i][j] = (sum_c dout[i][c] W5[c][j]) * dsilu4[i][j]
-// (BF16, also transposed), and dW5 += dout^T H4, db5 += sum dout.  Thread j
-// of a block handles hidden unit j over the block's rows, 32 rows at a time:
-// the tile of 32 x 256 BF16 gradients passes through shared memory so that
-// each thread writes 32 consecutive entries of one transposed row (64 bytes)
-// instead of 32 scattered 2-byte values.  The rows of a block start at a
-// multiple of 32 (n is a multiple of 1024).
+// (BF16, also transposed), and dW5 += dout^T H4, db5 += sum dout.  A block
+// takes 32 rows at a time; a thread handles two neighbouring hidden units of
+// every second row, so that a warp's loads and stores are of whole lines.  The tile of 32 x 256
+// BF16 gradients passes through shared memory so that each thread writes 32
+// consecutive entries of one transposed row (64 bytes) instead of 32 scattered
+// 2-byte values.  The rows of a block start at a multiple of 32 (n is a
+// multiple of 1024).  What bounds it: memory, 167 MB for 65536 rows (24 us).
+// With one unit a thread, 2-byte accesses and 1024 blocks that all add to dW5
+// it took 66 us; now 49 (304, 608 and 1216 blocks: a batch of 65536 in 727, 700 and
+// 698 us).
 constexpr int kHeadTile = 32;
-__global__ void k_head_backward(long long n, const float* __restrict__ dout, const __nv_bfloat16* __restrict__ H,
-                                const float* __restrict__ W5, const float* __restrict__ dsilu,
-                                __nv_bfloat16* __restrict__ dZ, __nv_bfloat16* __restrict__ dZT,
-                                float* __restrict__ dW5, float* __restrict__ db5) {
-  __shared__ float sW[kMlpOut * kMlpHidden];
+__global__ void __launch_bounds__(kMlpHidden)
+    k_head_backward(long long n, const float* __restrict__ dout, const __nv_bfloat16* __restrict__ H,
+                    const float* __restrict__ W5, const float* __restrict__ dsilu, __nv_bfloat16* __restrict__ dZ,
+                    __nv_bfloat16* __restrict__ dZT, float* __restrict__ dW5, float* __restrict__ db5) {
   // [row][unit], 8 BF16 of padding a row: column reads hit 16 banks, one word per lane pair
   __shared__ __align__(16) __nv_bfloat16 tile[kHeadTile][kMlpHidden + 8];
-  for (int t = threadIdx.x; t < kMlpOut * kMlpHidden; t += blockDim.x) sW[t] = W5[t];
-  __syncthreads();
-  const int j = threadIdx.x;  // blockDim.x == kMlpHidden
+  __shared__ float part[kMlpOut][kMlpHidden];
+  const int c2 = 2 * (threadIdx.x & (kMlpHidden / 2 - 1)), half = threadIdx.x / (kMlpHidden / 2);
+  float2 w[kMlpOut];
+#pragma unroll
+  for (int c = 0; c < kMlpOut; c++) w[c] = *reinterpret_cast<const float2*>(W5 + c * kMlpHidden + c2);
   const long long tiles = n / kHeadTile;
-  const long long tiles_per_block = (tiles + gridDim.x - 1) / gridDim.x;
-  const long long t0 = blockIdx.x * tiles_per_block, t1 = min(tiles, t0 + tiles_per_block);
-  float gw[kMlpOut] = {}, gb[kMlpOut] = {};
-  for (long long tl = t0; tl < t1; tl++) {
+  float2 gw[kMlpOut] = {};
+  float gb[kMlpOut] = {};
+  for (long long tl = blockIdx.x; tl < tiles; tl += gridDim.x) {
     const long long i0 = tl * kHeadTile;
 #pragma unroll 8
-    for (int ii = 0; ii < kHeadTile; ii++) {
+    for (int ii = half; ii < kHeadTile; ii += 2) {
       const long long i = i0 + ii;
       const float4 d = *reinterpret_cast<const float4*>(dout + i * kMlpOut);
       const float dd[kMlpOut] = {d.x, d.y, d.z, d.w};
-      const float h = __bfloat162float(H[i * kMlpHidden + j]);
-      float dh = 0;
+      const float2 h = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(H + i * kMlpHidden + c2));
+      const float2 ds = *reinterpret_cast<const float2*>(dsilu + i * kMlpHidden + c2);
+      float2 dh = make_float2(0.0f, 0.0f);
 #pragma unroll
       for (int c = 0; c < kMlpOut; c++) {
-        gw[c] = fmaf(dd[c], h, gw[c]);
+        gw[c].x = fmaf(dd[c], h.x, gw[c].x);
+        gw[c].y = fmaf(dd[c], h.y, gw[c].y);
         gb[c] += dd[c];
-        dh = fmaf(dd[c], sW[c * kMlpHidden + j], dh);
+        dh.x = fmaf(dd[c], w[c].x, dh.x);
+        dh.y = fmaf(dd[c], w[c].y, dh.y);
       }
-      const __nv_bfloat16 dz = __float2bfloat16(dh * dsilu[i * kMlpHidden + j]);
-      dZ[i * kMlpHidden + j] = dz;
-      tile[ii][j] = dz;
+      const __nv_bfloat162 dz = __floats2bfloat162_rn(dh.x * ds.x, dh.y * ds.y);
+      *reinterpret_cast<__nv_bfloat162*>(dZ + i * kMlpHidden + c2) = dz;
+      *reinterpret_cast<__nv_bfloat162*>(&tile[ii][c2]) = dz;
     }
     __syncthreads();
     // transposed row j, entries i0 .. i0 + 31: four 16-byte stores
+    const int j = threadIdx.x;  // blockDim.x == kMlpHidden
     uint4* dst = reinterpret_cast<uint4*>(dZT + (long long)j * n + i0);
 #pragma unroll
     for (int q = 0; q < kHeadTile / 8; q++) {
-      uint32_t w[4];
+      uint32_t t[4];
 #pragma unroll
       for (int e = 0; e < 4; e++) {
         __nv_bfloat162 pr;
         pr.x = tile[8 * q + 2 * e][j];
         pr.y = tile[8 * q + 2 * e + 1][j];
-        w[e] = *reinterpret_cast<const uint32_t*>(&pr);
+        t[e] = *reinterpret_cast<const uint32_t*>(&pr);
       }
-      dst[q] = make_uint4(w[0], w[1], w[2], w[3]);
+      dst[q] = make_uint4(t[0], t[1], t[2], t[3]);
     }
     __syncthreads();
   }
+  // the two halves of the rows, then one addition a block
+  if (half == 1) {
 #pragma unroll
-  for (int c = 0; c < kMlpOut; c++) atomicAdd(dW5 + c * kMlpHidden + j, gw[c]);
-  if (j == 0) {
+    for (int c = 0; c < kMlpOut; c++) *reinterpret_cast<float2*>(&part[c][c2]) = gw[c];
+  }
+  __syncthreads();
+  if (half == 0) {
+#pragma unroll
+    for (int c = 0; c < kMlpOut; c++) {
+      const float2 o = *reinterpret_cast<const float2*>(&part[c][c2]);
+      atomicAdd(reinterpret_cast<float2*>(dW5 + c * kMlpHidden + c2), make_float2(gw[c].x + o.x, gw[c].y + o.y));
+    }
+  }
+  if (c2 == 0) {
 #pragma unroll
     for (int c = 0; c < kMlpOut; c++) atomicAdd(db5 + c, gb[c]);
   }
@@ -371,7 +412,9 @@ void launch_features(long long n, const float* coords, __nv_bfloat16* F, __nv_bf
 }
 void launch_head_forward(long long n, const __nv_bfloat16* H, const float* W5, const float* b5, float* out,
                          cudaStream_t st) {
-  k_head_forward<<<grid_for(n * 32, 256), 256, 0, st>>>(n, H, W5, b5, out);
+  // eight rows a warp or more, where the rows are many
+  const long long blocks = (n + 8 * kHeadRows - 1) / (8 * kHeadRows);
+  k_head_forward<<<(unsigned)min(blocks, 1216LL), 256, 0, st>>>(n, H, W5, b5, out);
 }
 void launch_loss_grad(long long n, const float* out, const float* target, float huber, float var_weight, float* dout,
                       float* loss, cudaStream_t st) {
@@ -380,7 +423,7 @@ void launch_loss_grad(long long n, const float* out, const float* target, float 
 void launch_head_backward(long long n, const float* dout, const __nv_bfloat16* H, const float* W5,
                           const float* dsilu, __nv_bfloat16* dZ, __nv_bfloat16* dZT, float* dW5, float* db5,
                           cudaStream_t st) {
-  const int blocks = (int)min(1024LL, (n / kHeadTile + 1) / 2);
+  const int blocks = (int)min(608LL, n / kHeadTile);
   k_head_backward<<<blocks, kMlpHidden, 0, st>>>(n, dout, H, W5, dsilu, dZ, dZT, dW5, db5);
 }
 void launch_bias_grad(long long n, int width, const __nv_bfloat16* dZT, float* db, cudaStream_t st) {
