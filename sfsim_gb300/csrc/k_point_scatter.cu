@@ -32,6 +32,7 @@
 // shuffles and every heading walked, it was 7.08 ms.  The 16 atmospheres of a
 // sweep (16x128x16x8) went from 11.8 to 5.3 to 4.6 ms, the reference's tables
 // (32x127x32x8, 71 directions) from 0.96 to 0.47 to 0.41 ms.
+#include <algorithm>
 #include <type_traits>
 
 #include "atmo_device.cuh"
@@ -104,6 +105,7 @@ struct HeadingPair {
 };
 
 constexpr int kPointThreads = 128;
+constexpr int kPointSlices = 8;  // at most
 
 // Blocks per SM the registers are limited for.  Three heading pairs measured
 // 3.11 / 2.96 / 3.04 / 3.25 ms of a production build (5 launches) at 2 / 3 /
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     k_point_scatter(const AtmoParams* params, BuildDims d, PointLayout lay, const RowInfo* rowinfo,
                     const SphereRing<Real>* rings, const Real* dirs4, const Real* offsets,
                     const PointRow<Real>* prow, const CellGeom<Real>* geom, const Vec4<Real>* dS, const Vec4<Real>* Mt, const Vec4<Real>* dE,
-                    Vec4<Real>* J, int groups, int chunks) {
+                    Vec4<Real>* J, int groups, int chunks, int slices) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using R2 = V2<Real>;
   constexpr int KS = row_stride<FIRST>();
@@ -298,8 +300,10 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
 
   // this thread's elevation and headings; a thread past the last item repeats it and stores nothing
   const int items = d.n1 * groups;
-  const int item_raw = chunk * nt + tid;
-  const bool valid = item_raw < items;
+  // the directions of every ring go to `slices` threads an item in turn (then all items are in one block)
+  const int slice = slices > 1 ? tid / items : 0;
+  const int item_raw = slices > 1 ? tid - slice * items : chunk * nt + tid;
+  const bool valid = item_raw < items && slice < slices;
   const int item = valid ? item_raw : items - 1;
   const int grp = item / d.n1, j = item - grp * d.n1;
   const int a0 = 1 + grp * 2 * HP;  // its headings a0 .. a0 + 2 HP - 1, those below n3 - 1
@@ -329,8 +333,8 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     const R2 c0 = dup(rc.x0 * lx);
     const Real mv0 = sv * rc.x0;
     const int n = rc.n;
-    const Real* x = sdirs + 4 * rc.w0;
-    const Real* e = sedge + 8 * rc.w0;
+    const Real* x = sdirs + 4 * (rc.w0 + slice);
+    const Real* e = sedge + 8 * (rc.w0 + slice);
     // beta_c(x) (atmosphere.clj:42-47, 140-151) times the ring's weight
     Real bR[3], bM[3];
 #pragma unroll
@@ -344,7 +348,7 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
       t.z = fma2(dup(wz), X.z, t.z);
     };
     auto walk = [&](auto ground) {
-      for (int m = 0; m < n; m++, x += 4, e += 8) {
+      for (int m = slice; m < n; m += slices, x += 4 * slices, e += 8 * slices) {
         R2 x1, x2;
         ld_pairs(x, x1, x2);
         const Real mv = fma(cv, x1.x, mv0);
@@ -374,7 +378,28 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
       tot[h].z = add2(tot[h].z, sum[h].z);
     }
   }
-  if (!valid) return;
+  if (slices > 1) {
+    // the slices' sums, in order
+    HeadingPair<Real>* sums = reinterpret_cast<HeadingPair<Real>*>(smem_raw);
+    __syncthreads();
+    if (valid && slice > 0) {
+#pragma unroll
+      for (int h = 0; h <= HP; h++) sums[((slice - 1) * (HP + 1) + h) * items + item] = tot[h];
+    }
+    __syncthreads();
+    if (slice == 0) {
+      for (int q = 0; q < (slices - 1); q++) {
+#pragma unroll
+        for (int h = 0; h <= HP; h++) {
+          const HeadingPair<Real> o = sums[(q * (HP + 1) + h) * items + item];
+          tot[h].a = add2(tot[h].a, o.a);
+          tot[h].b = add2(tot[h].b, o.b);
+          tot[h].z = add2(tot[h].z, o.z);
+        }
+      }
+    }
+  }
+  if (!valid || slice > 0) return;
   auto put = [&](int at, R2 xy, Real z) {
     Vec4<Real> o;
     o.x = xy.x;
@@ -414,19 +439,32 @@ int launch_point_scatter(const AtmoParams* params, const BuildDims& d, const Row
                          const PointRow<Real>* prow, const CellGeom<Real>* geom, const Vec4<Real>* dS, const Vec4<Real>* mie, const Vec4<Real>* dE,
                          Vec4<Real>* J, cudaStream_t st) {
   const bool first = mie != nullptr;
-  const PointLayout lay = point_layout<Real>(d, first);
+  PointLayout lay = point_layout<Real>(d, first);
   const int inner = d.n3 - 2;
   int hp = sizeof(Real) == 8 ? 1 : inner > 4 ? 3 : inner > 2 ? 2 : 1;
   const int groups = inner > 0 ? (inner + 2 * hp - 1) / (2 * hp) : 1;
   const int items = d.n1 * groups;
   const int chunks = (items + kPointThreads - 1) / kPointThreads;
-  const int block = ((items + chunks - 1) / chunks + 31) / 32 * 32;
+  int block = ((items + chunks - 1) / chunks + 31) / 32 * 32;
+  // Few elevations leave a warp's lanes unused, and in a small build most of
+  // the warps that an SM holds: then several threads share an item's
+  // directions.  16 elevations, 4 headings, 8 heights and sun elevations, two
+  // iterations: FP32 46 us with 1 thread an item, 31 with 4, 27 with 8; FP64
+  // 885, 305 and 219.
+  const bool few = (long long)d.n0 * d.n2 * chunks * d.B * (block / 32) < 1824;  // 12 warps an SM
+  int slices = 1;
+  while (chunks == 1 && 2 * slices * items <= kPointThreads && slices < kPointSlices && (few || slices * items < 32))
+    slices *= 2;
+  if (slices > 1) {
+    block = (slices * items + 31) / 32 * 32;
+    lay.bytes = std::max<unsigned>(lay.bytes, sizeof(HeadingPair<Real>) * (hp + 1) * items * (slices - 1));
+  }
   const dim3 grid((unsigned)(d.n0 * d.n2 * chunks), d.B);
   auto go = [&](auto kernel) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.bytes) != cudaSuccess)
       return -1;
     kernel<<<grid, block, lay.bytes, st>>>(params, d, lay, rowinfo, rings, dirs4, offsets, prow, geom, dS, mie,
-                                           dE, J, groups, chunks);
+                                           dE, J, groups, chunks, slices);
     return 0;
   };
   if constexpr (std::is_same<Real, float>::value) {
