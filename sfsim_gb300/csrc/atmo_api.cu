@@ -541,12 +541,12 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
               Timer& tm, const sfsim_atmo_intermediates* inter, Vec4<float>* jsum = nullptr,
               cudaEvent_t early_done = nullptr, const IterationHooks* hooks = nullptr) {
   int launches = 0;
-  // The first order needs the sun tables, the rows (row info, point rows)
+  // The first order needs the sun rays' fits, the rows (row info, point rows)
   // and the view-row samples; each of its blocks forms its cells' light
   // directions itself (as k_remap4 does).  So the build stream runs the rows
-  // and the view-row samples, the side stream the sun tables and then the
-  // node maps (remap4), the other set-up tables, the transmittance nodes and
-  // E0 beside the first order; the outputs and the iterations wait for all
+  // and the view-row samples, the side stream the fits, the other set-up
+  // tables with the transmittance nodes and E0, and then the node maps
+  // (remap4) beside the first order; the outputs and the iterations wait for all
   // of them.  Builds with stage timing on, entry points without a side
   // stream, and rows whose cells' geometry does not fit beside their samples
   // in shared memory keep the node maps before the first order.
@@ -565,24 +565,34 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
     }
     CUDA_TRY(cudaEventRecord(g_side_sun[tm.dev], ss));
   }
+  auto tables = [&](unsigned which, cudaStream_t on) {
+    launch_setup_tables<Real>(w.params, d, w.dirs, w.hdirs, w.setup, w.T, w.E0, which, on);
+    launches++;
+  };
+  constexpr unsigned T_part = 1u << kPartTransmittance, E0_part = 1u << kPartBase;
   tm.mark_begin(0);
-  launch_setup_rows<Real>(w.params, d, w.setup, st);
+  if (setup_fork) {
+    tables(kSetupRows, st);
+    tables(kSetupRest | T_part | E0_part, ss);
+  } else {
+    tables(kSetupRows | kSetupRest, st);
+  }
   if (cells) {
     CUDA_TRY(cudaEventRecord(g_side_rows[tm.dev], st));
     CUDA_TRY(cudaStreamWaitEvent(ss, g_side_rows[tm.dev], 0));
   }
   launch_node_maps<Real>(w.params, d, w.setup, cells ? ss : st);
   launch_view_rows<Real>(w.params, d, w.setup, st);
-  launches += 4 + launch_setup_aux<Real>(w.params, d, w.dirs, w.hdirs, w.setup, sa);
+  launches += 2 + launch_surface_weights<Real>(w.params, d, w.setup, sa);
   tm.mark_end();
-  tm.mark_begin(1, sa);
-  launch_transmittance<Real>(w.params, d, w.T, sa);
-  launches++;
-  tm.mark_end(sa);
-  tm.mark_begin(2, sa);
-  launch_surface_base<Real>(w.params, d, w.E0, sa);
-  launches++;
-  tm.mark_end(sa);
+  if (!setup_fork) {
+    tm.mark_begin(1);
+    tables(T_part, st);
+    tm.mark_end();
+    tm.mark_begin(2);
+    tables(E0_part, st);
+    tm.mark_end();
+  }
   if (setup_fork) {
     CUDA_TRY(cudaEventRecord(g_side_setup[tm.dev], ss));
     CUDA_TRY(cudaStreamWaitEvent(st, (cells ? g_side_sun : g_side_setup)[tm.dev], 0));
@@ -919,7 +929,10 @@ int census_impl(const sfsim_atmo_config& cfg, unsigned long long* out, int n) {
     CUDA_TRY(cudaMemcpyAsync(w.dirs, dirs.data(), sizeof(DirLocal) * dirs.size(), cudaMemcpyHostToDevice, st));
   }
   CUDA_TRY(cudaMemsetAsync(dcount, 0, 2 * sizeof(unsigned long long), st));
-  launch_setup<Real>(w.params, d, w.dirs, w.hdirs, w.setup, st);
+  launch_setup_tables<Real>(w.params, d, w.dirs, w.hdirs, w.setup, w.T, w.E0, kSetupRows | kSetupRest, st);
+  launch_node_maps<Real>(w.params, d, w.setup, st);
+  launch_view_rows<Real>(w.params, d, w.setup, st);
+  launch_surface_weights<Real>(w.params, d, w.setup, st);
   launch_sphere_dirs<Real>(w.params, d, w.dirs, dsd, st);
   launch_first_order_census<Real>(w.params, d, w.setup.rowinfo, w.setup.rows, w.setup.geom, dcount, st);
   CUDA_TRY(cudaGetLastError());

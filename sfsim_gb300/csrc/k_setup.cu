@@ -17,11 +17,9 @@ namespace sfsim {
 // Per view row (i, j), once: the row's geometry (RowInfo) and its height and
 // elevation coordinates, which every node and ray sample of the row shares.
 template <class Real>
-__global__ void k_row_info(const AtmoParams* params, BuildDims d, RowInfo* info, Remap2<Real>* rowmap) {
+__device__ void row_info(const AtmoParams* params, const BuildDims& d, RowInfo* info, Remap2<Real>* rowmap,
+                         long long row, int b) {
   const long long nrows = d.rows();
-  const long long row = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const int b = blockIdx.y;
-  if (row >= nrows) return;
   const AtmoParams& P = params[b];
   const int j = (int)(row % d.n1), i = (int)(row / d.n1);
   double r, sv, cv;
@@ -87,11 +85,8 @@ __global__ void k_remap4(BuildDims d, const RowInfo* info, const PointRow<Real>*
 }
 
 template <class Real>
-__global__ void k_remapT(const AtmoParams* params, BuildDims d, Remap2<Real>* out) {
+__device__ void remap_T(const AtmoParams* params, const BuildDims& d, Remap2<Real>* out, long long node, int b) {
   const long long n = d.nT();
-  const long long node = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const int b = blockIdx.y;
-  if (node >= n) return;
   const AtmoParams& P = params[b];
   int j = (int)(node % d.nT1), i = (int)(node / d.nT1);
   double r = index_to_radius(P, d.nT0, (double)i), sv, cv;
@@ -113,11 +108,8 @@ __host__ __device__ inline void surface_node(const AtmoParams& P, const BuildDim
 }
 
 template <class Real>
-__global__ void k_remapE(const AtmoParams* params, BuildDims d, Remap2<Real>* out) {
+__device__ void remap_E(const AtmoParams* params, const BuildDims& d, Remap2<Real>* out, long long node, int b) {
   const long long n = d.nE();
-  const long long node = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const int b = blockIdx.y;
-  if (node >= n) return;
   const AtmoParams& P = params[b];
   int k = (int)(node % d.nE1), i = (int)(node / d.nE1);
   d3 x, l;
@@ -133,11 +125,8 @@ __global__ void k_remapE(const AtmoParams* params, BuildDims d, Remap2<Real>* ou
 // ---------------------------------------------------------------------------
 
 template <class Real>
-__global__ void k_transmittance(const AtmoParams* params, BuildDims d, Vec4<Real>* T) {
+__device__ void transmittance_node(const AtmoParams* params, const BuildDims& d, Vec4<Real>* T, long long node, int b) {
   const long long n = d.nT();
-  const long long node = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const int b = blockIdx.y;
-  if (node >= n) return;
   const AtmoParams& P = params[b];
   int j = (int)(node % d.nT1), i = (int)(node / d.nT1);
   double r = index_to_radius(P, d.nT0, (double)i), sv, cv;
@@ -160,11 +149,8 @@ __global__ void k_transmittance(const AtmoParams* params, BuildDims d, Vec4<Real
 // ---------------------------------------------------------------------------
 
 template <class Real>
-__global__ void k_surface_base(const AtmoParams* params, BuildDims d, Vec4<Real>* E0) {
+__device__ void surface_base_node(const AtmoParams* params, const BuildDims& d, Vec4<Real>* E0, long long node, int b) {
   const long long n = d.nE();
-  const long long node = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const int b = blockIdx.y;
-  if (node >= n) return;
   const AtmoParams& P = params[b];
   int k = (int)(node % d.nE1), i = (int)(node / d.nE1);
   d3 x, l;
@@ -349,80 +335,89 @@ __global__ void k_view_rows_scan(const AtmoParams* params, BuildDims d, const Ro
 }
 
 // ---------------------------------------------------------------------------
+// Rings of the quadratures
+// ---------------------------------------------------------------------------
+
+// First direction of ring k of `rings` between polar angles 0 and `range`: the
+// directions follow one another by ring and their polar cosine falls from ring
+// to ring.
+__device__ inline int ring_start(const DirLocal* dirs, int count, int rings, double range, int k) {
+  if (k == 0) return 0;
+  if (k >= rings) return count;
+  const double edge = cos(range * k / rings);  // between rings k - 1 and k
+  int lo = 0, hi = count;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (dirs[mid].x < edge)
+      hi = mid;
+    else
+      lo = mid + 1;
+  }
+  return lo;
+}
+
+// ---------------------------------------------------------------------------
 // Sphere rings of point scatter per height row (atmosphere.clj:203-222,
 // sphere.clj:62-105): where the ring's directions end, whether that end is on
 // the ground, the elevation coordinate of the dS lookup and, for ground ends,
 // T(x, g) * brightness / pi.  x = (r, 0, 0), so the ring's directions have
 // the same first component and with it the same end; the ring's first
-// direction stands for all.  One block per height: a warp finds the rings in
-// the direction list (the directions of a ring follow one another and share
-// their polar cosine), then each warp takes a ring, its lanes the samples of
-// the ground's optical depth.
+// direction stands for all.  A warp takes a ring, its lanes the samples of the
+// ground's optical depth.
 // ---------------------------------------------------------------------------
 
 template <class Real>
-__global__ void __launch_bounds__(256) k_sphere_rings(const AtmoParams* params, BuildDims d, const DirLocal* dirs,
-                                                      SphereRing<Real>* out, Real* dirs4, Real* offsets) {
-  extern __shared__ int start[];  // first direction of each ring, and P
-  const int i = blockIdx.x, b = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0) {
-    int found = 0;
-    for (int t0 = 0; t0 < d.P; t0 += 32) {
-      const int t = t0 + lane;
-      const bool first = t < d.P && (t == 0 || dirs[t].x != dirs[t - 1].x);
-      const unsigned ballot = __ballot_sync(0xffffffffu, first);
-      const int pos = found + __popc(ballot & ((1u << lane) - 1u));
-      if (first && pos < d.T) start[pos] = t;
-      found += __popc(ballot);
-    }
-    if (lane == 0) start[d.T] = d.P;
-  }
-  __syncthreads();
+__device__ void sphere_ring(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs, SphereRing<Real>* out,
+                            int i, int k, int b, int lane) {
   const AtmoParams& P = params[b];
   const double r = index_to_radius(P, d.n0, (double)i);
   const d3 x = mk3(r, 0, 0);
   const d3 n = mul3(x, 1.0 / mag3(x));
   const d3 o1 = orthogonal(n);
   const d3 o2 = cross3(n, o1);
+  const int w = ring_start(dirs, d.P, d.T, M_PI, k);
+  const d3 omega = to_world(n, o1, o2, dirs[w]);
+  const d3 g = ray_extremity(P, x, omega);
+  const int surface = surface_point(P, g);
+  SphereRing<Real> o;
+  o.x0 = (Real)omega.x;
+  o.weight = (Real)dirs[w].w;
+  o.surface = surface;
+  o.w0 = w;
+  o.n = ring_start(dirs, d.P, d.T, M_PI, k + 1) - w;
+  split_coord<Real>(elevation_to_index(P, d.n1, x, omega, !surface), d.n1, &o.u1, &o.s1);
+  o.tR = o.ground[0] = o.ground[1] = o.ground[2] = 0;
+  if (surface) {
+    Real tau[3];
+    segment_depth_warp<Real>(P, x, sub3(g, x), d.S, lane, tau);
+    for (int c = 0; c < 3; c++) o.ground[c] = exp_neg(tau[c]) * (Real)(P.brightness[c] / M_PI);
+    const double tR = mag3(sub3(g, x)) / P.R;
+    o.tR = tR < 1.0e30 ? (Real)tR : Real(0);  // point scatter forms table indices from it
+  }
+  if (lane == 0) out[((long long)b * d.n0 + i) * d.T + k] = o;
+}
+
+// Per direction: its components across the axis (the same at every height),
+// and in FP64 builds the ground point's height coordinate, which is on the
+// ground up to its rounding.
+template <class Real>
+__device__ void sphere_direction(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs, Real* dirs4,
+                                 Real* offsets, int i, int t, int b) {
+  const AtmoParams& P = params[b];
+  const d3 x = mk3(index_to_radius(P, d.n0, (double)i), 0, 0);
+  const d3 n = mul3(x, 1.0 / mag3(x));
+  const d3 o1 = orthogonal(n);
+  const d3 omega = to_world(n, o1, cross3(n, o1), dirs[t]);
   if (i == 0 && b == 0) {
-    for (int t = threadIdx.x; t < d.P; t += blockDim.x) {
-      const d3 omega = to_world(n, o1, o2, dirs[t]);
-      dirs4[4 * t] = dirs4[4 * t + 1] = (Real)omega.y;
-      dirs4[4 * t + 2] = dirs4[4 * t + 3] = (Real)omega.z;
-    }
+    dirs4[4 * t] = dirs4[4 * t + 1] = (Real)omega.y;
+    dirs4[4 * t + 2] = dirs4[4 * t + 3] = (Real)omega.z;
   }
   if (std::is_same<Real, double>::value) {
-    // per direction: the ground point is on the ground up to its rounding
-    for (int t = threadIdx.x; t < d.P; t += blockDim.x) {
-      const d3 g = ray_extremity(P, x, to_world(n, o1, o2, dirs[t]));
-      int u = 0;
-      Real s = 0;
-      if (surface_point(P, g)) split_coord<Real>(height_to_index(P, d.nE0, mag3(g)), d.nE0, &u, &s);
-      offsets[((long long)b * d.n0 + i) * d.P + t] = s;
-    }
-  }
-  for (int k = warp; k < d.T; k += blockDim.x >> 5) {
-    const int w = start[k];
-    const d3 omega = to_world(n, o1, o2, dirs[w]);
     const d3 g = ray_extremity(P, x, omega);
-    const int surface = surface_point(P, g);
-    SphereRing<Real> o;
-    o.x0 = (Real)omega.x;
-    o.weight = (Real)dirs[w].w;
-    o.surface = surface;
-    o.w0 = w;
-    o.n = start[k + 1] - w;
-    split_coord<Real>(elevation_to_index(P, d.n1, x, omega, !surface), d.n1, &o.u1, &o.s1);
-    o.tR = o.ground[0] = o.ground[1] = o.ground[2] = 0;
-    if (surface) {
-      Real tau[3];
-      segment_depth_warp<Real>(P, x, sub3(g, x), d.S, lane, tau);
-      for (int c = 0; c < 3; c++) o.ground[c] = exp_neg(tau[c]) * (Real)(P.brightness[c] / M_PI);
-      const double tR = mag3(sub3(g, x)) / P.R;
-      o.tR = tR < 1.0e30 ? (Real)tR : Real(0);  // point scatter forms table indices from it
-    }
-    if (lane == 0) out[((long long)b * d.n0 + i) * d.T + k] = o;
+    int u = 0;
+    Real s = 0;
+    if (surface_point(P, g)) split_coord<Real>(height_to_index(P, d.nE0, mag3(g)), d.nE0, &u, &s);
+    offsets[((long long)b * d.n0 + i) * d.P + t] = s;
   }
 }
 
@@ -472,15 +467,7 @@ __global__ void k_sphere_setup(const AtmoParams* params, BuildDims d, const DirL
 // sun at elevation k, and beta_c(x) (atmosphere.clj:42-47, 140-151), in FP64
 // once here instead of in every thread of the point-scatter blocks.
 template <class Real>
-__global__ void k_point_rows(const AtmoParams* params, BuildDims d, PointRow<Real>* out, double* hdvs) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int b = blockIdx.y;
-  if (b == 0) {
-    // v.l of heading a as index_to_sun_direction forms it, for every atmosphere
-    const int nt = gridDim.x * blockDim.x;
-    for (int a = t; a < d.n3; a += nt) hdvs[a] = dsub(dmul(2.0, (double)a / (d.n3 - 1)), 1.0);
-  }
-  if (t >= d.n0 * d.n2) return;
+__device__ void point_row(const AtmoParams* params, const BuildDims& d, PointRow<Real>* out, int t, int b) {
   const AtmoParams& P = params[b];
   const int i = t / d.n2, k = t % d.n2;
   const double r = index_to_radius(P, d.n0, (double)i);
@@ -502,17 +489,144 @@ __global__ void k_point_rows(const AtmoParams* params, BuildDims d, PointRow<Rea
   out[(long long)b * d.n0 * d.n2 + t] = o;
 }
 
+// The world frame of the directions at x = (r, 0, 0), whatever r.
+struct Frame {
+  d3 n, o1, o2;
+  __device__ Frame() : n(mk3(1, 0, 0)), o1(orthogonal(n)), o2(cross3(n, o1)) {}
+  __device__ d3 world(const DirLocal& q) const { return to_world(n, o1, o2, q); }
+};
+
+// Surface radiance's tables that do not depend on the light's direction
+// (k_surface.cu), in this order: nodes,
+// elevation coordinates per (height, ring), and once for all atmospheres the
+// rings and the directions.
+template <class Real>
+__device__ void surface_row(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs,
+                            const SetupBuffers<Real>& o, long long t, int b) {
+  const AtmoParams& P = params[b];
+  if (t < d.nE()) {
+    const double r = index_to_radius(P, d.nE0, (double)(t / d.nE1));
+    const double ss = index_to_sin_sun_elevation(d.nE1, (double)(t % d.nE1));
+    const d3 x = mk3(r, 0, 0), l = mk3(ss, sqrt(dmax(0.0, 1 - sqr(ss))), 0);
+    SurfRow<Real> row;
+    split_coord<Real>(height_to_index(P, d.n0, mag3(x)), d.n0, &row.u0, &row.s0);
+    split_coord<Real>(sun_elevation_to_index(d.n2, x, l), d.n2, &row.u2, &row.s2);
+    row.lx = (Real)l.x;
+    row.ly = (Real)l.y;
+    o.erow[(long long)b * d.nE() + t] = row;
+    return;
+  }
+  t -= d.nE();
+  if (t < (long long)d.nE0 * d.Th) {
+    const int i = (int)(t / d.Th), k = (int)(t - (long long)i * d.Th);
+    const d3 x = mk3(index_to_radius(P, d.nE0, (double)i), 0, 0);
+    Coord<Real> c;
+    split_coord<Real>(elevation_to_index(P, d.n1, x, Frame().world(dirs[ring_start(dirs, d.Ph, d.Th, M_PI / 2, k)]), 1), d.n1, &c.u,
+                      &c.s);
+    o.half_rows[(long long)b * d.nE0 * d.Th + t] = c;
+    return;
+  }
+  t -= (long long)d.nE0 * d.Th;
+  if (b > 0) return;
+  if (t <= d.Th) {
+    HalfRing<Real> ring{};
+    ring.w0 = ring_start(dirs, d.Ph, d.Th, M_PI / 2, (int)t);
+    if (t < d.Th) {
+      const double x0 = Frame().world(dirs[ring.w0]).x;
+      ring.x0 = (Real)x0;
+      ring.weight = (Real)(dirs[ring.w0].w * x0);
+    }
+    o.half_rings[t] = ring;
+    return;
+  }
+  t -= d.Th + 1;
+  if (t < d.Ph) o.half_y[t] = (Real)Frame().world(dirs[t]).y;
+}
+
+__host__ __device__ inline long long surface_row_items(const BuildDims& d) {
+  // a build without iterations may ask for no directions (ray steps below 4)
+  return d.nE() + (d.Th > 0 ? (long long)d.nE0 * d.Th + d.Th + 1 + d.Ph : 0);
+}
+
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
 
 static inline dim3 grid1(long long n, int block, int B) { return dim3((unsigned)((n + block - 1) / block), B); }
 
+// The set-up tables that need nothing but the parameters and the quadrature
+// directions, in one launch: they are FP64 chains of 10 to 25 us each (small
+// tables), and nine launches one after another held the iterations of a small
+// build back by 150 of its 260 us; now 162 us (8x16x8x4 tables, FP32).  Blocks
+// of one warp, so that what work there is spreads over the SMs' FP64 units.
+// Where the work is large (16 atmospheres of 16x128x16x8) they take as long as
+// they did apart, 1.9 ms with the maps and view rows, bound by FP64.
+struct SetupParts {
+  int blocks[kSetupParts];  // blocks of each part, 0 where it is not asked for
+};
+
 template <class Real>
-void launch_setup_rows(const AtmoParams* params, const BuildDims& d, const SetupBuffers<Real>& o, cudaStream_t st) {
-  const int blk = 128;
-  k_row_info<Real><<<grid1(d.rows(), blk, d.B), blk, 0, st>>>(params, d, o.rowinfo, o.rowmap);
-  k_point_rows<Real><<<grid1((long long)d.n0 * d.n2, blk, d.B), blk, 0, st>>>(params, d, o.prow, o.hdvs);
+__global__ void __launch_bounds__(32)
+    k_setup_tables(const AtmoParams* params, BuildDims d, const DirLocal* dirs, const DirLocal* half_dirs,
+                   SetupBuffers<Real> o, Vec4<Real>* T, Vec4<Real>* E0, SetupParts parts) {
+  const int b = blockIdx.y, lane = threadIdx.x;
+  int block = blockIdx.x, part = 0;
+  while (block >= parts.blocks[part]) block -= parts.blocks[part++];
+  const long long t = block * 32LL + lane;
+  switch (part) {
+    case kPartRings: {  // a warp a ring
+      const int i = block / d.T;
+      sphere_ring<Real>(params, d, dirs, o.rings, i, block - i * d.T, b, lane);
+      break;
+    }
+    case kPartTransmittance:
+      if (t < d.nT()) transmittance_node<Real>(params, d, T, t, b);
+      break;
+    case kPartBase:
+      if (t < d.nE()) surface_base_node<Real>(params, d, E0, t, b);
+      break;
+    case kPartRows:
+      if (t < d.rows()) row_info<Real>(params, d, o.rowinfo, o.rowmap, t, b);
+      break;
+    case kPartPoints:
+      if (t < d.n0 * d.n2) point_row<Real>(params, d, o.prow, (int)t, b);
+      break;
+    case kPartHeadings:
+      // v.l of heading a as index_to_sun_direction forms it, for every atmosphere
+      if (b == 0 && t < d.n3) o.hdvs[t] = dsub(dmul(2.0, (double)t / (d.n3 - 1)), 1.0);
+      break;
+    case kPartSurface:
+      surface_row<Real>(params, d, half_dirs, o, t, b);
+      break;
+    case kPartDirections:
+      if (t < (long long)(sizeof(Real) == 8 ? d.n0 : 1) * d.P)
+        sphere_direction<Real>(params, d, dirs, o.dirs4, o.offsets, (int)(t / d.P), (int)(t % d.P), b);
+      break;
+    case kPartMapT:
+      if (t < d.nT()) remap_T<Real>(params, d, o.remapT, t, b);
+      break;
+    case kPartMapE:
+      if (t < d.nE()) remap_E<Real>(params, d, o.remapE, t, b);
+      break;
+  }
+}
+
+// The parts in `which` (bits 1 << kPart...).
+template <class Real>
+void launch_setup_tables(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs, const DirLocal* half_dirs,
+                         const SetupBuffers<Real>& o, Vec4<Real>* T, Vec4<Real>* E0, unsigned which, cudaStream_t st) {
+  const long long items[kSetupParts] = {
+      32LL * d.n0 * d.T, d.nT(), d.nE(), d.rows(), (long long)d.n0 * d.n2, d.n3, surface_row_items(d),
+      (long long)(sizeof(Real) == 8 ? d.n0 : 1) * d.P, d.nT(), d.nE()};
+  SetupParts parts;
+  int blocks = 0;
+  for (int p = 0; p < kSetupParts; p++) {
+    // a build without iterations may ask for no sphere directions (sphere steps below 2): no rings
+    parts.blocks[p] = which >> p & 1u ? (int)((items[p] + 31) / 32) : 0;
+    blocks += parts.blocks[p];
+  }
+  if (blocks > 0)
+    k_setup_tables<Real><<<dim3((unsigned)blocks, d.B), 32, 0, st>>>(params, d, dirs, half_dirs, o, T, E0, parts);
 }
 
 template <class Real>
@@ -523,34 +637,12 @@ void launch_node_maps(const AtmoParams* params, const BuildDims& d, const SetupB
 
 template <class Real>
 void launch_view_rows(const AtmoParams* params, const BuildDims& d, const SetupBuffers<Real>& o, cudaStream_t st) {
-  const int blk = 128;
+  // one warp a block: a small build's samples spread over the SMs' FP64 units
+  const int blk = 32;
   if (d.scan_rays)
     k_view_rows_scan<Real><<<grid1(d.rows(), blk / 32, d.B), blk, 0, st>>>(params, d, o.rowinfo, o.rows);
   else
     k_view_rows<Real><<<grid1(d.rows() * d.S, blk, d.B), blk, 0, st>>>(params, d, o.rowinfo, o.rows);
-}
-
-template <class Real>
-int launch_setup_aux(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs,
-                     const DirLocal* half_dirs, const SetupBuffers<Real>& o, cudaStream_t st) {
-  const int blk = 128;
-  k_remapT<Real><<<grid1(d.nT(), blk, d.B), blk, 0, st>>>(params, d, o.remapT);
-  k_remapE<Real><<<grid1(d.nE(), blk, d.B), blk, 0, st>>>(params, d, o.remapE);
-  // a build without iterations may ask for no sphere directions (sphere
-  // steps below 2) or no half-sphere ones (ray steps below 4): nothing to launch
-  if (d.P > 0)
-    k_sphere_rings<Real><<<dim3(d.n0, d.B), 256, sizeof(int) * (d.T + 1), st>>>(params, d, dirs, o.rings, o.dirs4,
-                                                                                   o.offsets);
-  return 2 + (d.P > 0) + launch_surface_rows<Real>(params, d, half_dirs, o, st);
-}
-
-template <class Real>
-void launch_setup(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs,
-                  const DirLocal* half_dirs, const SetupBuffers<Real>& o, cudaStream_t st) {
-  launch_setup_rows<Real>(params, d, o, st);
-  launch_node_maps<Real>(params, d, o, st);
-  launch_view_rows<Real>(params, d, o, st);
-  launch_setup_aux<Real>(params, d, dirs, half_dirs, o, st);
 }
 
 template <class Real>
@@ -560,45 +652,18 @@ void launch_sphere_dirs(const AtmoParams* params, const BuildDims& d, const DirL
   if (d.P > 0) k_sphere_setup<Real><<<grid1((long long)d.n0 * d.P, blk, d.B), blk, 0, st>>>(params, d, dirs, out);
 }
 
-template <class Real>
-void launch_transmittance(const AtmoParams* params, const BuildDims& d, Vec4<Real>* T, cudaStream_t st) {
-  const int blk = 128;
-  k_transmittance<Real><<<grid1(d.nT(), blk, d.B), blk, 0, st>>>(params, d, T);
-}
-
-template <class Real>
-void launch_surface_base(const AtmoParams* params, const BuildDims& d, Vec4<Real>* E0, cudaStream_t st) {
-  const int blk = 128;
-  k_surface_base<Real><<<grid1(d.nE(), blk, d.B), blk, 0, st>>>(params, d, E0);
-}
-
-template void launch_setup_rows<float>(const AtmoParams*, const BuildDims&, const SetupBuffers<float>&,
-                                       cudaStream_t);
-template void launch_setup_rows<double>(const AtmoParams*, const BuildDims&, const SetupBuffers<double>&,
-                                        cudaStream_t);
-template void launch_node_maps<float>(const AtmoParams*, const BuildDims&, const SetupBuffers<float>&,
-                                      cudaStream_t);
-template void launch_node_maps<double>(const AtmoParams*, const BuildDims&, const SetupBuffers<double>&,
-                                       cudaStream_t);
-template void launch_view_rows<float>(const AtmoParams*, const BuildDims&, const SetupBuffers<float>&,
-                                      cudaStream_t);
-template void launch_view_rows<double>(const AtmoParams*, const BuildDims&, const SetupBuffers<double>&,
-                                       cudaStream_t);
-template int launch_setup_aux<float>(const AtmoParams*, const BuildDims&, const DirLocal*, const DirLocal*,
-                                     const SetupBuffers<float>&, cudaStream_t);
-template int launch_setup_aux<double>(const AtmoParams*, const BuildDims&, const DirLocal*, const DirLocal*,
-                                      const SetupBuffers<double>&, cudaStream_t);
-template void launch_setup<float>(const AtmoParams*, const BuildDims&, const DirLocal*, const DirLocal*,
-                                  const SetupBuffers<float>&, cudaStream_t);
-template void launch_setup<double>(const AtmoParams*, const BuildDims&, const DirLocal*, const DirLocal*,
-                                   const SetupBuffers<double>&, cudaStream_t);
-template void launch_sphere_dirs<float>(const AtmoParams*, const BuildDims&, const DirLocal*, SphereDir<float>*,
-                                        cudaStream_t);
-template void launch_sphere_dirs<double>(const AtmoParams*, const BuildDims&, const DirLocal*, SphereDir<double>*,
+#define SFSIM_INSTANTIATE(Real)                                                                                  \
+  template void launch_setup_tables<Real>(const AtmoParams*, const BuildDims&, const DirLocal*, const DirLocal*, \
+                                          const SetupBuffers<Real>&, Vec4<Real>*, Vec4<Real>*, unsigned,         \
+                                          cudaStream_t);                                                         \
+  template void launch_node_maps<Real>(const AtmoParams*, const BuildDims&, const SetupBuffers<Real>&,           \
+                                       cudaStream_t);                                                            \
+  template void launch_view_rows<Real>(const AtmoParams*, const BuildDims&, const SetupBuffers<Real>&,           \
+                                       cudaStream_t);                                                            \
+  template void launch_sphere_dirs<Real>(const AtmoParams*, const BuildDims&, const DirLocal*, SphereDir<Real>*, \
                                          cudaStream_t);
-template void launch_transmittance<float>(const AtmoParams*, const BuildDims&, Vec4<float>*, cudaStream_t);
-template void launch_transmittance<double>(const AtmoParams*, const BuildDims&, Vec4<double>*, cudaStream_t);
-template void launch_surface_base<float>(const AtmoParams*, const BuildDims&, Vec4<float>*, cudaStream_t);
-template void launch_surface_base<double>(const AtmoParams*, const BuildDims&, Vec4<double>*, cudaStream_t);
+
+SFSIM_INSTANTIATE(float)
+SFSIM_INSTANTIATE(double)
 
 }  // namespace sfsim

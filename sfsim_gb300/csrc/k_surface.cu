@@ -27,81 +27,6 @@
 
 namespace sfsim {
 
-namespace {
-
-// First direction of ring k: the directions follow one another by ring and
-// their polar cosine falls from ring to ring.
-__device__ inline int ring_start(const DirLocal* dirs, const BuildDims& d, int k) {
-  if (k == 0) return 0;
-  if (k >= d.Th) return d.Ph;
-  const double edge = cos(0.5 * M_PI * k / d.Th);  // between rings k - 1 and k
-  int lo = 0, hi = d.Ph;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (dirs[mid].x < edge)
-      hi = mid;
-    else
-      lo = mid + 1;
-  }
-  return lo;
-}
-
-// The world frame of the directions at x = (r, 0, 0), whatever r.
-struct Frame {
-  d3 n, o1, o2;
-  __device__ Frame() : n(mk3(1, 0, 0)), o1(orthogonal(n)), o2(cross3(n, o1)) {}
-  __device__ d3 world(const DirLocal& q) const { return to_world(n, o1, o2, q); }
-};
-
-}  // namespace
-
-// What does not depend on the light's direction, FP64, in this order: nodes,
-// elevation coordinates per (height, ring), and once for all atmospheres the
-// rings and the directions.
-template <class Real>
-__global__ void k_surface_rows(const AtmoParams* params, BuildDims d, const DirLocal* dirs, SetupBuffers<Real> o) {
-  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const int b = blockIdx.y;
-  const AtmoParams& P = params[b];
-  if (t < d.nE()) {
-    const double r = index_to_radius(P, d.nE0, (double)(t / d.nE1));
-    const double ss = index_to_sin_sun_elevation(d.nE1, (double)(t % d.nE1));
-    const d3 x = mk3(r, 0, 0), l = mk3(ss, sqrt(dmax(0.0, 1 - sqr(ss))), 0);
-    SurfRow<Real> row;
-    split_coord<Real>(height_to_index(P, d.n0, mag3(x)), d.n0, &row.u0, &row.s0);
-    split_coord<Real>(sun_elevation_to_index(d.n2, x, l), d.n2, &row.u2, &row.s2);
-    row.lx = (Real)l.x;
-    row.ly = (Real)l.y;
-    o.erow[(long long)b * d.nE() + t] = row;
-    return;
-  }
-  t -= d.nE();
-  if (t < (long long)d.nE0 * d.Th) {
-    const int i = (int)(t / d.Th), k = (int)(t - (long long)i * d.Th);
-    const d3 x = mk3(index_to_radius(P, d.nE0, (double)i), 0, 0);
-    Coord<Real> c;
-    split_coord<Real>(elevation_to_index(P, d.n1, x, Frame().world(dirs[ring_start(dirs, d, k)]), 1), d.n1, &c.u,
-                      &c.s);
-    o.half_rows[(long long)b * d.nE0 * d.Th + t] = c;
-    return;
-  }
-  t -= (long long)d.nE0 * d.Th;
-  if (b > 0) return;
-  if (t <= d.Th) {
-    HalfRing<Real> ring{};
-    ring.w0 = ring_start(dirs, d, (int)t);
-    if (t < d.Th) {
-      const double x0 = Frame().world(dirs[ring.w0]).x;
-      ring.x0 = (Real)x0;
-      ring.weight = (Real)(dirs[ring.w0].w * x0);
-    }
-    o.half_rings[t] = ring;
-    return;
-  }
-  t -= d.Th + 1;
-  if (t < d.Ph) o.half_y[t] = (Real)Frame().world(dirs[t]).y;
-}
-
 // Weights of the lights [k0, k0 + kn), a warp per (light, ring).  A texel's
 // part in the clamped linear interpolation at a direction is 1 less the
 // distance of the direction's coordinate, if that is positive.  The lanes
@@ -213,16 +138,13 @@ static void launch_half_weights(const AtmoParams* params, const BuildDims& d, co
   k_half_weights<Real><<<dim3((unsigned)(kn * d.Th), d.B), 32, 0, st>>>(params, d, o, k0);
 }
 
+// The weights of all lights, where they are kept; the number of kernels launched.
 template <class Real>
-int launch_surface_rows(const AtmoParams* params, const BuildDims& d, const DirLocal* half_dirs,
-                        const SetupBuffers<Real>& o, cudaStream_t st) {
-  const int blk = 64;
-  // a build without iterations may ask for no directions (ray steps below 4)
-  const long long n = d.nE() + (d.Th > 0 ? (long long)d.nE0 * d.Th + d.Th + 1 + d.Ph : 0);
-  k_surface_rows<Real><<<grid1(n, blk, d.B), blk, 0, st>>>(params, d, half_dirs, o);
-  if (d.Th == 0 || d.half_slab < d.nE1) return 1;
+int launch_surface_weights(const AtmoParams* params, const BuildDims& d, const SetupBuffers<Real>& o,
+                           cudaStream_t st) {
+  if (d.Th == 0 || d.half_slab < d.nE1) return 0;
   launch_half_weights(params, d, o, 0, d.nE1, st);
-  return 2;
+  return 1;
 }
 
 // Where the weights of all lights are not kept (half_slab), those of half_slab
@@ -248,8 +170,8 @@ int launch_surface_radiance(const AtmoParams* params, const BuildDims& d, const 
 }
 
 #define SFSIM_INSTANTIATE(Real)                                                                                   \
-  template int launch_surface_rows<Real>(const AtmoParams*, const BuildDims&, const DirLocal*,                    \
-                                         const SetupBuffers<Real>&, cudaStream_t);                                \
+  template int launch_surface_weights<Real>(const AtmoParams*, const BuildDims&, const SetupBuffers<Real>&,       \
+                                            cudaStream_t);                                                        \
   template int launch_surface_radiance<Real>(const AtmoParams*, const BuildDims&, const SetupBuffers<Real>&,      \
                                              const Vec4<Real>*, const Vec4<Real>*, Vec4<Real>*, cudaStream_t);
 

@@ -38,29 +38,38 @@ size_t point_scatter_capacity(const BuildDims& d);
 template <class Real>
 size_t ray_scatter_capacity(const BuildDims& d);
 
-// The set-up tables in parts: the rows (row info and point rows), then the
-// 4-D node maps with each node's light direction (remap4) and the view-row
-// samples, which both read the rows but not each other, and the rest
-// (remapT, remapE, sphere rings, surface radiance's tables).  launch_setup runs them all on one stream.
+// The set-up tables that read no other table, and the transmittance and E0
+// nodes: launch_setup_tables forms the parts whose bits are in `which` in one
+// launch.
+enum SetupPart {
+  kPartRings,          // point scatter's rings
+  kPartTransmittance,  // T (atmosphere_lut.clj:74)
+  kPartBase,           // E0 (atmosphere.clj:131-137)
+  kPartRows,           // row info and row map
+  kPartPoints,         // point rows
+  kPartHeadings,       // hdvs
+  kPartSurface,        // surface radiance's rows and rings
+  kPartDirections,     // point scatter's directions
+  kPartMapT,           // remapT
+  kPartMapE,           // remapE
+  kSetupParts
+};
+// What the view rows and node maps read, and the rest of the set-up.
+constexpr unsigned kSetupRows = 1u << kPartRows | 1u << kPartPoints | 1u << kPartHeadings;
+constexpr unsigned kSetupRest =
+    1u << kPartRings | 1u << kPartSurface | 1u << kPartDirections | 1u << kPartMapT | 1u << kPartMapE;
 template <class Real>
-void launch_setup_rows(const AtmoParams* params, const BuildDims& d, const SetupBuffers<Real>& o, cudaStream_t st);
+void launch_setup_tables(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs, const DirLocal* half_dirs,
+                         const SetupBuffers<Real>& o, Vec4<Real>* T, Vec4<Real>* E0, unsigned which, cudaStream_t st);
+// The 4-D node maps with each node's light direction, and the view-row
+// samples; both read kSetupRows.
 template <class Real>
 void launch_node_maps(const AtmoParams* params, const BuildDims& d, const SetupBuffers<Real>& o, cudaStream_t st);
 template <class Real>
 void launch_view_rows(const AtmoParams* params, const BuildDims& d, const SetupBuffers<Real>& o, cudaStream_t st);
-// Returns the number of kernels it launched.
+// Surface radiance's weights, from kPartSurface; the number of kernels launched.
 template <class Real>
-int launch_setup_aux(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs,
-                     const DirLocal* half_dirs, const SetupBuffers<Real>& o, cudaStream_t st);
-template <class Real>
-void launch_setup(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs,
-                  const DirLocal* half_dirs, const SetupBuffers<Real>& o, cudaStream_t st);
-
-template <class Real>
-void launch_transmittance(const AtmoParams* params, const BuildDims& d, Vec4<Real>* T, cudaStream_t st);
-
-template <class Real>
-void launch_surface_base(const AtmoParams* params, const BuildDims& d, Vec4<Real>* E0, cudaStream_t st);
+int launch_surface_weights(const AtmoParams* params, const BuildDims& d, const SetupBuffers<Real>& o, cudaStream_t st);
 
 // First-order Rayleigh ray scatter and Mie strength (fused).  With `geom`
 // NULL each block forms its cells' light directions from the point rows and
@@ -111,10 +120,6 @@ template <class Real>
 void launch_sphere_dirs(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs, SphereDir<Real>* out,
                         cudaStream_t st);
 
-// Surface radiance's set-up tables; the number of kernels launched.
-template <class Real>
-int launch_surface_rows(const AtmoParams* params, const BuildDims& d, const DirLocal* half_dirs,
-                        const SetupBuffers<Real>& o, cudaStream_t st);
 // dE = surface radiance of dS (same first-iteration convention); the number
 // of kernels launched.
 template <class Real>
