@@ -106,11 +106,28 @@ __device__ __forceinline__ float q_weight(float f, int bits) {
   return floorf(f * s + 0.5f) / s;
 }
 
-__device__ __forceinline__ f3 texel(const float* t, int w, int h, int x, int y) {
-  x = min(max(x, 0), w - 1);
+// Texels x and x + 1 of row y, each clamped to the table (w >= 2): 24
+// contiguous bytes, read in 16-byte words.  The six 4-byte loads it replaces
+// each went through L1 for 32 scattered addresses, which bound the lookups: L1
+// 91 % busy, 10 of its cycles a load, the L2 a fifth.  Measured, 1049353
+// in-scatter lookups of 32x127x32x8 tables 141 -> 100 us, 524309 attenuated
+// rays 156 -> 119.  The tables start at 256-byte boundaries of one allocation,
+// so a table's last word is inside it.
+__device__ __forceinline__ void texel_pair(const float* t, int w, int h, int x, int y, f3& a, f3& b) {
+  const int xa = min(max(x, 0), w - 1), xb = min(max(x + 1, 0), w - 1), x0 = min(xa, w - 2);
   y = min(max(y, 0), h - 1);
-  const float* p = t + 3 * ((long long)y * w + x);
-  return F3(p[0], p[1], p[2]);
+  const long long f = 3 * ((long long)y * w + x0);
+  const int o = (int)(f & 3);
+  const float4* p = reinterpret_cast<const float4*>(t + (f - o));
+  const float4 p0 = p[0], p1 = p[1];
+  const float w8 = o == 3 ? t[f + 5] : 0.0f;  // the word after, where the texels reach it
+  const bool two = o & 2, one = o & 1;
+  const float s0 = two ? p0.z : p0.x, s1 = two ? p0.w : p0.y, s2 = two ? p1.x : p0.z, s3 = two ? p1.y : p0.w,
+              s4 = two ? p1.z : p1.x, s5 = two ? p1.w : p1.y, s6 = two ? w8 : p1.z;
+  const f3 first = F3(one ? s1 : s0, one ? s2 : s1, one ? s3 : s2);
+  const f3 second = F3(one ? s4 : s3, one ? s5 : s4, one ? s6 : s5);
+  a = xa == x0 ? first : second;
+  b = xb == x0 ? first : second;
 }
 
 __device__ __forceinline__ f3 texture_g(const float* t, int w, int h, float u, float v, int bits) {
@@ -118,8 +135,9 @@ __device__ __forceinline__ f3 texture_g(const float* t, int w, int h, float u, f
   const float x0 = floorf(x), y0 = floorf(y);
   const float fx = q_weight(x - x0, bits), fy = q_weight(y - y0, bits);
   const int ix = (int)x0, iy = (int)y0;
-  const f3 a = texel(t, w, h, ix, iy), b = texel(t, w, h, ix + 1, iy);
-  const f3 c = texel(t, w, h, ix, iy + 1), d = texel(t, w, h, ix + 1, iy + 1);
+  f3 a, b, c, d;
+  texel_pair(t, w, h, ix, iy, a, b);
+  texel_pair(t, w, h, ix, iy + 1, c, d);
   const f3 top = fadd(fmul(a, 1 - fx), fmul(b, fx));
   const f3 bot = fadd(fmul(c, 1 - fx), fmul(d, fx));
   return fadd(fmul(top, 1 - fy), fmul(bot, fy));
@@ -232,21 +250,24 @@ __device__ f3 in_scatter_at_g(const GlslEnv& e, f3 l, f3 p, f3 d) {
   return in_scatter_g(e, idx, fdot(d, l));
 }
 
-__global__ void k_query_table(GlslEnv e, int kind, long long n, const float* A, const float* Bv, const float* L,
-                              float* out) {
+// Blocks an SM that the lookups' registers are limited for: 1049353 lookups of
+// in-scatter took 109 / 103 / 100 / 102 us at 4 / 5 / 6 / 8; the attenuation, with
+// twice the lookups at a time, 119 / 119 / 119 / 128.
+constexpr int kLookupBlocks = 6, kAttenuationBlocks = 4;
+template <int KIND>
+__global__ void __launch_bounds__(128, kLookupBlocks)
+    k_query_table(GlslEnv e, long long n, const float* A, const float* Bv, const float* L, float* out) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= n) return;
   const f3 a = F3(A[3 * t], A[3 * t + 1], A[3 * t + 2]);
   const f3 b = F3(Bv[3 * t], Bv[3 * t + 1], Bv[3 * t + 2]);
   const f3 l = L ? F3(L[3 * t], L[3 * t + 1], L[3 * t + 2]) : F3(0, 0, 1);
   f3 r;
-  switch (kind) {
-    case 0: r = transmittance_track_g(e, a, b); break;
-    case 1: r = transmittance_outer_g(e, a, b); break;
-    case 2: r = ray_scatter_track_g(e, l, a, b); break;
-    case 3: r = ray_scatter_outer_g(e, l, a, b); break;
-    default: r = in_scatter_at_g(e, l, a, b); break;
-  }
+  if (KIND == 0) r = transmittance_track_g(e, a, b);
+  if (KIND == 1) r = transmittance_outer_g(e, a, b);
+  if (KIND == 2) r = ray_scatter_track_g(e, l, a, b);
+  if (KIND == 3) r = ray_scatter_outer_g(e, l, a, b);
+  if (KIND == 4) r = in_scatter_at_g(e, l, a, b);
   out[3 * t] = r.x;
   out[3 * t + 1] = r.y;
   out[3 * t + 2] = r.z;
@@ -301,7 +322,7 @@ __device__ float4 attenuation_track_g(const GlslEnv& e, f3 l, f3 origin, f3 dire
 // with the uniform origin, the eye, in D) and transmittance-point.glsl (3,
 // alpha 1); normalize(v) is v times 1 / length(v), as the track lookups
 // divide a vector by a distance.
-__global__ void k_query_attenuation(GlslEnv e, int kind, long long n, const float* L, const float* P,
+__global__ void __launch_bounds__(128, kAttenuationBlocks) k_query_attenuation(GlslEnv e, int kind, long long n, const float* L, const float* P,
                                     const float* D, const float* Sg, const float* In, float amplification,
                                     float* out) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -361,7 +382,12 @@ void launch_query_table(const QueryTables& q, int kind, long long n, const float
                         float* out, int weight_bits, cudaStream_t st) {
   const GlslEnv e = make_env(q, weight_bits);
   const int blk = 128;
-  k_query_table<<<(unsigned)((n + blk - 1) / blk), blk, 0, st>>>(e, kind, n, a, b, l, out);
+  const auto kernel = kind == 0   ? k_query_table<0>
+                      : kind == 1 ? k_query_table<1>
+                      : kind == 2 ? k_query_table<2>
+                      : kind == 3 ? k_query_table<3>
+                                  : k_query_table<4>;
+  kernel<<<(unsigned)((n + blk - 1) / blk), blk, 0, st>>>(e, n, a, b, l, out);
 }
 
 void launch_query_attenuation(const QueryTables& q, int kind, long long n, const float* light, const float* p,
@@ -400,7 +426,7 @@ __device__ __forceinline__ void network_coords(const GlslEnv& e, f3 p, f3 d, f3 
 
 // The surrogate's coordinates of (x, v, l); the table value there (S + M
 // phase) as a by-product when `table` is set.
-__global__ void k_query_coords(GlslEnv e, long long n, const double* X, const double* V, const double* L,
+__global__ void __launch_bounds__(128, kLookupBlocks) k_query_coords(GlslEnv e, long long n, const double* X, const double* V, const double* L,
                                float* coords, float* table) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= n) return;
