@@ -263,9 +263,10 @@ int make_params(const sfsim_atmo_config& c, AtmoParams& P) {
     double* ph = m ? P.d_phM : P.d_phR;
     float* fph = m ? P.f_phM : P.f_phR;
     ph[0] = 3.0 * (1.0 - g * g) / (8.0 * M_PI * (2.0 + g * g));
-    ph[1] = 1.0 + g * g;
-    ph[2] = -2.0 * g;
-    for (int k = 0; k < 3; k++) fph[k] = (float)ph[k];
+    ph[1] = (1.0 - std::fabs(g)) * (1.0 - std::fabs(g));
+    ph[2] = 2.0 * std::fabs(g);
+    ph[3] = g < 0.0 ? 1.0 : -1.0;
+    for (int k = 0; k < 4; k++) fph[k] = (float)ph[k];
   }
   for (int ch = 0; ch < 3; ch++) {
     P.d_srcR[ch] = P.intensity[ch] * P.ray_base[ch];

@@ -44,10 +44,12 @@ struct AtmoParams {
   float f_R, f_Hh2, f_mie_g;
   float f_bright_pi[3];               // brightness / pi
   float f_intensity[3];
-  // Cornette-Shanks phase as k (1 + mu^2) (a + b mu)^-3/2: {k, a, b} with
-  // k = 3 (1 - g^2) / (8 pi (2 + g^2)), a = 1 + g^2, b = -2 g
-  double d_phR[3], d_phM[3];
-  float f_phR[3], f_phM[3];
+  // Cornette-Shanks phase as k (1 + mu^2) (a + b (1 + c mu))^-3/2: {k, a, b, c}
+  // with k = 3 (1 - g^2) / (8 pi (2 + g^2)), a = (1 - |g|)^2, b = 2 |g|, c =
+  // -sign(g); the sum is 1 + g^2 - 2 g mu in terms that do not cancel where it
+  // is least, at the peak
+  double d_phR[4], d_phM[4];
+  float f_phR[4], f_phM[4];
   // intensity * scatter base, the first-order source factors
   double d_srcR[3], d_srcM[3];
   float f_srcR[3], f_srcM[3];

@@ -26,12 +26,13 @@
 // heading and direction gathers 24 bytes of its ring's row (two channels'
 // values and steps in one load, the third's in another) and 24 more of the
 // ground's.  Production tables (32x255x32x8, 336 directions, 5 iterations):
-// 98M wavefronts and 0.55 ms a launch, 2.96 ms for the build's five; with
+// 98M wavefronts and 0.57 ms a launch, 3.09 ms for the build's five, 0.13 of
+// them for the phases' distances |omega -+ v|, |omega -+ l| (PhaseCS::at); with
 // 4-byte loads it was 160M and 3.49 ms.  With a row per direction instead of
 // per ring (gathered to HBM by a kernel of its own), the phases exchanged by
 // shuffles and every heading walked, it was 7.08 ms.  The 16 atmospheres of a
-// sweep (16x128x16x8) went from 11.8 to 5.3 to 4.6 ms, the reference's tables
-// (32x127x32x8, 71 directions) from 0.96 to 0.47 to 0.41 ms.
+// sweep (16x128x16x8) went from 11.8 to 4.8 ms, the reference's tables
+// (32x127x32x8, 71 directions) from 0.96 to 0.43.
 #include <algorithm>
 #include <type_traits>
 
@@ -187,12 +188,15 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
   __syncthreads();
 
   const PhaseCS<Real> phR(Bulk<Real>::phase_ray(P)), phM(Bulk<Real>::phase_mie(P));
+  // Rayleigh's phase as the reference has it, g = 0, is k (1 + mu^2)
+  const bool flat = phR.b == Real(0);
+  const Real flatR = phR(Real(0));
   const Real scale3 = Real(0.5) * Real(d.n3 - 1);
   const Real scaleE = Bulk<Real>::sun_scale_E(d);
   const unsigned kstride = KS * sizeof(Real), estride = ES * sizeof(Real);
   const unsigned ebase = lookup_base<Real>(lay.etab, estride);
   const Real log2e = Real(1.4426950408889634);
-  const Real zA = -log2e * fma(Real(3), pk.gA, Real(0.6));
+  const Real zA = fma(Real(-3) * log2e, pk.gA, Real(-0.6 * 1.4426950408889634 + Bulk<Real>::kExp2Shift));
   const Real lx = (Real)pk.ss;
   // the light reaching x from direction (x0, x1, x2) of a ring, for the two
   // light directions (lx, ly, lz) of a pair: dS along the ring's row and, for
@@ -212,7 +216,10 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     ld_pairs(rb, v, step);
     X.b = fma2(step, dup(s.y), v);
     if (FIRST) {
-      const R2 ph = phM.pair(mu);
+      // |omega -+ l|^2 for the phase of the light
+      const Real dx = fma(phM.s, lx, rc.x0);
+      const R2 dy = fma2(dup(phM.s), ly, x1), dz = fma2(dup(phM.s), lz, x2);
+      const R2 ph = phM.at(mu, fma2(dy, dy, fma2(dz, dz, dup(dx * dx))));
       R2 thirdm;
       ld_pairs(ra + 4, v, step);
       X.a = fma2(fma2(step, dup(s.x), v), dup(ph.x), X.a);
@@ -331,7 +338,7 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     const SphereRing<Real>& rc = sring[r];
     const unsigned rbase = ring_base(r);
     const R2 c0 = dup(rc.x0 * lx);
-    const Real mv0 = sv * rc.x0;
+    const Real mv0 = sv * rc.x0, dv = fma(phM.s, sv, rc.x0), dv2 = dv * dv, cvs = phM.s * cv;
     const int n = rc.n;
     const Real* x = sdirs + 4 * (rc.w0 + slice);
     const Real* e = sedge + 8 * (rc.w0 + slice);
@@ -352,7 +359,10 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
         R2 x1, x2;
         ld_pairs(x, x1, x2);
         const Real mv = fma(cv, x1.x, mv0);
-        const Real fR = phR(mv), fM = phM(mv);
+        Real fR = flatR * fma(mv, mv, Real(1));
+        if (!flat) fR = phR(mv);
+        const Real dy = x1.x + cvs;  // |omega -+ v|^2 for the phase of the view
+        const Real fM = phM.at(mv, fma(dy, dy, fma(x2.x, x2.x, dv2)));
         const R2 w = fma2(mk2(bM[0], bM[1]), dup(fM), mul2(mk2(bR[0], bR[1]), dup(fR)));
         const Real wz = fma(bM[2], fM, bR[2] * fR);
 #pragma unroll

@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(WIDE ? kRayThreadsWide : kRayThreads, WIDE || 
   const int inner = d.n3 - 2, ncol = d.n2 * (d.n3 + 2);
   const Real log2e = Real(1.4426950408889634);
   const Real kfrac = Real(1.0 / 0.97267627755270747);  // 1 / (1 - exp(-3.6))
-  const R2 zc = dup(Real(-0.6) * log2e), last = dup(Real(d.n2 - 1));
+  const R2 zc = dup(Real(-0.6 * 1.4426950408889634 + Bulk<Real>::kExp2Shift)), last = dup(Real(d.n2 - 1));
 
   for (int c0 = 0; c0 < ncol; c0 += nt) {
     // column c0 + tid; the inner headings' columns, then the two
