@@ -1220,6 +1220,7 @@ struct sfsim_atmo_context {
   AtmoParams* params;
   float *T, *E, *S, *M;
   Vec4<float>* jsum;  // point scatter summed over the iterations, NULL without iterations
+  unsigned char* sun; // the build's sun-ray fits, NULL where it integrated them
   void* geom;         // per-node light directions (CellGeom<Real>)
   Surrogate* sur;     // trained surrogate or NULL
 };
@@ -1265,6 +1266,7 @@ int context_build(sfsim_atmo_context* c) {
   CUDA_TRY(cudaStreamSynchronize(st));
   c->dims = d;
   c->params = w.params;
+  c->sun = w.sun;
   c->geom = w.setup.geom;
   c->T = w.oT;
   c->E = w.oE;
@@ -1922,7 +1924,7 @@ int sfsim_atmo_query_direct(const sfsim_atmo_context* ctx, long long n, const do
   if (n < 0) return fail(SFSIM_ATMO_EINVAL, "n must be non-negative");
   if (n == 0) return 0;
   if (!x || !v || !l || !out) return fail(SFSIM_ATMO_ENULL, "a point array is NULL");
-  launch_query_direct(ctx->params, ctx->dims, ctx->jsum, n, x, v, l, out, (cudaStream_t)stream);
+  launch_query_direct(ctx->params, ctx->dims, ctx->jsum, ctx->sun, n, x, v, l, out, (cudaStream_t)stream);
   CUDA_TRY(cudaGetLastError());
   return 0;
 }
@@ -2060,7 +2062,7 @@ int surrogate_pools(sfsim_atmo_context* c, long long n_direct, unsigned long lon
       const long long m = std::min(chunk, n_direct - o);
       launch_random_queries(m, seed * 1000003ull + (unsigned long long)o, c->cfg.radius, c->cfg.height, xvl,
                             xvl + 3 * chunk, xvl + 6 * chunk, st);
-      launch_query_direct(c->params, d, c->jsum, m, xvl, xvl + 3 * chunk, xvl + 6 * chunk, vals, st);
+      launch_query_direct(c->params, d, c->jsum, c->sun, m, xvl, xvl + 3 * chunk, xvl + 6 * chunk, vals, st);
       launch_query_coords(q, m, xvl, xvl + 3 * chunk, xvl + 6 * chunk, crd, tab, st);
       launch_make_pool(m, crd, vals, tab, kLogEps, *direct_pool + kPoolRow * o, st);
     }
@@ -2252,7 +2254,7 @@ int surrogate_query(Surrogate& S, const float* bias0, const sfsim_atmo_context* 
                 cudaStreamSynchronize(st) != cudaSuccess))
       rc = fail(SFSIM_ATMO_ECUDA, "fallback count readback failed");
     if (!rc && h > (unsigned long long)n) rc = fail(SFSIM_ATMO_ECUDA, "fallback count out of range");
-    if (!rc) launch_query_direct(ctx->params, ctx->dims, ctx->jsum, (long long)h, x, v, l, out, st, list);
+    if (!rc) launch_query_direct(ctx->params, ctx->dims, ctx->jsum, ctx->sun, (long long)h, x, v, l, out, st, list);
     if (!rc && cudaGetLastError() != cudaSuccess) rc = fail(SFSIM_ATMO_ECUDA, "fallback launch failed");
     if (!rc && n_fallback) *n_fallback = (long long)h;
     cudaStreamSynchronize(st);

@@ -614,7 +614,42 @@ __device__ __forceinline__ void optical_sums_w(Real A, Real B, Real C, Real w0, 
                                                Real alpha, Real beta, Real kr, Real km, Real& sum_r, Real& sum_m) {
   Real sr = 0, cr = 0, sm = 0, cm = 0;
   Real fn = 0;
-  for (int n = 0; n < steps; n++) {
+  int n = 0;
+  if constexpr (std::is_same<Real, float>::value) {
+    // samples n and n + 1 side by side, each lane with its own compensated
+    // sums: half the instructions
+    const float2 C2 = dup(C), B2 = dup(B), A2 = dup(A), du2 = dup(du), w2 = dup(w0), al2 = dup(alpha), be2 = dup(beta);
+    float2 c2[NP];
+#pragma unroll
+    for (int k = 0; k < NP; k++) c2[k] = dup(c[k]);
+    float2 s_r = dup(0.0f), c_r = s_r, s_m = s_r, c_m = s_r, f2 = make_float2(0.0f, 1.0f);
+    auto add = [](float2& sum, float2& comp, float2 x) {  // kahan_add
+      const float2 y = sub2(x, comp), t = add2(sum, y);
+      comp = sub2(sub2(t, sum), y);
+      sum = t;
+    };
+#pragma unroll 2
+    for (; n + 2 <= steps; n += 2) {
+      const float2 w = fma2(f2, du2, w2);
+      const float2 q = fma2(w, fma2(w, C2, B2), A2);
+      const float2 z = fma2(q, al2, be2);
+      float2 p = c2[NP - 1];
+#pragma unroll
+      for (int k = NP - 2; k >= 0; k--) p = fma2(p, z, c2[k]);
+      const float2 h = mul2(q, p), hr = mul2(h, dup(kr)), hm = mul2(h, dup(km));
+      add(s_r, c_r, make_float2(Bulk<float>::exp2(hr.x), Bulk<float>::exp2(hr.y)));
+      add(s_m, c_m, make_float2(Bulk<float>::exp2(hm.x), Bulk<float>::exp2(hm.y)));
+      f2 = add2(f2, dup(2.0f));
+    }
+    // the second lane's sum onto the first's
+    sr = s_r.x, cr = c_r.x, sm = s_m.x, cm = c_m.x;
+    kahan_add(sr, cr, s_r.y);
+    kahan_add(sr, cr, -c_r.y);
+    kahan_add(sm, cm, s_m.y);
+    kahan_add(sm, cm, -c_m.y);
+    fn = f2.x;
+  }
+  for (; n < steps; n++) {
     Real w = fma(fn, du, w0);
     Real q = fma(w, fma(w, C, B), A);
     Real h = height_from_q<Real, NP>(q, c, alpha, beta);

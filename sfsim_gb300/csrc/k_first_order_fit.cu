@@ -42,12 +42,9 @@
 // blocks per SM at 128 samples a batch within 1%.)
 #include "atmo_device.cuh"
 #include "kernels.h"
+#include "sun_fit.cuh"
 
 namespace sfsim {
-
-constexpr int kFitRows = 8192;   // values of sqrt(q / q_top)
-constexpr int kFitDeg = 5;       // degree of the segments' polynomials
-constexpr int kFitNodes = kFitDeg + 1;
 
 size_t sun_fit_bytes(int segs) { return sizeof(float2) * kFitNodes * (size_t)segs * kFitRows; }
 
@@ -58,18 +55,6 @@ struct FitBasis {
   double inv[kFitNodes][kFitNodes];  // [power][node]
   float node[kFitNodes];             // t + 1/2
 };
-
-// Geometry of a height: q, cq = top^2 - r^2, the range [dmin, dmin + range] of exit distances.
-struct FitRange {
-  float cq, dmin, range;
-};
-__device__ __forceinline__ FitRange fit_range(const AtmoParams& P, float q) {
-  FitRange f;
-  f.cq = fmaxf(P.f_Hh2 - q, 0.0f);
-  f.dmin = f.cq / (P.f_top + sqrtf(fmaf(P.f_R, P.f_R, q)));
-  f.range = sqrtf(q) + P.f_Hh - f.dmin;
-  return f;
-}
 
 // One block: kFitPerBlock heights, one thread per (height, segment, node).
 constexpr int kFitPerBlock = 4;
@@ -171,12 +156,6 @@ struct alignas(16) FitPair {
   int2 row;
   int2 pad;
 };
-
-__device__ __forceinline__ float reciprocal(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
 
 // Samples whose coefficients are in shared memory at a time: 24.6 KB at 8 segments.
 constexpr int kFitBatch = 64 * 8;  // segments x samples

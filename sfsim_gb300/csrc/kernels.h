@@ -172,9 +172,10 @@ void launch_query_attenuation(const QueryTables& q, int kind, long long n, const
 
 // Rendered in-scatter S + M phase(mie, v.l) at (x, v, l) by quadrature with
 // the order-summed point-scatter table Jsum (NULL: first order only).
-// With `indices`, warp w evaluates query indices[w] (n of them).
-void launch_query_direct(const AtmoParams* params, const BuildDims& d, const Vec4<float>* Jsum, long long n,
-                         const double* x, const double* v, const double* l, float* out, cudaStream_t st,
+// With `indices`, warp w evaluates query indices[w] (n of them).  `fits`: the
+// atmosphere's sun-ray fits (launch_sun_fit), NULL to integrate every sun ray.
+void launch_query_direct(const AtmoParams* params, const BuildDims& d, const Vec4<float>* Jsum,
+                         const unsigned char* fits, long long n, const double* x, const double* v, const double* l, float* out, cudaStream_t st,
                          const long long* indices = nullptr);
 
 // The surrogate's kMlpCoords coordinates of (x, v, l), the first four the
