@@ -619,12 +619,18 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
   if (cells) CUDA_TRY(cudaStreamWaitEvent(st, g_side_setup[tm.dev], 0));  // node maps, T, E0 and the rest
   // the transmittance and Mie-strength tables are final here: their outputs
   // (and, for host outputs, their copies) need not wait for the iterations
-  tm.mark_begin(9);
-  launch_output2<Real>(d.B, d.nT0, d.nT1, w.setup.remapT, w.T, oT, st);
-  launch_output4<Real>(d, w.setup, w.M, oM, st);
+  // (on the side stream where the iterations fork and join it again)
+  cudaStream_t so = setup_fork && !inter && !hooks && d.iterations > 0 ? ss : st;
+  if (so == ss) {
+    CUDA_TRY(cudaEventRecord(g_side_fork[tm.dev], st));
+    CUDA_TRY(cudaStreamWaitEvent(ss, g_side_fork[tm.dev], 0));
+  }
+  tm.mark_begin(9, so);
+  launch_output2<Real>(d.B, d.nT0, d.nT1, w.setup.remapT, w.T, oT, so);
+  launch_output4<Real>(d, w.setup, w.M, oM, so);
   launches += 2;
-  tm.mark_end();
-  if (early_done) CUDA_TRY(cudaEventRecord(early_done, st));
+  tm.mark_end(so);
+  if (early_done) CUDA_TRY(cudaEventRecord(early_done, so));
   CUDA_TRY(cudaGetLastError());
   if (inter) {
     if (inter->transmittance_nodes) launch_export<Real>(d.B * d.nT(), w.T, inter->transmittance_nodes, st);

@@ -14,11 +14,11 @@ namespace sfsim {
 // atmosphere_lut.clj:94-101).  These kernels store that coordinate per node.
 // ---------------------------------------------------------------------------
 
-// Per view row (i, j), once: the row's geometry (RowInfo) and its height and
-// elevation coordinates, which every node and ray sample of the row shares.
-template <class Real>
-__device__ void row_info(const AtmoParams* params, const BuildDims& d, RowInfo* info, Remap2<Real>* rowmap,
-                         long long row, int b) {
+// Per view row (i, j), once: the row's geometry (RowInfo), and its height and
+// elevation coordinates, which every node of the row shares (row_map: only the
+// accumulations and the outputs read them, so they are no part of the chain to
+// the first order).
+__device__ void row_info(const AtmoParams* params, const BuildDims& d, RowInfo* info, long long row, int b) {
   const long long nrows = d.rows();
   const AtmoParams& P = params[b];
   const int j = (int)(row % d.n1), i = (int)(row / d.n1);
@@ -51,10 +51,19 @@ __device__ void row_info(const AtmoParams* params, const BuildDims& d, RowInfo* 
   ri.f_Ls = (float)ri.Ls;
   ri.above = above;
   info[b * nrows + row] = ri;
+}
+
+template <class Real>
+__device__ void row_map(const AtmoParams* params, const BuildDims& d, Remap2<Real>* rowmap, long long row, int b) {
+  const AtmoParams& P = params[b];
+  double r, sv, cv;
+  int above;
+  view_geometry(P, d, (int)(row / d.n1), (int)(row % d.n1), &r, &sv, &cv, &above);
+  const d3 x = mk3(r, 0, 0), v = mk3(sv, cv, 0);
   Remap2<Real> m;
   split_coord<Real>(height_to_index(P, d.n0, mag3(x)), d.n0, &m.u[0], &m.s[0]);
   split_coord<Real>(elevation_to_index(P, d.n1, x, v, above), d.n1, &m.u[1], &m.s[1]);
-  rowmap[b * nrows + row] = m;
+  rowmap[b * d.rows() + row] = m;
 }
 
 // The height and elevation coordinates of a node are its row's (k_row_info);
@@ -586,7 +595,10 @@ __global__ void __launch_bounds__(32)
       if (t < d.nE()) surface_base_node<Real>(params, d, E0, t, b);
       break;
     case kPartRows:
-      if (t < d.rows()) row_info<Real>(params, d, o.rowinfo, o.rowmap, t, b);
+      if (t < d.rows()) row_info(params, d, o.rowinfo, t, b);
+      break;
+    case kPartRowMap:
+      if (t < d.rows()) row_map<Real>(params, d, o.rowmap, t, b);
       break;
     case kPartPoints:
       if (t < d.n0 * d.n2) point_row<Real>(params, d, o.prow, (int)t, b);
@@ -617,7 +629,7 @@ void launch_setup_tables(const AtmoParams* params, const BuildDims& d, const Dir
                          const SetupBuffers<Real>& o, Vec4<Real>* T, Vec4<Real>* E0, unsigned which, cudaStream_t st) {
   const long long items[kSetupParts] = {
       32LL * d.n0 * d.T, d.nT(), d.nE(), d.rows(), (long long)d.n0 * d.n2, d.n3, surface_row_items(d),
-      (long long)(sizeof(Real) == 8 ? d.n0 : 1) * d.P, d.nT(), d.nE()};
+      (long long)(sizeof(Real) == 8 ? d.n0 : 1) * d.P, d.nT(), d.nE(), d.rows()};
   SetupParts parts;
   int blocks = 0;
   for (int p = 0; p < kSetupParts; p++) {

@@ -45,19 +45,21 @@ enum SetupPart {
   kPartRings,          // point scatter's rings
   kPartTransmittance,  // T (atmosphere_lut.clj:74)
   kPartBase,           // E0 (atmosphere.clj:131-137)
-  kPartRows,           // row info and row map
+  kPartRows,           // row info
   kPartPoints,         // point rows
   kPartHeadings,       // hdvs
   kPartSurface,        // surface radiance's rows and rings
   kPartDirections,     // point scatter's directions
   kPartMapT,           // remapT
   kPartMapE,           // remapE
+  kPartRowMap,         // row map
   kSetupParts
 };
 // What the view rows and node maps read, and the rest of the set-up.
 constexpr unsigned kSetupRows = 1u << kPartRows | 1u << kPartPoints | 1u << kPartHeadings;
 constexpr unsigned kSetupRest =
-    1u << kPartRings | 1u << kPartSurface | 1u << kPartDirections | 1u << kPartMapT | 1u << kPartMapE;
+    1u << kPartRings | 1u << kPartSurface | 1u << kPartDirections | 1u << kPartMapT | 1u << kPartMapE |
+                                1u << kPartRowMap;
 template <class Real>
 void launch_setup_tables(const AtmoParams* params, const BuildDims& d, const DirLocal* dirs, const DirLocal* half_dirs,
                          const SetupBuffers<Real>& o, Vec4<Real>* T, Vec4<Real>* E0, unsigned which, cudaStream_t st);
