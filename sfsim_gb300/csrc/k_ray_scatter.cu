@@ -26,6 +26,15 @@
 // a texel, st = 4 * odd > n2: a warp of 32 sun elevations of one heading
 // reads 32 different banks, and the builder's stores (for 8 headings, 4 sun
 // elevations x 8 headings a warp) do too.
+//
+// What bounds it: the L1 data pipe, 90 % busy with 261M wavefronts a launch of
+// the production tables (32x255x32x8, 128 samples): of 250 a row and sample 60
+// are the gathers, 58 the constants, 48 the loads of J, 32 the stores.  0.92 ms
+// a launch, 4.60 ms of a build; with a bilinear gather per node (four texels,
+// every heading) 5.70.  The reference's tables (32x127x32x8, 100 samples) 2.20 ->
+// 1.83 ms; 16 atmospheres of 16x128x16x8 7.6 ms either way.  Separate builder
+// and gatherer warps took 6.1 to 7.8 ms, corners prefetched into registers 5.6,
+// two columns and cells a thread 4.6 to 5.2 (231M wavefronts, but fewer warps).
 #include <type_traits>
 
 #include "atmo_device.cuh"
@@ -102,15 +111,10 @@ __device__ __forceinline__ int mask_of(double v) { return (int)__double_as_longl
 
 // WIDE: more columns than kRayThreads; they go in passes (the planes are built
 // again for each) and the threads walk the cells without keeping corners.
-#ifndef RSB
-#define RSB 3
-#endif
-#ifndef RSU
-#define RSU 2
-#endif
-constexpr int kRayUnroll = RSU;
+constexpr int kRayBlocks = 3;  // blocks per SM: 4.60 ms of a production build, two 5.04
+constexpr int kRayUnroll = 2;  // samples whose new corners are on their way together
 template <class Real, bool WIDE>
-__global__ void __launch_bounds__(WIDE ? kRayThreadsWide : kRayThreads, WIDE || sizeof(Real) == 8 ? 1 : RSB)
+__global__ void __launch_bounds__(WIDE ? kRayThreadsWide : kRayThreads, WIDE || sizeof(Real) == 8 ? 1 : kRayBlocks)
     k_ray_scatter(BuildDims d, RayLayout lay, const RowInfo* rowinfo, const RowSample<Real>* rows,
                   const CellGeom<Real>* geom, const Coord<Real>* angle, const Vec4<Real>* J, Vec4<Real>* dS) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
