@@ -39,9 +39,9 @@ UNIT = "ray-scatter cells/s (full multi-order LUT build)"
 # build, mean over its five launches in one ncu capture of this workload
 # (dram__bytes_read.sum + dram__bytes_write.sum); ncu does not run here, so the
 # figure is a recorded capture, not a measurement of this run
-PS_DRAM_BYTES_PER_LAUNCH = 89_500_000
+PS_DRAM_BYTES_PER_LAUNCH = 39_200_000
 TABLES = ("transmittance", "surface_radiance", "ray_scatter", "mie_strength")
-SUN_TABLE_NODES = 2048 * 2048 + 1024 * 2048  # climbing and descending sun-ray tables of the FP32 first order
+SUN_FIT_NODES = 8192 * 8 * 6  # sun rays integrated for the fits: heights x segments x Chebyshev nodes
 WORKLOAD = ("production LUT build: T 255x255, E 16x64, S/M 32x255x32x8 RGB, 5 iterations, "
             "128 ray steps, sphere steps 32 (336 directions), R 6378 km, H 100 km")
 
@@ -259,12 +259,13 @@ def run_ours(args):
     counts = (ctypes.c_ulonglong * 10)()
     _lib.check(L.sfsim_atmo_census(ctypes.byref(cfg), counts, 10), "census")
     lit, climb = counts[0], counts[6]
-    dir_evals, ground_evals, first_evals, flat_evals = counts[3], counts[7], counts[8], counts[9]
-    # per direction: the dS heading-row interpolation, 2 corners x RGB float
-    # (24 B); the first iteration's Mie row another 24 B; a ground direction's
-    # dE gather 48 B (4 corners), or 24 B when its lower height row alone has
-    # weight
-    ps_bytes = 24 * dir_evals + 24 * first_evals + 48 * (ground_evals - flat_evals) + 24 * flat_evals
+    dir_evals, ground_evals, first_evals = counts[3], counts[7], counts[8]
+    # per direction and inner heading: the ring row's RGB value and step to the
+    # next texel (24 B); the first iteration's Mie row another 24 B, a ground
+    # direction's surface radiance another 24 B.  The first and last heading's
+    # sums are formed once per block and read together (24 B a direction).
+    n3 = cfg.ray_scatter_shape[3]
+    ps_bytes = 24 * (dir_evals + first_evals + ground_evals) * (n3 - 2) // n3 + 24 * dir_evals // n3
     smem_peak = ctypes.c_double()
     _lib.check(L.sfsim_atmo_smem_peak(ctypes.byref(smem_peak)), "smem_peak")
     ps_ms = stages["point_scatter"]
@@ -273,19 +274,18 @@ def run_ours(args):
     peak = ctypes.c_double()
     _lib.check(L.sfsim_atmo_sfu_peak(ctypes.byref(peak)), "sfu_peak")
     fo_ms = stages["first_order"]
-    # exponentials of the first-order stage: 3 transmittances per lit
-    # (node, sample) pair, 2 more per descending sun ray (its lookup is the
-    # log of a mean density), and the sun tables' 2048 x 2048 + 1024 x 2048
-    # nodes of S samples (2 each); the FP32 production build reads every sun
-    # ray's optical depths from these tables
-    fo_ex2 = 3 * lit + 2 * (lit - climb) + 2 * SUN_TABLE_NODES * cfg.ray_steps
+    # exponentials of the first-order stage: per lit (node, sample) pair 3
+    # transmittances and 2 mean densities from the fitted sun rays, and the
+    # fits' own integrations (S samples of 2)
+    fo_ex2 = 5 * lit + 2 * SUN_FIT_NODES * cfg.ray_steps
     fo_achieved = fo_ex2 / (fo_ms * 1e-3) / 1e9
     peak_g = peak.value / 1e9
-    # ray scatter: per (node, ray sample) the bilinear gather from the
-    # sample's [sun elevation][heading] plane in shared memory reads 4 RGB
-    # texels (48 B); every iteration gathers at every node and sample
+    # ray scatter: per view row and ray sample a plane of n2 x n3 cells is
+    # written (12 B each) and n2 x (n3 + 2) heading columns gather two of its
+    # texels each (24 B), in every iteration
     rs_ms = stages["ray_scatter"]
-    rs_bytes = 48 * n4 * cfg.ray_steps * cfg.iterations
+    rs_samples = n4 // n3 * cfg.ray_steps * cfg.iterations  # (row, sun elevation, sample)
+    rs_bytes = (12 * n3 + 24 * (n3 + 2)) * rs_samples
     rs_achieved = rs_bytes / (rs_ms * 1e-3) / 1e9
 
     sweep = run_sweep(L, A, C) if args.extras else None
@@ -323,29 +323,31 @@ def run_ours(args):
                          "traffic": PS_DRAM_BYTES_PER_LAUNCH,
                          "traffic_source": "ncu capture of this workload (recorded figure, not measured in this run)",
                          "note": ("achieved = algorithmic shared-memory gather bytes of the point-scatter stage "
-                                  "(24 B per direction evaluation for the dS row, 24 B more in the first "
-                                  "iteration, 48 B per ground direction, 24 B when one dE height row has all the "
-                                  "weight; census counts) / its event time; peak = "
+                                  "(24 B per direction and inner heading for the ring's row, 24 B more in the first "
+                                  "iteration and on the ground, 24 B per direction for the two outer headings; "
+                                  "census counts) / its event time; lanes that share a record are served together, "
+                                  "and the FMA pipe is as busy; peak = "
                                   "conflict-free shared-memory read bandwidth measured live on this GPU by "
                                   "sfsim_atmo_smem_peak (no such figure in MEASURED_PEAKS.json); DRAM is not "
                                   "the bound (the tables live in L2); traffic = DRAM bytes read + written per "
                                   "point-scatter launch, mean of the build's five launches in one ncu capture of "
                                   "this workload"),
                          "direction_evaluations": dir_evals, "kernel_ms": ps_ms},
-            "roofline_first_order": {"bound": "sfu", "kernel": "k_first_order", "achieved": fo_achieved,
+            "roofline_first_order": {"bound": "issue", "kernel": "k_first_order_fit", "achieved": fo_achieved,
                                      "peak": peak_g, "unit": "Gex2/s", "frac": fo_achieved / peak_g if peak_g else None,
-                                     "note": ("exponentials of the stage: 3 transmittances per lit sample, 2 per "
-                                              "descending sun-ray lookup, 2 per sample of the sun tables (2048 x 2048 "
-                                              "climbing + 1024 x 2048 descending nodes); every sun ray's optical "
-                                              "depths are read from the tables, so the stage is bound by the tables' "
-                                              "L1 gathers, not the SFU; peak = ex2.approx throughput measured live"),
+                                     "note": ("exponentials of the stage: 3 transmittances and 2 fitted mean densities "
+                                              "per lit sample, 2 per sample of the fits' own sun rays (8192 heights x 8 "
+                                              "segments x 6 nodes); the stage is bound by instruction issue and "
+                                              "latency, not the SFU; peak = ex2.approx throughput measured live"),
                                      "lit_pairs": lit, "climbing_pairs": climb, "kernel_ms": fo_ms},
             "roofline_ray_scatter": {"bound": "smem", "kernel": "k_ray_scatter", "achieved": rs_achieved,
                                      "peak": smem_peak_g, "unit": "GB/s",
                                      "frac": rs_achieved / smem_peak_g if smem_peak_g else None,
-                                     "note": ("achieved = shared-memory plane gather bytes of the stage (4 RGB "
-                                              "texels, 48 B, per node and ray sample, every iteration) / its event "
-                                              "time; peak = the live conflict-free shared-memory read bandwidth"),
+                                     "note": ("achieved = shared-memory bytes of the stage (planes written, 12 B a "
+                                              "cell, and two RGB texels, 24 B, gathered per heading column) / its "
+                                              "event time; the L1 data pipe also carries the builders' constants and "
+                                              "the J loads; peak = the live conflict-free shared-memory read "
+                                              "bandwidth"),
                                      "node_samples": n4 * cfg.ray_steps * cfg.iterations, "kernel_ms": rs_ms},
             "clocks": clk,
             "err_vs_fp64": {"tables": err_fp64, "against": ("the FP64 production build of the same kernels "
