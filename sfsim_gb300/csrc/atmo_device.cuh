@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "atmo_params.h"
+#include "exp2_table.cuh"
 
 namespace sfsim {
 
@@ -354,7 +355,7 @@ struct Bulk<float> {
 template <>
 struct Bulk<double> {
   static constexpr double kExp2Shift = 0.0;
-  static __device__ __forceinline__ double exp2(double x) { return ::exp2(x); }
+  static __device__ __forceinline__ double exp2(double x) { return exp2_table(x); }
   static __device__ __forceinline__ double sqrt(double x) { return ::sqrt(x); }
   static __device__ __forceinline__ double rsqrt(double x) { return 1.0 / ::sqrt(x); }
   static __device__ __forceinline__ double div(double a, double b) { return a / b; }
