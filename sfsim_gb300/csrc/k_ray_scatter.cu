@@ -28,13 +28,15 @@
 // elevations x 8 headings a warp) do too.
 //
 // What bounds it: the L1 data pipe, 90 % busy with 261M wavefronts a launch of
-// the production tables (32x255x32x8, 128 samples): of 250 a row and sample 60
-// are the gathers, 58 the constants, 48 the loads of J, 32 the stores.  0.92 ms
-// a launch, 4.60 ms of a build; with a bilinear gather per node (four texels,
-// every heading) 5.70.  The reference's tables (32x127x32x8, 100 samples) 2.20 ->
-// 1.83 ms; 16 atmospheres of 16x128x16x8 7.6 ms either way.  Separate builder
-// and gatherer warps took 6.1 to 7.8 ms, corners prefetched into registers 5.6,
-// two columns and cells a thread 4.6 to 5.2 (231M wavefronts, but fewer warps).
+// the production tables (32x255x32x8, 128 samples) before the corners' offsets
+// were read only where they are needed: of 250 a row and sample 60 are the
+// gathers, 58 the constants (10 fewer since), 48 the loads of J, 32 the stores.
+// 0.88 ms a launch, 4.42 ms of a build, 4.60 with the offsets of every sample;
+// with a bilinear gather per node (four texels, every heading) 5.70.  The
+// reference's tables (32x127x32x8, 100 samples) 2.20 -> 1.83 -> 1.75 ms; 16
+// atmospheres of 16x128x16x8 7.6 -> 6.9.  Separate builder and gatherer warps
+// took 6.1 to 7.8 ms, corners prefetched into registers 5.6, two columns and
+// cells a thread 4.6 to 5.2 (231M wavefronts, but fewer warps).
 #include <type_traits>
 
 #include "atmo_device.cuh"
@@ -150,11 +152,13 @@ __global__ void __launch_bounds__(WIDE ? kRayThreadsWide : kRayThreads, WIDE || 
     ld_pairs(k, w01, w23);
     ld_pairs(k + 4, T01, T2m);
     const int mask = WIDE ? 15 : mask_of(T2m.y);
-    const int4 q = cp[u];
-    if (mask & 1) v[0] = Jc[q.x];
-    if (mask & 2) v[1] = Jc[q.y];
-    if (mask & 4) v[2] = Jc[q.z];
-    if (mask & 8) v[3] = Jc[q.w];
+    if (mask) {  // about half of the samples stay in the cell of the one before
+      const int4 q = cp[u];
+      if (mask & 1) v[0] = Jc[q.x];
+      if (mask & 2) v[1] = Jc[q.y];
+      if (mask & 4) v[2] = Jc[q.z];
+      if (mask & 8) v[3] = Jc[q.w];
+    }
     o[0] = fma(w01.x, v[0].x, fma(w01.y, v[1].x, fma(w23.x, v[2].x, w23.y * v[3].x))) * T01.x;
     o[1] = fma(w01.x, v[0].y, fma(w01.y, v[1].y, fma(w23.x, v[2].y, w23.y * v[3].y))) * T01.y;
     o[2] = fma(w01.x, v[0].z, fma(w01.y, v[1].z, fma(w23.x, v[2].z, w23.y * v[3].z))) * T2m.x;
