@@ -62,7 +62,7 @@ struct RayLayout {
   int ch;  // planes per buffer
 };
 template <class Real>
-__host__ inline RayLayout ray_layout(const BuildDims& d, int ch) {
+__host__ inline RayLayout ray_layout(const BuildDims& d, int ch, int groups) {
   auto up = [](size_t x) { return (x + 15) & ~size_t(15); };
   RayLayout l;
   size_t o = 0;
@@ -76,7 +76,7 @@ __host__ inline RayLayout ray_layout(const BuildDims& d, int ch) {
   o = up(o + sizeof(Real) * 12 * d.n2);
   l.planes = (unsigned)o;
   l.plane_bytes = (unsigned)(sizeof(Real) * 3 * ray_column(d.n2) * d.n3);
-  o += 2 * (size_t)ch * l.plane_bytes;
+  o += 2 * (size_t)ch * groups * l.plane_bytes;
   l.bytes = (unsigned)o;
   l.ch = ch;
   return l;
@@ -115,13 +115,17 @@ __device__ __forceinline__ int mask_of(double v) { return (int)__double_as_longl
 // again for each) and the threads walk the cells without keeping corners.
 constexpr int kRayBlocks = 3;  // blocks per SM: 4.60 ms of a production build, two 5.04
 constexpr int kRayUnroll = 2;  // samples whose new corners are on their way together
-template <class Real, bool WIDE>
+// SPLIT: several groups of threads share the ray's samples.
+template <class Real, bool WIDE, bool SPLIT>
 __global__ void __launch_bounds__(WIDE ? kRayThreadsWide : kRayThreads, WIDE || sizeof(Real) == 8 ? 1 : kRayBlocks)
     k_ray_scatter(BuildDims d, RayLayout lay, const RowInfo* rowinfo, const RowSample<Real>* rows,
-                  const CellGeom<Real>* geom, const Coord<Real>* angle, const Vec4<Real>* J, Vec4<Real>* dS) {
+                  const CellGeom<Real>* geom, const Coord<Real>* angle, const Vec4<Real>* J, Vec4<Real>* dS,
+                  int ngroups) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using R2 = V2<Real>;
   const int tid = threadIdx.x, nt = blockDim.x;
+  const int groups = SPLIT ? ngroups : 1;
+  const int per = SPLIT ? nt / groups : nt, group = SPLIT ? tid / per : 0, gt = SPLIT ? tid - group * per : tid;
   const int b = blockIdx.y;
   const long long row = blockIdx.x, nrows = d.rows();
   const int ncell = d.n2 * d.n3, CH = lay.ch;
@@ -135,7 +139,7 @@ __global__ void __launch_bounds__(WIDE ? kRayThreadsWide : kRayThreads, WIDE || 
   const int st = ray_column(d.n2);
   const unsigned plane_bytes = lay.plane_bytes;
   // the texel past the last sun elevation, read with weight 0 at the top
-  for (int t = tid; t < 2 * CH * d.n3; t += nt) {
+  for (int t = tid; t < 2 * CH * groups * d.n3; t += nt) {
     Real* p = reinterpret_cast<Real*>(smem_raw + lay.planes) + 3 * (t * st + d.n2);
     p[0] = p[1] = p[2] = Real(0);
   }
@@ -145,13 +149,14 @@ __global__ void __launch_bounds__(WIDE ? kRayThreadsWide : kRayThreads, WIDE || 
   Vec4<Real> v[4];
 #pragma unroll
   for (int q = 0; q < 4; q++) v[q].x = v[q].y = v[q].z = v[q].w = Real(0);
+  int g0 = 0;  // the group's first sample of the batch
   // the cell in the plane of batch sample u: new corners by the sample's mask, then their mix
   auto form = [&](int u, const Vec4<Real>* Jc, Real* o) {
     const Real* k = cb + 8 * u;
     R2 w01, w23, T01, T2m;
     ld_pairs(k, w01, w23);
     ld_pairs(k + 4, T01, T2m);
-    const int mask = WIDE ? 15 : mask_of(T2m.y);
+    const int mask = WIDE || (SPLIT && u == g0) ? 15 : mask_of(T2m.y);
     if (mask) {  // about half of the samples stay in the cell of the one before
       const int4 q = cp[u];
       if (mask & 1) v[0] = Jc[q.x];
@@ -164,19 +169,19 @@ __global__ void __launch_bounds__(WIDE ? kRayThreadsWide : kRayThreads, WIDE || 
     o[2] = fma(w01.x, v[0].z, fma(w01.y, v[1].z, fma(w23.x, v[2].z, w23.y * v[3].z))) * T2m.x;
   };
   const int pitch = (int)(plane_bytes / sizeof(Real));
-  const int own = 3 * ((tid % d.n3) * st + tid / d.n3);
+  const int own = 3 * ((gt % d.n3) * st + gt / d.n3);
   // planes of batch samples u0 .. u1 - 1
   auto build = [&](int u0, int u1, int buf) {
-    Real* plane = reinterpret_cast<Real*>(smem_raw + lay.planes + (unsigned)(buf * CH) * plane_bytes);
+    Real* plane = reinterpret_cast<Real*>(smem_raw + lay.planes + (unsigned)((2 * group + buf) * CH) * plane_bytes);
     if constexpr (WIDE) {
       for (int cell = tid; cell < ncell; cell += nt) {
         Real* o = plane + 3 * ((cell % d.n3) * st + cell / d.n3);
         for (int u = u0; u < u1; u++, o += pitch) form(u, Jb + cell, o);
       }
-    } else if (tid < ncell) {
+    } else if (gt < ncell) {
       Real* o = plane + own;
 #pragma unroll kRayUnroll
-      for (int u = u0; u < u1; u++, o += pitch) form(u, Jb + tid, o);
+      for (int u = u0; u < u1; u++, o += pitch) form(u, Jb + gt, o);
     }
   };
 
@@ -185,16 +190,16 @@ __global__ void __launch_bounds__(WIDE ? kRayThreadsWide : kRayThreads, WIDE || 
   const Real kfrac = Real(1.0 / 0.97267627755270747);  // 1 / (1 - exp(-3.6))
   const R2 zc = dup(Real(-0.6 * 1.4426950408889634 + Bulk<Real>::kExp2Shift)), last = dup(Real(d.n2 - 1));
 
-  for (int c0 = 0; c0 < ncol; c0 += nt) {
-    // column c0 + tid; the inner headings' columns, then the two
+  for (int c0 = 0; c0 < ncol; c0 += per) {
+    // column c0 + gt; the inner headings' columns, then the two
     // columns of the first and of the last heading, each for every sun elevation
     R2 acc[3] = {dup(Real(0)), dup(Real(0)), dup(Real(0))};  // even and odd samples
     R2 Dl = dup(Real(0)), b0 = dup(Real(0));
     unsigned col = 0;
     int cell = -1, slot = -1;  // the node to store, or the edge sum's slot
     Real wedge = 0;
-    if (c0 + tid < ncol) {
-      const int h = (c0 + tid) / d.n2, k = (c0 + tid) - h * d.n2;
+    if (c0 + gt < ncol) {
+      const int h = (c0 + gt) / d.n2, k = (c0 + gt) - h * d.n2;
       const int e = h - inner;
       const int a = e < 0 ? h + 1 : e < 2 ? 0 : d.n3 - 1;
       const CellGeom<Real> g = geom[node0 + k * d.n3 + a];
@@ -249,12 +254,17 @@ __global__ void __launch_bounds__(WIDE ? kRayThreadsWide : kRayThreads, WIDE || 
         k[7] = mask_value(Real(0), mask);
       }
       __syncthreads();
-      build(0, min(CH, n), 0);
+      // every group's part of the batch, in pairs; all groups meet every barrier
+      const int part = !SPLIT ? n : 2 * ((n / 2 + groups - 1) / groups);
+      g0 = SPLIT ? min(group * part, n) : 0;
+      const int g1 = SPLIT ? min(g0 + part, n) : n;
+      build(g0, min(g0 + CH, g1), 0);
       __syncthreads();
-      for (int u0 = 0, buf = 0; u0 < n; u0 += CH, buf ^= 1) {
-        const int u1 = min(u0 + CH, n);
+      for (int off = 0, buf = 0; off < part; off += CH, buf ^= 1) {
+        const int u0 = g0 + off, u1 = min(u0 + CH, g1);
         {
-          unsigned pa = lookup_base<Real>(lay.planes + (unsigned)(buf * CH) * plane_bytes + col, 3 * sizeof(Real));
+          unsigned pa = lookup_base<Real>(lay.planes + (unsigned)((2 * group + buf) * CH) * plane_bytes + col,
+                                             3 * sizeof(Real));
           const Real* k = cg + 2 * u0;
           auto pair = [&]() {
             R2 us, ir;
@@ -281,8 +291,25 @@ __global__ void __launch_bounds__(WIDE ? kRayThreadsWide : kRayThreads, WIDE || 
             for (int u = u0; u < u1; u += 2) pair();
           }
         }
-        if (u1 < n) build(u1, min(u1 + CH, n), buf ^ 1);
+        if (u1 < g1) build(u1, min(u1 + CH, g1), buf ^ 1);
         __syncthreads();
+      }
+    }
+    if constexpr (SPLIT) {
+      // the groups' sums, in order (the planes are no longer read)
+      Real* sums = reinterpret_cast<Real*>(smem_raw + lay.planes);
+      if (group > 0) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) sums[((group - 1) * 3 + c) * per + gt] = acc[c].x + acc[c].y;
+      }
+      __syncthreads();
+      if (group == 0) {
+        for (int g = 0; g < groups - 1; g++) {
+#pragma unroll
+          for (int c = 0; c < 3; c++) acc[c].x += sums[(g * 3 + c) * per + gt];
+        }
+      } else {
+        cell = slot = -1;
       }
     }
     if (cell >= 0) {
@@ -324,20 +351,31 @@ template <class Real>
 int launch_ray_scatter(const BuildDims& d, const RowInfo* rowinfo, const RowSample<Real>* rows,
                        const CellGeom<Real>* geom, const Coord<Real>* angle, const Vec4<Real>* J, Vec4<Real>* dS,
                        cudaStream_t st) {
-  // the most planes per buffer that let two blocks share an SM, else that fit
-  RayLayout lay = ray_layout<Real>(d, 8);
-  for (int ch = 8; ch >= 2 && lay.bytes > 100 * 1024; ch /= 2) lay = ray_layout<Real>(d, ch);
   const int ncol = d.n2 * (d.n3 + 2);
   const bool wide = ncol > kRayThreads;
-  const int block = wide ? kRayThreadsWide : (ncol + 31) / 32 * 32;
+  // Few columns and few rows leave the SMs with a warp or two each, one after
+  // another along the ray: then up to four groups of a block share its samples.
+  // 128 rows of 48 columns, 64 samples, two iterations, 1 / 2 / 4 groups: FP32 37 /
+  // 28 / 24 us; a build 144 / 137 / 131, in FP64 1650 / 1557 / 1531.
+  int groups = 1;
+  const int per = wide ? kRayThreadsWide : (ncol + 31) / 32 * 32;
+  while (!wide && groups < 4 && 2 * groups * per <= kRayThreads &&
+         d.rows() * d.B * (2 * groups * per / 32) <= 4864)  // 32 warps an SM
+    groups *= 2;
+  const int block = per * groups;
+  // the most planes per buffer that let two blocks share an SM, else that fit
+  RayLayout lay = ray_layout<Real>(d, 8, groups);
+  for (int ch = 8; ch >= 2 && lay.bytes > 100 * 1024; ch /= 2) lay = ray_layout<Real>(d, ch, groups);
   const dim3 grid((unsigned)d.rows(), d.B);
   auto go = [&](auto kernel) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.bytes) != cudaSuccess)
       return -1;
-    kernel<<<grid, block, lay.bytes, st>>>(d, lay, rowinfo, rows, geom, angle, J, dS);
+    kernel<<<grid, block, lay.bytes, st>>>(d, lay, rowinfo, rows, geom, angle, J, dS, groups);
     return 0;
   };
-  return wide ? go(k_ray_scatter<Real, true>) : go(k_ray_scatter<Real, false>);
+  return wide ? go(k_ray_scatter<Real, true, false>)
+         : groups > 1 ? go(k_ray_scatter<Real, false, true>)
+                      : go(k_ray_scatter<Real, false, false>);
 }
 
 template int launch_ray_scatter<float>(const BuildDims&, const RowInfo*, const RowSample<float>*,

@@ -43,3 +43,16 @@ def test_ray_scatter_shapes(shape, steps, precision):
     else:
         bound = 1e-4 * np.maximum(np.abs(want), 1e-6 * np.abs(want).max()) + 8 * 2.0 ** -24 * (shape[2] - 1) * most
     assert (np.abs(got - want) <= bound).all(), float((np.abs(got - want) / bound).max())
+
+
+# fewer columns than a block holds in few rows: the ray's samples are shared by
+# groups of threads (4, 4, 2 and, with too many rows, 1), over parts that are
+# uneven, shorter than a group's planes, empty, and of several batches
+SPLIT = [((2, 5, 3, 3), 4), ((2, 5, 3, 3), 6), ((3, 7, 8, 4), 64), ((3, 7, 8, 4), 301), ((2, 9, 16, 8), 131),
+         ((20, 150, 4, 4), 9)]
+
+
+@pytest.mark.parametrize("shape,steps", SPLIT, ids=[f"{'x'.join(map(str, s))}-S{n}" for s, n in SPLIT])
+@pytest.mark.parametrize("precision", [C.FP64, C.FP32], ids=["fp64", "fp32"])
+def test_samples_shared_by_groups(shape, steps, precision):
+    test_ray_scatter_shapes(shape, steps, precision)
