@@ -620,8 +620,9 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
   // the transmittance and Mie-strength tables are final here: their outputs
   // (and, for host outputs, their copies) need not wait for the iterations
   // (on the side stream where the iterations fork and join it again)
-  cudaStream_t so = setup_fork && !inter && !hooks && d.iterations > 0 ? ss : st;
-  if (so == ss) {
+  const bool aside = setup_fork && !inter && !hooks && d.iterations > 0;
+  cudaStream_t so = aside ? ss : st;
+  if (aside) {
     CUDA_TRY(cudaEventRecord(g_side_fork[tm.dev], st));
     CUDA_TRY(cudaStreamWaitEvent(ss, g_side_fork[tm.dev], 0));
   }
