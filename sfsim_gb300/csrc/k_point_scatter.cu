@@ -460,8 +460,9 @@ int launch_point_scatter(const AtmoParams* params, const BuildDims& d, const Row
   // the warps that an SM holds: then several threads share an item's
   // directions.  16 elevations, 4 headings, 8 heights and sun elevations, two
   // iterations: FP32 46 us with 1 thread an item, 31 with 4, 27 with 8; FP64
-  // 885, 305 and 219.
-  const bool few = (long long)d.n0 * d.n2 * chunks * d.B * (block / 32) < 1824;  // 12 warps an SM
+  // 885, 305 and 219.  What counts is one atmosphere's size: the slices order
+  // the sums, and an atmosphere of a batch has the bits of its own build.
+  const bool few = (long long)d.n0 * d.n2 * chunks * (block / 32) < 1824;  // 12 warps an SM
   int slices = 1;
   while (chunks == 1 && 2 * slices * items <= kPointThreads && slices < kPointSlices && (few || slices * items < 32))
     slices *= 2;

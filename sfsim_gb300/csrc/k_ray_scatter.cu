@@ -356,11 +356,13 @@ int launch_ray_scatter(const BuildDims& d, const RowInfo* rowinfo, const RowSamp
   // Few columns and few rows leave the SMs with a warp or two each, one after
   // another along the ray: then up to four groups of a block share its samples.
   // 128 rows of 48 columns, 64 samples, two iterations, 1 / 2 / 4 groups: FP32 37 /
-  // 28 / 24 us; a build 144 / 137 / 131, in FP64 1650 / 1557 / 1531.
+  // 28 / 24 us; a build 144 / 137 / 131, in FP64 1650 / 1557 / 1531.  The rows
+  // are one atmosphere's: the groups order the sums, and an atmosphere of a
+  // batch has the bits of its own build.
   int groups = 1;
   const int per = wide ? kRayThreadsWide : (ncol + 31) / 32 * 32;
   while (!wide && groups < 4 && 2 * groups * per <= kRayThreads &&
-         d.rows() * d.B * (2 * groups * per / 32) <= 4864)  // 32 warps an SM
+         d.rows() * (2 * groups * per / 32) <= 4864)  // 32 warps an SM
     groups *= 2;
   const int block = per * groups;
   // the most planes per buffer that let two blocks share an SM, else that fit
