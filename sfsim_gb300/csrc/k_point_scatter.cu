@@ -26,13 +26,13 @@
 // heading and direction gathers 24 bytes of its ring's row (two channels'
 // values and steps in one load, the third's in another) and 24 more of the
 // ground's.  Production tables (32x255x32x8, 336 directions, 5 iterations):
-// 98M wavefronts and 0.57 ms a launch, 3.09 ms for the build's five, 0.13 of
-// them for the phases' distances |omega -+ v|, |omega -+ l| (PhaseCS::at); with
-// 4-byte loads it was 160M and 3.49 ms.  With a row per direction instead of
-// per ring (gathered to HBM by a kernel of its own), the phases exchanged by
-// shuffles and every heading walked, it was 7.08 ms.  The 16 atmospheres of a
-// sweep (16x128x16x8) went from 11.8 to 4.8 ms, the reference's tables
-// (32x127x32x8, 71 directions) from 0.96 to 0.43.
+// 98M wavefronts and 0.58 ms a launch, 3.18 ms for the build's five, 0.13 of
+// them for the phases' distances |omega -+ v|, |omega -+ l| (PhaseCS::at), 0.10
+// for the compensation of the sums; with 4-byte loads it was 160M and 3.49 ms.
+// With a row per direction instead of per ring (gathered to HBM by a kernel of
+// its own), the phases exchanged by shuffles and every heading walked, it was
+// 7.08 ms.  The 16 atmospheres of a sweep (16x128x16x8) went from 11.8 to 5.0
+// ms, the reference's tables (32x127x32x8, 71 directions) from 0.96 to 0.44.
 #include <algorithm>
 #include <type_traits>
 
@@ -107,6 +107,11 @@ struct HeadingPair {
 
 constexpr int kPointThreads = 128;
 constexpr int kPointSlices = 8;  // at most
+// Directions summed plainly at most, between steps of the compensated totals:
+// production 3.27 / 3.18 / 3.14 ms (of 3.08 with plain totals) with 8 / 16 / 32;
+// the sums' spread is the same with 8 and 16 (4.9e-8 of a sum of 1172
+// directions; plain totals 7.6e-8, 32 5.6e-8).
+constexpr int kPointRun = 16;
 
 // Blocks per SM the registers are limited for.  Three heading pairs measured
 // 3.11 / 2.96 / 3.04 / 3.25 ms of a production build (5 launches) at 2 / 3 /
@@ -328,12 +333,29 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     ly[h] = mk2(ga.ly, gb.ly);
     lz[h] = mk2(ga.lz, gb.lz);
   }
-  // sums over the directions so far, and over the ring being walked (pair HP: the first and last heading)
-  HeadingPair<Real> tot[HP + 1];
+  // Compensated sums over the directions (pair HP: the first and last
+  // heading): runs of up to kPointRun directions are summed plainly, and each
+  // run starts from what the total lost when it took the last one.
+  HeadingPair<Real> tot[HP + 1], run[HP + 1];
   const HeadingPair<Real> none{dup(Real(0)), dup(Real(0)), dup(Real(0))};
 #pragma unroll
-  for (int h = 0; h <= HP; h++) tot[h] = none;
+  for (int h = 0; h <= HP; h++) tot[h] = run[h] = none;
+  auto flush = [&]() {
+    auto take = [](R2& t, R2& x) {
+      const R2 n = add2(t, x);
+      x = sub2(x, sub2(n, t));
+      t = n;
+    };
+#pragma unroll
+    for (int h = 0; h <= HP; h++) {
+      take(tot[h].a, run[h].a);
+      take(tot[h].b, run[h].b);
+      take(tot[h].z, run[h].z);
+    }
+  };
 
+  const int shift = __ffs(slices) - 1;
+  int pending = 0;  // directions in the run
   for (int r = 0; r < d.T; r++) {
     const SphereRing<Real>& rc = sring[r];
     const unsigned rbase = ring_base(r);
@@ -346,67 +368,77 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     Real bR[3], bM[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) bR[c] = rc.weight * pk.bR[c], bM[c] = rc.weight * pk.bM[c];
-    HeadingPair<Real> sum[HP + 1];
-#pragma unroll
-    for (int h = 0; h <= HP; h++) sum[h] = none;
     auto add = [](HeadingPair<Real>& t, R2 w, Real wz, const HeadingPair<Real>& X) {
       t.a = fma2(w, X.a, t.a);
       t.b = fma2(w, X.b, t.b);
       t.z = fma2(dup(wz), X.z, t.z);
     };
     auto walk = [&](auto ground) {
-      for (int m = slice; m < n; m += slices, x += 4 * slices, e += 8 * slices) {
-        R2 x1, x2;
-        ld_pairs(x, x1, x2);
-        const Real mv = fma(cv, x1.x, mv0);
-        Real fR = flatR * fma(mv, mv, Real(1));
-        if (!flat) fR = phR(mv);
-        const Real dy = x1.x + cvs;  // |omega -+ v|^2 for the phase of the view
-        const Real fM = phM.at(mv, fma(dy, dy, fma(x2.x, x2.x, dv2)));
-        const R2 w = fma2(mk2(bM[0], bM[1]), dup(fM), mul2(mk2(bR[0], bR[1]), dup(fR)));
-        const Real wz = fma(bM[2], fM, bR[2] * fR);
-#pragma unroll
-        for (int h = 0; h < HP; h++) {
-          HeadingPair<Real> X;
-          incoming(ground, rc, rbase, c0, x1, x2, ly[h], lz[h], offset(rc.w0 + m), X);
-          add(sum[h], w, wz, X);
+      for (int m0 = slice; m0 < n; m0 += kPointRun * slices) {
+        const int len = min(kPointRun, (n - m0 + slices - 1 + slice) >> shift);  // the slices' longest
+        if (pending + len > kPointRun) {
+          flush();
+          pending = 0;
         }
-        HeadingPair<Real> X;
-        ld_pairs(e, X.a, X.b);
-        X.z = *reinterpret_cast<const R2*>(e + 4);
-        add(sum[HP], w, wz, X);
+        pending += len;
+        const int m1 = min(n, m0 + kPointRun * slices);
+        for (int m = m0; m < m1; m += slices, x += 4 * slices, e += 8 * slices) {
+          R2 x1, x2;
+          ld_pairs(x, x1, x2);
+          const Real mv = fma(cv, x1.x, mv0);
+          Real fR = flatR * fma(mv, mv, Real(1));
+          if (!flat) fR = phR(mv);
+          const Real dy = x1.x + cvs;  // |omega -+ v|^2 for the phase of the view
+          const Real fM = phM.at(mv, fma(dy, dy, fma(x2.x, x2.x, dv2)));
+          const R2 w = fma2(mk2(bM[0], bM[1]), dup(fM), mul2(mk2(bR[0], bR[1]), dup(fR)));
+          const Real wz = fma(bM[2], fM, bR[2] * fR);
+#pragma unroll
+          for (int h = 0; h < HP; h++) {
+            HeadingPair<Real> X;
+            incoming(ground, rc, rbase, c0, x1, x2, ly[h], lz[h], offset(rc.w0 + m), X);
+            add(run[h], w, wz, X);
+          }
+          HeadingPair<Real> X;
+          ld_pairs(e, X.a, X.b);
+          X.z = *reinterpret_cast<const R2*>(e + 4);
+          add(run[HP], w, wz, X);
+        }
       }
     };
     if (rc.surface)
       walk(std::true_type{});
     else
       walk(std::false_type{});
-#pragma unroll
-    for (int h = 0; h <= HP; h++) {
-      tot[h].a = add2(tot[h].a, sum[h].a);
-      tot[h].b = add2(tot[h].b, sum[h].b);
-      tot[h].z = add2(tot[h].z, sum[h].z);
-    }
   }
+  flush();
   if (slices > 1) {
     // the slices' sums, in order
     HeadingPair<Real>* sums = reinterpret_cast<HeadingPair<Real>*>(smem_raw);
     __syncthreads();
     if (valid && slice > 0) {
 #pragma unroll
-      for (int h = 0; h <= HP; h++) sums[((slice - 1) * (HP + 1) + h) * items + item] = tot[h];
+      for (int h = 0; h <= HP; h++) {
+        HeadingPair<Real>* o = sums + 2 * ((slice - 1) * (HP + 1) + h) * items + item;
+        o[0] = tot[h];
+        o[items] = run[h];
+      }
     }
     __syncthreads();
     if (slice == 0) {
+      auto plus = [](HeadingPair<Real>& x, const HeadingPair<Real>& y) {
+        x.a = add2(x.a, y.a);
+        x.b = add2(x.b, y.b);
+        x.z = add2(x.z, y.z);
+      };
       for (int q = 0; q < (slices - 1); q++) {
+        const HeadingPair<Real>* o = sums + 2 * q * (HP + 1) * items + item;
 #pragma unroll
-        for (int h = 0; h <= HP; h++) {
-          const HeadingPair<Real> o = sums[(q * (HP + 1) + h) * items + item];
-          tot[h].a = add2(tot[h].a, o.a);
-          tot[h].b = add2(tot[h].b, o.b);
-          tot[h].z = add2(tot[h].z, o.z);
-        }
+        for (int h = 0; h <= HP; h++) plus(run[h], o[2 * h * items]);
+        flush();
+#pragma unroll
+        for (int h = 0; h <= HP; h++) plus(run[h], o[(2 * h + 1) * items]);
       }
+      flush();
     }
   }
   if (!valid || slice > 0) return;
@@ -468,7 +500,7 @@ int launch_point_scatter(const AtmoParams* params, const BuildDims& d, const Row
     slices *= 2;
   if (slices > 1) {
     block = (slices * items + 31) / 32 * 32;
-    lay.bytes = std::max<unsigned>(lay.bytes, sizeof(HeadingPair<Real>) * (hp + 1) * items * (slices - 1));
+    lay.bytes = std::max<unsigned>(lay.bytes, sizeof(HeadingPair<Real>) * 2 * (hp + 1) * items * (slices - 1));
   }
   const dim3 grid((unsigned)(d.n0 * d.n2 * chunks), d.B);
   auto go = [&](auto kernel) {
