@@ -742,10 +742,15 @@ __device__ inline void segment_depth_warp(const AtmoParams& P, d3 x, d3 D, int s
     kahan_add(sr, cr, Bulk<Real>::exp2(h * Bulk<Real>::kr(P)));
     kahan_add(sm, cm, Bulk<Real>::exp2(h * Bulk<Real>::km(P)));
   }
+  // the lanes' sums with what they lost
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    sr += __shfl_xor_sync(0xffffffffu, sr, o);
-    sm += __shfl_xor_sync(0xffffffffu, sm, o);
+    const Real r = __shfl_xor_sync(0xffffffffu, sr, o), rc = __shfl_xor_sync(0xffffffffu, cr, o);
+    const Real m = __shfl_xor_sync(0xffffffffu, sm, o), mc = __shfl_xor_sync(0xffffffffu, cm, o);
+    kahan_add(sr, cr, r);
+    kahan_add(sr, cr, -rc);
+    kahan_add(sm, cm, m);
+    kahan_add(sm, cm, -mc);
   }
   const Real a = L > 0.0 ? (Real)(L / steps) : Real(0);
 #pragma unroll
