@@ -177,7 +177,7 @@ size_t first_order_fit_smem(const BuildDims& d) {
   fit_shape(d.n2 * d.n3, &cells, &groups);
   const int batch = fit_batch(d);
   const size_t coef = sizeof(float2) * kFitNodes * (size_t)d.sun_segs * batch;
-  const size_t sums = sizeof(float) * 6 * (size_t)cells * groups;
+  const size_t sums = sizeof(float) * 12 * (size_t)cells * groups;
   return (sizeof(CellGeom<float>) + sizeof(double2)) * (size_t)d.n2 * d.n3 + sizeof(FitPair) * (batch / 2) + (coef > sums ? coef : sums);
 }
 
@@ -231,7 +231,8 @@ __global__ void __launch_bounds__(kFitThreads, 4)
     const int cell = c0 + lane;
     const bool active = group < groups && cell < ncell;
     float b0 = 0, Dl = 0;
-    float2 tot[3] = {make_float2(0, 0), make_float2(0, 0), make_float2(0, 0)};  // (Rayleigh, Mie) per channel
+    // (Rayleigh, Mie) per channel, and what the totals lost
+    float2 tot[3] = {make_float2(0, 0), make_float2(0, 0), make_float2(0, 0)}, lost[3] = {tot[0], tot[0], tot[0]};
     __syncthreads();  // the cells' directions are there; the last pass is done with the sums
     if (active) {
       const CellGeom<float> g = cg[cell];
@@ -279,11 +280,13 @@ __global__ void __launch_bounds__(kFitThreads, 4)
       }
       __syncthreads();
       if (active) {
-        // 8 pairs' sums at a time (x: even, y: odd samples), then the totals
+        // 8 pairs' sums at a time (x: even, y: odd samples), then the totals; the
+        // next sums start from what the totals lost (1 % of the stage; with plain
+        // totals 4096 steps spread a sum by 1.5e-7, so by 0.7e-7, its roundings)
         for (int v0 = group; v0 < n / 2; v0 += 8 * groups) {
           float2 accR[3], accM[3];
 #pragma unroll
-          for (int c = 0; c < 3; c++) accR[c] = accM[c] = make_float2(0, 0);
+          for (int c = 0; c < 3; c++) accR[c] = make_float2(lost[c].x, 0), accM[c] = make_float2(lost[c].y, 0);
           const int v1 = min(v0 + 8 * groups, n / 2);
 #pragma unroll 1
           for (int v = v0; v < v1; v += groups) {
@@ -352,31 +355,39 @@ __global__ void __launch_bounds__(kFitThreads, 4)
             }
           }
 #pragma unroll
-          for (int c = 0; c < 3; c++)
-            tot[c] = add2(tot[c], make_float2(accR[c].x + accR[c].y, accM[c].x + accM[c].y));
+          for (int c = 0; c < 3; c++) {
+            const float2 x = make_float2(accR[c].x + accR[c].y, accM[c].x + accM[c].y), n = add2(tot[c], x);
+            lost[c] = sub2(x, sub2(n, tot[c]));
+            tot[c] = n;
+          }
         }
       }
     }
-    // the groups' sums
-    float* sums = reinterpret_cast<float*>(coef);
+    // the groups' sums, each with what it lost
+    float2* sums = reinterpret_cast<float2*>(coef);
     if (groups > 1) {
       __syncthreads();
       if (group < groups) {
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-          sums[((2 * c) * groups + group) * cells + lane] = tot[c].x;
-          sums[((2 * c + 1) * groups + group) * cells + lane] = tot[c].y;
+          sums[((2 * c) * groups + group) * cells + lane] = tot[c];
+          sums[((2 * c + 1) * groups + group) * cells + lane] = lost[c];
         }
       }
       __syncthreads();
       if (group == 0) {
 #pragma unroll
         for (int c = 0; c < 3; c++)
-          for (int g = 1; g < groups; g++)
-            tot[c] = add2(tot[c], make_float2(sums[((2 * c) * groups + g) * cells + lane],
-                                              sums[((2 * c + 1) * groups + g) * cells + lane]));
+          for (int g = 1; g < groups; g++) {
+            const float2 x = sums[((2 * c) * groups + g) * cells + lane], n = add2(tot[c], x), v = sub2(n, tot[c]);
+            lost[c] = add2(lost[c], add2(add2(sub2(tot[c], sub2(n, v)), sub2(x, v)),
+                                         sums[((2 * c + 1) * groups + g) * cells + lane]));
+            tot[c] = n;
+          }
       }
     }
+#pragma unroll
+    for (int c = 0; c < 3; c++) tot[c] = add2(tot[c], lost[c]);
     if (group == 0 && active) {
       const float w = ri.f_Ls;
       const float phR = w * PhaseCS<float>(P.f_phR)(cg[cell].mu);
