@@ -140,7 +140,7 @@ int sfsim_atmo_build_device(const sfsim_atmo_config* cfg, float* transmittance,
  * corrupt each other; order them on one stream.  FP64 builds equal
  * sfsim_atmo_build_device's bit for bit.  So do FP32 builds,
  * except where the fitted sun rays (3 MB or more, taken by FP32 builds whose
- * ray-scatter cells times ray steps exceed about 3.5e6) no longer fit beside
+ * ray-scatter cells times ray steps exceed about 1.9e7) no longer fit beside
  * the scratch tables: then every sun ray is integrated directly and the two
  * agree within 2e-5 relative.  Stage timings are not recorded. */
 int sfsim_atmo_build_static(const sfsim_atmo_config* cfg, float* transmittance,
@@ -456,7 +456,7 @@ int sfsim_atmo_wait_selftest(int polls);
  * samples, [3] = point-scatter direction evaluations, [4] = ray-scatter
  * J lookups, [5] = surface-radiance direction evaluations, [6] = the pairs
  * of [0] whose sun ray climbs (FP32 builds whose ray-scatter cells times ray
- * steps exceed about 3.5e6 evaluate the optical depths of every pair of [0]
+ * steps exceed about 1.9e7 evaluate the optical depths of every pair of [0]
  * from polynomials fitted to the integrals; smaller builds integrate them), [7] = the point-scatter
  * direction
  * evaluations of [3] that end on the ground, [8] = those of the first

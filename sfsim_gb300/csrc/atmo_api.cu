@@ -379,10 +379,16 @@ struct Work {
 //    smooth fit follows; 3 sqrt(H / h) keeps the ripple below 1e-6.
 //  * The fits cost 6 rays per segment at 8192 heights of each atmosphere and
 //    about 20 us of their own latency, the direct integration one ray for each
-//    lit (node, ray sample) pair, about a third of all pairs.  Measured, whole
-//    builds at 8 segments, fitted / direct: 2.9M pairs 351 / 344 us, 4.9M 400 /
-//    438, 11M 532 / 638, 26M 807 / 1428.
-constexpr double kSunFitPays = 18.0;  // direct rays per segment and height above which the fits are taken
+//    lit (node, ray sample) pair, about a third of all pairs; they break even
+//    at 18 rays per segment and height (8 segments: 3.5M pairs).
+//  * But integrated rays are the more precise: over 12 atmospheres of 3.6 to
+//    18M pairs the first order's error against FP64 is 1.11e-7 (Rayleigh) and
+//    1.24e-7 (Mie) in the 2-norm integrated and 1.15e-7 and 1.28e-7 fitted, at
+//    the darkest thousandth of the nodes 1.9e-6 and 3.3e-6 (Mie).  So the fits
+//    wait until the integrals take longer than two tables of 6.3M sun rays
+//    would, whose error the fits are below (2.0e-7 to 2.6e-7 in a sweep).
+constexpr double kSunFitPays = 18.0;      // direct rays per segment and height above which the fits pay
+constexpr double kSunFitRays = 6291456.0;  // direct rays above which they are taken
 int sun_fit_segments(const sfsim_atmo_config* cfgs, int B, const BuildDims& d) {
   if (cfgs[0].precision != SFSIM_ATMO_FP32) return 0;
   double ratio = 1.0;
@@ -395,7 +401,7 @@ int sun_fit_segments(const sfsim_atmo_config* cfgs, int B, const BuildDims& d) {
   BuildDims f = d;
   f.sun_segs = segs;
   if (first_order_fit_smem(f) > kMaxSmem) return 0;
-  return (double)d.n4() * d.S / 3.0 > kSunFitPays * segs * 8192.0 ? segs : 0;
+  return (double)d.n4() * d.S / 3.0 > std::fmax(kSunFitRays, kSunFitPays * segs * 8192.0) ? segs : 0;
 }
 
 template <class Real>
