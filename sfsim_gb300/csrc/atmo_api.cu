@@ -375,8 +375,16 @@ struct Work {
 //    within 1e-5 of the optical depth at depth 15 and 1e-8 of the
 //    transmittance (numpy model).
 //  * The sums must resolve the density peak themselves: with fewer than about
-//    2.4 sqrt(H / h) steps they ripple with the samples' positions, which no
-//    smooth fit follows; 3 sqrt(H / h) keeps the ripple below 1e-6.
+//    2.4 sqrt(H / h) steps they ripple with the samples' positions; 3 sqrt(H / h)
+//    keeps the ripple below 1e-6.  With fewer, 128 segments follow it while H <=
+//    2000 h: first order against FP64, fitted / by tables of 6.3M rays /
+//    integrated, 64 steps, H = 1250 h, 2-norm (Rayleigh, Mie) 0.9, 1.8 / 2.4, 2.2 / 1.0,
+//    1.8e-7, the darkest thousandth 4.7, 4.3 / 3.6, 8.5 / 3.9, 2.1e-6; at 2500 h a
+//    node is off by 1.3e-4, at 20000 h some are lost.  A production build of two
+//    iterations with 48 and 64 steps takes 3.1 and 3.6 ms so, 4.0 and 4.4 with
+//    tables, 4.3 and 5.1 integrated.  Up to 32 steps integrals are the faster;
+//    thinner layers are integrated too, which costs more than tables did
+//    (100 and 128 steps 10.6 and 12.9 ms, 5.8 and 6.5 with tables).
 //  * The fits cost 6 rays per segment at 8192 heights of each atmosphere and
 //    about 20 us of their own latency, the direct integration one ray for each
 //    lit (node, ray sample) pair, about a third of all pairs; they break even
@@ -394,9 +402,12 @@ int sun_fit_segments(const sfsim_atmo_config* cfgs, int B, const BuildDims& d) {
   double ratio = 1.0;
   for (int b = 0; b < B; b++)
     ratio = std::fmax(ratio, cfgs[b].height / std::fmin(cfgs[b].mie.scatter_scale, cfgs[b].rayleigh.scatter_scale));
-  if (d.S < 3.0 * std::sqrt(ratio)) return 0;
   int segs = 8;
   while (segs < 128 && 2.0 * std::sqrt(ratio) > 2.85 * segs) segs *= 2;
+  if (d.S < 3.0 * std::sqrt(ratio)) {
+    if (d.S <= 32 || ratio > 2000.0) return 0;
+    segs = 128;
+  }
   if (2.0 * std::sqrt(ratio) > 2.85 * segs) return 0;
   BuildDims f = d;
   f.sun_segs = segs;

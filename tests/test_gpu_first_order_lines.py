@@ -5,8 +5,8 @@ node's first order then depends on its own coordinates alone, so the nodes
 that a small and a larger table share are equal bit for bit.  Above it the
 fits are taken (one launch more), within 1e-4 per node and 5e-6 in the 2-norm
 of the FP64 build, over cells in several passes, few cells with their samples
-split over warps, odd step counts, and segment counts that follow the scale
-heights."""
+split over warps, odd step counts, segment counts that follow the scale
+heights, and steps that do not resolve the density peak."""
 import ctypes
 
 import numpy as np
@@ -36,7 +36,9 @@ def test_integrated_below(steps, physics):
 CASES = [((8, 101, 32, 9), 90, {}), ((14, 101, 19, 6), 129, {}), ((25, 250, 8, 4), 100, {}),
          ((14, 100, 31, 7), 64, dict(radius=3000e3, mie_scale=800.0, rayleigh_scale=6000.0)),
          ((8, 101, 32, 8), 100, dict(height=60000.0, mie_scale=200.0)),
-         ((16, 160, 16, 8), 61, dict(height=35000.0))]
+         ((16, 160, 16, 8), 61, dict(height=35000.0)),
+         # steps that do not resolve the density peak (3 sqrt(H / h) = 67 and 52)
+         ((15, 255, 32, 8), 64, dict(mie_scale=200.0)), ((21, 255, 32, 8), 45, dict(height=60000.0, mie_scale=200.0))]
 
 
 @pytest.mark.parametrize("shape,steps,physics", CASES, ids=["x".join(map(str, s)) + f"-S{n}" for s, n, _ in CASES])
