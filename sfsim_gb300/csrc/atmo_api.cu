@@ -355,6 +355,33 @@ struct Carver {
   }
 };
 
+// The atmospheres of a batch by the segments of their fitted sun rays, 0 for
+// integrating every sun ray: each has those of its own build.
+struct FitGroups {
+  struct Group {
+    int segs;
+    int first, count;  // its atmospheres are AtmoParams[first .. first + count).order
+    size_t offset;     // of its fits, in the batch's
+  };
+  int n = 0;
+  Group group[6];  // 0, 8, 16 .. 128
+  size_t bytes = 0;
+  BuildDims dims(const BuildDims& d, int i) const {
+    BuildDims g = d;
+    g.B = group[i].count;
+    g.sun_segs = group[i].segs;
+    return g;
+  }
+  int first(int i) const { return n > 1 ? group[i].first : -1; }
+  bool integrated() const { return n == 0 || group[0].segs == 0; }
+  static FitGroups none(int B) {
+    FitGroups f;
+    f.n = 1;
+    f.group[0] = Group{0, 0, B, 0};
+    return f;
+  }
+};
+
 template <class Real>
 struct Work {
   AtmoParams* params;
@@ -364,7 +391,8 @@ struct Work {
   Vec4<Real>*T, *E0, *dE[2], *Eacc[2];
   Vec4<Real>*S1R, *M, *J, *dS[2], *Sacc[2];
   float *oT, *oE, *oS, *oM;  // device outputs when the caller passes host buffers
-  unsigned char* sun;        // the first order's fitted sun rays (BuildDims::sun_segs > 0), or NULL
+  FitGroups fits;            // set before the tables are carved
+  unsigned char* sun;        // the fitted sun rays of the groups that have them, or NULL
 };
 
 // Segments of the FP32 first order's fitted sun rays, or 0 for integrating
@@ -397,11 +425,10 @@ struct Work {
 //    would, whose error the fits are below (2.0e-7 to 2.6e-7 in a sweep).
 constexpr double kSunFitPays = 18.0;      // direct rays per segment and height above which the fits pay
 constexpr double kSunFitRays = 6291456.0;  // direct rays above which they are taken
-int sun_fit_segments(const sfsim_atmo_config* cfgs, int B, const BuildDims& d) {
-  if (cfgs[0].precision != SFSIM_ATMO_FP32) return 0;
-  double ratio = 1.0;
-  for (int b = 0; b < B; b++)
-    ratio = std::fmax(ratio, cfgs[b].height / std::fmin(cfgs[b].mie.scatter_scale, cfgs[b].rayleigh.scatter_scale));
+int sun_fit_segments(const sfsim_atmo_config& cfg, const BuildDims& d) {
+  if (cfg.precision != SFSIM_ATMO_FP32) return 0;
+  const double ratio =
+      std::fmax(1.0, cfg.height / std::fmin(cfg.mie.scatter_scale, cfg.rayleigh.scatter_scale));
   int segs = 8;
   while (segs < 128 && 2.0 * std::sqrt(ratio) > 2.85 * segs) segs *= 2;
   if (d.S < 3.0 * std::sqrt(ratio)) {
@@ -413,6 +440,23 @@ int sun_fit_segments(const sfsim_atmo_config* cfgs, int B, const BuildDims& d) {
   f.sun_segs = segs;
   if (first_order_fit_smem(f) > kMaxSmem) return 0;
   return (double)d.n4() * d.S / 3.0 > std::fmax(kSunFitRays, kSunFitPays * segs * 8192.0) ? segs : 0;
+}
+
+// The groups of a batch; its parameters take the order.
+FitGroups fit_groups(const sfsim_atmo_config* cfgs, int B, const BuildDims& d, AtmoParams* params) {
+  std::vector<int> segs(B);
+  for (int b = 0; b < B; b++) segs[b] = sun_fit_segments(cfgs[b], d);
+  FitGroups f;
+  int at = 0;
+  for (int s = 0; s <= 128; s = s == 0 ? 8 : 2 * s) {
+    const int first = at;
+    for (int b = 0; b < B; b++)
+      if (segs[b] == s) params[at++].order = b;
+    if (at == first) continue;
+    f.group[f.n++] = FitGroups::Group{s, first, at - first, f.bytes};
+    f.bytes += sun_fit_bytes(s) * (at - first);
+  }
+  return f;
 }
 
 template <class Real>
@@ -460,7 +504,7 @@ size_t carve(Work<Real>& w, char* base, const BuildDims& d, bool outputs) {
   } else {
     w.oT = w.oE = w.oS = w.oM = nullptr;
   }
-  w.sun = d.sun_segs > 0 ? c.take<unsigned char>(B * sun_fit_bytes(d.sun_segs)) : nullptr;
+  w.sun = w.fits.bytes > 0 ? c.take<unsigned char>(w.fits.bytes) : nullptr;
   return c.off + 256;
 }
 
@@ -570,15 +614,21 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
   // in shared memory keep the node maps before the first order.
   cudaStream_t ss = tm.side ? g_side_stream[tm.dev] : nullptr;
   const bool setup_fork = ss != nullptr && !g_timing;
-  const bool cells = setup_fork && (w.sun || first_order_smem<Real>(d, true) <= kMaxSmem);
+  const bool cells = setup_fork && (!w.fits.integrated() || first_order_smem<Real>(d, true) <= kMaxSmem);
   cudaStream_t sa = setup_fork ? ss : st;
+  auto sun_fits = [&](cudaStream_t on) {
+    for (int i = 0; i < w.fits.n; i++) {
+      if (w.fits.group[i].segs == 0) continue;
+      launch_sun_fit(w.params, w.fits.dims(d, i), w.sun + w.fits.group[i].offset, on, w.fits.first(i));
+      launches++;
+    }
+  };
   if (setup_fork) {
     CUDA_TRY(cudaEventRecord(g_side_fork[tm.dev], st));
     CUDA_TRY(cudaStreamWaitEvent(ss, g_side_fork[tm.dev], 0));
     if (w.sun) {
       tm.mark_begin(3, ss);
-      launch_sun_fit(w.params, d, w.sun, ss);
-      launches++;
+      sun_fits(ss);
       tm.mark_end(ss);
     }
     CUDA_TRY(cudaEventRecord(g_side_sun[tm.dev], ss));
@@ -616,22 +666,24 @@ int run_build(const Work<Real>& w, const BuildDims& d, float* oT, float* oE, flo
     CUDA_TRY(cudaStreamWaitEvent(st, (cells ? g_side_sun : g_side_setup)[tm.dev], 0));
   }
   tm.mark_begin(3);
-  if (w.sun && !setup_fork) {
-    launch_sun_fit(w.params, d, w.sun, st);
+  if (w.sun && !setup_fork) sun_fits(st);
+  int failed = 0;
+  for (int i = 0; i < w.fits.n; i++) {
+    const BuildDims g = w.fits.dims(d, i);
+    if constexpr (sizeof(Real) == sizeof(float)) {
+      if (g.sun_segs > 0) {
+        failed |= launch_first_order_fit(w.params, g, w.setup.rowinfo, w.setup.rows, w.setup.prow, w.setup.hdvs,
+                                         w.sun + w.fits.group[i].offset, w.S1R, w.M, st, w.fits.first(i));
+        launches++;
+        continue;
+      }
+    }
+    failed |= launch_first_order<Real>(w.params, g, w.setup.rowinfo, w.setup.rows, cells ? nullptr : w.setup.geom,
+                                       w.setup.prow, w.setup.hdvs, w.S1R, w.M, st, w.fits.first(i));
     launches++;
   }
-  int first = 0;
-  if constexpr (sizeof(Real) == sizeof(float)) {
-    if (w.sun)
-      first = launch_first_order_fit(w.params, d, w.setup.rowinfo, w.setup.rows, w.setup.prow, w.setup.hdvs, w.sun,
-                                     w.S1R, w.M, st);
-  }
-  if (!w.sun)
-    first = launch_first_order<Real>(w.params, d, w.setup.rowinfo, w.setup.rows, cells ? nullptr : w.setup.geom,
-                                     w.setup.prow, w.setup.hdvs, w.S1R, w.M, st);
-  if (first)
+  if (failed)
     return fail(SFSIM_ATMO_ECUDA, "first order launch configuration failed");
-  launches++;
   tm.mark_end();
   if (cells) CUDA_TRY(cudaStreamWaitEvent(st, g_side_setup[tm.dev], 0));  // node maps, T, E0 and the rest
   // the transmittance and Mie-strength tables are final here: their outputs
@@ -833,8 +885,8 @@ int build_impl(const sfsim_atmo_config* cfgs, int B, float* T, float* E, float* 
   sphere_directions(cfgs[0].sphere_steps >> 1, cfgs[0].sphere_steps, M_PI, dirs);
   sphere_directions(cfgs[0].ray_steps >> 2, cfgs[0].ray_steps, M_PI / 2, hdirs);
 
-  d.sun_segs = sun_fit_segments(cfgs, B, d);
   Work<Real> w;
+  w.fits = fit_groups(cfgs, B, d, hp.data());
   size_t bytes = carve<Real>(w, nullptr, d, host_out);
   if ((rc = ensure_arena(dev, bytes))) return rc;
   carve<Real>(w, (char*)g_arena[dev].base, d, host_out);
@@ -1262,8 +1314,9 @@ int context_build(sfsim_atmo_context* c) {
   std::vector<DirLocal> dirs, hdirs;
   sphere_directions(cfg.sphere_steps >> 1, cfg.sphere_steps, M_PI, dirs);
   sphere_directions(cfg.ray_steps >> 2, cfg.ray_steps, M_PI / 2, hdirs);
-  d.sun_segs = sun_fit_segments(&cfg, 1, d);
   Work<Real> w;
+  w.fits = fit_groups(&cfg, 1, d, &hp);
+  d.sun_segs = w.fits.group[0].segs;  // for the direct queries
   const size_t wbytes = carve<Real>(w, nullptr, d, true);
   const size_t total = wbytes + sizeof(Vec4<float>) * (size_t)d.n4() + 256;
   cudaError_t e = cudaMalloc(&c->mem, total);
@@ -1694,8 +1747,8 @@ int build_static_impl(const sfsim_atmo_config& cfg, float* T, float* E, float* S
   void* base = nullptr;
   if ((rc = static_scratch_base(dev, &base))) return rc;
   // the fitted sun rays where they fit as well, else every sun ray is integrated
-  d.sun_segs = sun_fit_segments(&cfg, 1, d);
-  if (carve<Real>(w, nullptr, d, false) > kStaticScratchBytes) d.sun_segs = 0;
+  w.fits = fit_groups(&cfg, 1, d, &hp);
+  if (carve<Real>(w, nullptr, d, false) > kStaticScratchBytes) w.fits = FitGroups::none(1);
   // and the surface-radiance weights of as many lights at a time as fit: the
   // count above has more room than one light's (directions per height, four
   // coordinates per node)
@@ -1751,7 +1804,7 @@ int plan_prepare(sfsim_atmo_plan* p, Work<Real>& w) {
   std::vector<DirLocal> dirs, hdirs;
   sphere_directions(cfg.sphere_steps >> 1, cfg.sphere_steps, M_PI, dirs);
   sphere_directions(cfg.ray_steps >> 2, cfg.ray_steps, M_PI / 2, hdirs);
-  d.sun_segs = sun_fit_segments(&cfg, 1, d);
+  w.fits = fit_groups(&cfg, 1, d, &hp);
   const size_t bytes = carve<Real>(w, nullptr, d, false);
   cudaError_t e = cudaMalloc(&p->mem, bytes);
   if (e != cudaSuccess) {

@@ -469,6 +469,12 @@ __device__ __forceinline__ void ld_pairs(const double* p, double2& a, double2& b
   b = reinterpret_cast<const double2*>(p)[1];
 }
 
+// The atmosphere of grid row y: of all of a batch, or of those from `first` in
+// their order by sun rays.
+__device__ __forceinline__ int atmosphere_of(const AtmoParams* params, int first, int y) {
+  return first < 0 ? y : params[first + y].order;
+}
+
 template <class Real>
 __device__ __forceinline__ V2<Real> dup(Real a) {
   return mk2(a, a);

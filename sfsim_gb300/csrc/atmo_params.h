@@ -55,6 +55,7 @@ struct AtmoParams {
   float f_srcR[3], f_srcM[3];
   float f_top, f_Hh;
   int hpoly_n;                        // number of coefficients
+  int order;                          // of a batch: the atmosphere at this place when they go by their sun rays
 };
 
 // Shapes, steps and sizes shared by every atmosphere of one batched build.

@@ -75,10 +75,10 @@ __global__ void __launch_bounds__(WARPS * 32, sizeof(Real) == 8 ? 2 : 4) k_first
                                                             const RowInfo* rowinfo, const RowSample<Real>* rows,
                                                             const CellGeom<Real>* geom, const PointRow<Real>* prow,
                                                             const double* hdvs, Vec4<Real>* rayleigh, Vec4<Real>* mie,
-                                                            int part) {
+                                                            int first, int part) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FirstOrderSmem<Real>* sm = reinterpret_cast<FirstOrderSmem<Real>*>(smem_raw);
-  const int b = blockIdx.y;
+  const int b = atmosphere_of(params, first, blockIdx.y);
   const long long row = blockIdx.x;
   const long long nrows = d.rows();
   const AtmoParams& P = params[b];
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(WARPS * 32, sizeof(Real) == 8 ? 2 : 4) k_first
 template <class Real>
 int launch_first_order(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
                        const RowSample<Real>* rows, const CellGeom<Real>* geom, const PointRow<Real>* prow,
-                       const double* hdvs, Vec4<Real>* rayleigh, Vec4<Real>* mie, cudaStream_t st) {
+                       const double* hdvs, Vec4<Real>* rayleigh, Vec4<Real>* mie, cudaStream_t st, int first) {
   constexpr int WARPS = 8;
   const bool cells = geom == nullptr;
   const size_t smem = first_order_smem<Real>(d, cells);
@@ -203,16 +203,16 @@ int launch_first_order(const AtmoParams* params, const BuildDims& d, const RowIn
   while ((long long)parts * d.rows() * d.B < 1216 && ncell > parts * WARPS) parts *= 2;
   const int part = ((ncell + parts - 1) / parts + WARPS - 1) / WARPS * WARPS;
   dim3 grid((unsigned)d.rows(), d.B, (ncell + part - 1) / part);
-  kernel<<<grid, WARPS * 32, smem, st>>>(params, d, rowinfo, rows, geom, prow, hdvs, rayleigh, mie, part);
+  kernel<<<grid, WARPS * 32, smem, st>>>(params, d, rowinfo, rows, geom, prow, hdvs, rayleigh, mie, first, part);
   return 0;
 }
 
 template int launch_first_order<float>(const AtmoParams*, const BuildDims&, const RowInfo*, const RowSample<float>*,
                                        const CellGeom<float>*, const PointRow<float>*, const double*, Vec4<float>*,
-                                       Vec4<float>*, cudaStream_t);
+                                       Vec4<float>*, cudaStream_t, int);
 template int launch_first_order<double>(const AtmoParams*, const BuildDims&, const RowInfo*,
                                         const RowSample<double>*, const CellGeom<double>*, const PointRow<double>*,
-                                        const double*, Vec4<double>*, Vec4<double>*, cudaStream_t);
+                                        const double*, Vec4<double>*, Vec4<double>*, cudaStream_t, int);
 
 // Work census of the first order: count[0] = the (node, sample) pairs whose
 // sun is above the horizon (sun-ray optical depths the reference integrates,

@@ -58,10 +58,10 @@ struct FitBasis {
 
 // One block: kFitPerBlock heights, one thread per (height, segment, node).
 constexpr int kFitPerBlock = 4;
-__global__ void k_sun_fit(const AtmoParams* params, int S, int segs, FitBasis basis, float2* out) {
+__global__ void k_sun_fit(const AtmoParams* params, int first, int S, int segs, FitBasis basis, float2* out) {
   extern __shared__ float2 F[];  // [height][segment][node]
   const int b = blockIdx.y;
-  const AtmoParams& P = params[b];
+  const AtmoParams& P = params[atmosphere_of(params, first, b)];
   const int per = segs * kFitNodes;
   for (int t = threadIdx.x; t < kFitPerBlock * per; t += blockDim.x) {
     const int h = t / per, e = t - h * per, g = e / kFitNodes, n = e - g * kFitNodes;
@@ -134,12 +134,12 @@ static FitBasis fit_basis() {
   return f;
 }
 
-void launch_sun_fit(const AtmoParams* params, const BuildDims& d, unsigned char* table, cudaStream_t st) {
+void launch_sun_fit(const AtmoParams* params, const BuildDims& d, unsigned char* table, cudaStream_t st, int first) {
   static const FitBasis basis = fit_basis();
   const int per = kFitPerBlock * d.sun_segs * kFitNodes;
   const int block = per < 512 ? (per + 31) / 32 * 32 : 512;
-  k_sun_fit<<<dim3(kFitRows / kFitPerBlock, d.B), block, sizeof(float2) * per, st>>>(params, d.S, d.sun_segs, basis,
-                                                                                    reinterpret_cast<float2*>(table));
+  k_sun_fit<<<dim3(kFitRows / kFitPerBlock, d.B), block, sizeof(float2) * per, st>>>(params, first, d.S, d.sun_segs,
+                                                                                    basis, reinterpret_cast<float2*>(table));
 }
 
 // What the cells share of two consecutive ray samples, side by side.  The sun
@@ -182,11 +182,11 @@ size_t first_order_fit_smem(const BuildDims& d) {
 }
 
 __global__ void __launch_bounds__(kFitThreads, 4)
-    k_first_order_fit(const AtmoParams* params, BuildDims d, int cells, int groups, int batch, const RowInfo* rowinfo,
+    k_first_order_fit(const AtmoParams* params, BuildDims d, int first, int cells, int groups, int batch, const RowInfo* rowinfo,
                       const RowSample<float>* rows, const PointRow<float>* prow, const double* hdvs,
                       const float4* table, Vec4<float>* rayleigh, Vec4<float>* mie) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int b = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
+  const int b = atmosphere_of(params, first, blockIdx.y), tid = threadIdx.x, nt = blockDim.x;
   const long long row = blockIdx.x, nrows = d.rows();
   const AtmoParams& P = params[b];
   const int ncell = d.n2 * d.n3;
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kFitThreads, 4)
   const int words = segs * (kFitNodes / 2);                               // of one sample's coefficients
   const unsigned coef0 = (unsigned)(reinterpret_cast<unsigned char*>(coef) - smem_raw);
   const float2 Hh2 = make_float2(P.f_Hh, P.f_Hh);
-  const float4* tab = table + (size_t)b * kFitRows * words;
+  const float4* tab = table + (size_t)blockIdx.y * kFitRows * words;
   const long long node0 = (b * nrows + row) * ncell;
   const int group = tid / cells, lane = tid - group * cells;
 
@@ -408,14 +408,14 @@ __global__ void __launch_bounds__(kFitThreads, 4)
 
 int launch_first_order_fit(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
                            const RowSample<float>* rows, const PointRow<float>* prow, const double* hdvs,
-                           const unsigned char* table, Vec4<float>* rayleigh, Vec4<float>* mie, cudaStream_t st) {
+                           const unsigned char* table, Vec4<float>* rayleigh, Vec4<float>* mie, cudaStream_t st, int first) {
   int cells, groups;
   fit_shape(d.n2 * d.n3, &cells, &groups);
   const size_t smem = first_order_fit_smem(d);
   if (cudaFuncSetAttribute(k_first_order_fit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return -1;
   k_first_order_fit<<<dim3((unsigned)d.rows(), d.B), cells * groups, smem, st>>>(
-      params, d, cells, groups, fit_batch(d), rowinfo, rows, prow, hdvs,
+      params, d, first, cells, groups, fit_batch(d), rowinfo, rows, prow, hdvs,
       reinterpret_cast<const float4*>(table), rayleigh, mie);
   return 0;
 }

@@ -76,7 +76,8 @@ int launch_surface_weights(const AtmoParams* params, const BuildDims& d, const S
 // First-order Rayleigh ray scatter and Mie strength (fused).  With `geom`
 // NULL each block forms its cells' light directions from the point rows and
 // the per-heading table (as k_remap4 does), so the launch needs the rows and
-// the view-row samples but not the node maps.  -1 when its shared memory
+// the view-row samples but not the node maps.  With `first` >= 0 it makes the
+// d.B atmospheres params[first ..].order of a batch, else the first d.B.  -1 when its shared memory
 // (first_order_smem: the row's samples, and the cells' geometry when
 // `cells`) cannot be configured.
 template <class Real>
@@ -84,19 +85,22 @@ size_t first_order_smem(const BuildDims& d, bool cells);
 template <class Real>
 int launch_first_order(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
                        const RowSample<Real>* rows, const CellGeom<Real>* geom, const PointRow<Real>* prow,
-                       const double* hdvs, Vec4<Real>* rayleigh, Vec4<Real>* mie, cudaStream_t st);
+                       const double* hdvs, Vec4<Real>* rayleigh, Vec4<Real>* mie, cudaStream_t st, int first = -1);
 
 // The FP32 first order with fitted sun rays (k_first_order_fit.cu): bytes of
 // the fits of one atmosphere with `segs` segments, the fits, and the first
 // order that reads them (its blocks form their cells' light directions
 // themselves).  BuildDims::sun_segs says how many segments, 0 for the direct
-// integration of launch_first_order.
+// integration of launch_first_order; `first` says which atmospheres, as there,
+// and the fits in `table` are theirs in that order.
 size_t sun_fit_bytes(int segs);
-void launch_sun_fit(const AtmoParams* params, const BuildDims& d, unsigned char* table, cudaStream_t st);
+void launch_sun_fit(const AtmoParams* params, const BuildDims& d, unsigned char* table, cudaStream_t st,
+                    int first = -1);
 size_t first_order_fit_smem(const BuildDims& d);
 int launch_first_order_fit(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,
                            const RowSample<float>* rows, const PointRow<float>* prow, const double* hdvs,
-                           const unsigned char* table, Vec4<float>* rayleigh, Vec4<float>* mie, cudaStream_t st);
+                           const unsigned char* table, Vec4<float>* rayleigh, Vec4<float>* mie, cudaStream_t st,
+                           int first = -1);
 
 template <class Real>
 void launch_first_order_census(const AtmoParams* params, const BuildDims& d, const RowInfo* rowinfo,

@@ -24,3 +24,20 @@ def test_batch_sizes(shape, precision):
         for n in range(size):
             for key, value in singles[n].items():
                 assert np.array_equal(batch[key][n], value), (size, n, key)
+
+
+def test_unlike_atmospheres():
+    """Atmospheres whose own builds take 8 or 16 segments of fitted sun rays, or
+    integrate every sun ray, keep that in a batch, in whatever order."""
+    def mk(height, mie_scale, base):
+        return C.make_config(radius=base.radius, height=height, mie=C.component((2e-5,) * 3, mie_scale, 0.9, 0.76),
+                             rayleigh=base.rayleigh, transmittance_shape=(4, 8), surface_radiance_shape=(3, 5),
+                             ray_scatter_shape=(8, 101, 32, 8), ray_steps=100, sphere_steps=6, iterations=1)
+    sweep = C.parameter_sweep(7)
+    kinds = [(100000.0, 1200.0), (60000.0, 20.0), (60000.0, 200.0), (60000.0, 20.0), (35000.0, 1200.0),
+             (60000.0, 250.0), (100000.0, 900.0)]
+    cfgs = [mk(h, m, b) for (h, m), b in zip(kinds, sweep)]
+    batch = A.build_batch(cfgs)
+    for n, cfg in enumerate(cfgs):
+        for key, value in A.build(cfg).items():
+            assert np.array_equal(batch[key][n], value), (n, key)
