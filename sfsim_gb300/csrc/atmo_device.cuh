@@ -286,6 +286,17 @@ __host__ __device__ inline d3 to_world(d3 n, d3 o1, d3 o2, const DirLocal& q) {
              dadd(dadd(dmul(n.z, q.x), dmul(o1.z, q.y)), dmul(o2.z, q.z)));
 }
 
+// Whether the radii's squares are ordinary numbers.  With radii above 1e150 or
+// below 1e-140 the geometry is NaN or noise, and so are the tables; but point
+// scatter forms offsets into shared memory from the directions and from the
+// ground points' sun elevation, which are then kept within theirs.
+__host__ __device__ inline bool ordinary_radii(const AtmoParams& P) { return P.R2 > 1e-280 && P.top2 < 1e300; }
+
+// The unit normal at x = (r, 0, 0), as the reference forms it.
+__host__ __device__ inline d3 axis_normal(const AtmoParams& P, d3 x) {
+  return ordinary_radii(P) ? mul3(x, 1.0 / mag3(x)) : mk3(1, 0, 0);
+}
+
 // Geometry of a 4-D node (ray-scatter-backward, atmosphere.clj:401-412).
 struct NodeGeom {
   double r;

@@ -243,7 +243,8 @@ __global__ void __launch_bounds__(kPointThreads, point_min_blocks<Real, HP>())
     if (decltype(ground)::value) {
       // the ground point's sin of the sun elevation, g.l / |g| = gA + tR (omega . l)
       // and its coordinate (1 - exp(-3 sin - 0.6)) / (1 - exp(-3.6)) (nE1 - 1),
-      // at least 0; the sine is at most 1 (k_sphere_rings keeps tR finite)
+      // at least 0; the sine is at most 1, as the point is on the ground
+      // (sphere_ring and point_row see to it where the radii are no ordinary numbers)
       const R2 z = fma2(dup(Real(-3) * log2e * rc.tR), mu, dup(zA));
       const R2 ex = mk2(Bulk<Real>::exp2(z.x), Bulk<Real>::exp2(z.y));
       R2 ie = fma2(dup(-scaleE), ex, dup(scaleE));

@@ -381,7 +381,7 @@ __device__ void sphere_ring(const AtmoParams* params, const BuildDims& d, const 
   const AtmoParams& P = params[b];
   const double r = index_to_radius(P, d.n0, (double)i);
   const d3 x = mk3(r, 0, 0);
-  const d3 n = mul3(x, 1.0 / mag3(x));
+  const d3 n = axis_normal(P, x);
   const d3 o1 = orthogonal(n);
   const d3 o2 = cross3(n, o1);
   const int w = ring_start(dirs, d.P, d.T, M_PI, k);
@@ -401,7 +401,7 @@ __device__ void sphere_ring(const AtmoParams* params, const BuildDims& d, const 
     segment_depth_warp<Real>(P, x, sub3(g, x), d.S, lane, tau);
     for (int c = 0; c < 3; c++) o.ground[c] = exp_neg(tau[c]) * (Real)(P.brightness[c] / M_PI);
     const double tR = mag3(sub3(g, x)) / P.R;
-    o.tR = tR < 1.0e30 ? (Real)tR : Real(0);  // point scatter forms table indices from it
+    o.tR = ordinary_radii(P) ? (Real)tR : Real(0);
   }
   if (lane == 0) out[((long long)b * d.n0 + i) * d.T + k] = o;
 }
@@ -414,7 +414,7 @@ __device__ void sphere_direction(const AtmoParams* params, const BuildDims& d, c
                                  Real* offsets, int i, int t, int b) {
   const AtmoParams& P = params[b];
   const d3 x = mk3(index_to_radius(P, d.n0, (double)i), 0, 0);
-  const d3 n = mul3(x, 1.0 / mag3(x));
+  const d3 n = axis_normal(P, x);
   const d3 o1 = orthogonal(n);
   const d3 omega = to_world(n, o1, cross3(n, o1), dirs[t]);
   if (i == 0 && b == 0) {
@@ -486,7 +486,7 @@ __device__ void point_row(const AtmoParams* params, const BuildDims& d, PointRow
   o.cs = sqrt(dmax(0.0, dsub(1.0, sqr(ss))));
   o.lz = (Real)sqrt(dmax(0.0, dsub(dsub(1.0, sqr(o.cs)), sqr(ss))));
   const double gA = r * ss / P.R;
-  o.gA = fabs(gA) < 1.0e30 ? (Real)gA : Real(0);  // point scatter forms table indices from it
+  o.gA = ordinary_radii(P) ? (Real)gA : Real(0);
   split_coord<Real>(height_to_index(P, d.n0, r), d.n0, &o.u0, &o.s0);
   split_coord<Real>(sun_elevation_to_index(d.n2, mk3(r, 0, 0), mk3(ss, 0, 0)), d.n2, &o.u2, &o.s2);
   const double h = r - P.R;
