@@ -14,6 +14,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "blue_density.h"
 #include "kernels.h"
 
 namespace sfsim {
@@ -287,34 +288,42 @@ __device__ int step(double* density, unsigned char* mask, const Walk& w, int tot
 // density-array (bluenoise.clj:79-96): pixel p sums the weights of the set
 // pixels in row-major order, as density-sample does.  One warp per pixel row
 // segment would reorder the sum; one thread per pixel keeps it, so the chain
-// of additions is the cost.  Each block, one warp so that they spread over all
-// SMs, first lists the set pixels in order, and the chain has no others.
-// 64x64: 87 us (2048 set pixels, 40 ns each), 114 with 16 blocks of 256 threads
-// that walk all pixels.
-constexpr int kDensityThreads = 32;
-__host__ __device__ inline size_t blue_density_smem(int m) {
-  const size_t h = (size_t)(m / 2 + 1);
-  return sizeof(double) * h * h + sizeof(uchar2) * (((size_t)m * m + 1) / 2);
-}
-__global__ void __launch_bounds__(kDensityThreads)
+// segment would reorder the sum; one thread per pixel keeps it, so the chain
+// of additions is the cost.  Each block (blue_density.h: one warp, or as many as
+// fill the SMs in one wave) first lists the set pixels in order, a stretch of
+// them a warp, and the chain has no others.  64x64: 87 us (2048 set pixels, 40
+// ns each), 114 with 16 blocks of 256 threads that walk all pixels.
+__global__ void __launch_bounds__(32 * kDensityWarps)
     k_blue_density(int m, const double* __restrict__ table, const unsigned char* __restrict__ mask, double* density) {
   extern __shared__ __align__(16) unsigned char dsm[];
-  const int h = (m >> 1) + 1, total = m * m, lane = threadIdx.x;
+  __shared__ int counts[kDensityWarps];
+  const int h = (m >> 1) + 1, total = m * m, most = (total + 1) / 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   double* tb = reinterpret_cast<double*>(dsm);
   uchar2* list = reinterpret_cast<uchar2*>(tb + h * h);  // (x, y), m <= 256; at most half of the pixels are set
-  for (int t = lane; t < h * h; t += kDensityThreads) tb[t] = table[t];
-  int count = 0;
-  for (int t0 = 0; t0 < total; t0 += kDensityThreads) {
-    const int t = t0 + lane;
-    const bool set = t < total && mask[t];
-    const unsigned bits = __ballot_sync(0xffffffffu, set);
-    const int at = count + __popc(bits & ((1u << lane) - 1u));
-    if (set && at < (total + 1) / 2) list[at] = make_uchar2((unsigned char)(t % m), (unsigned char)(t / m));
-    count += __popc(bits);
+  for (int t = threadIdx.x; t < h * h; t += blockDim.x) tb[t] = table[t];
+  const int stretch = ((total + 31) / 32 + warps - 1) / warps * 32;
+  const int begin = warp * stretch, end = min(total, begin + stretch);
+  // the set pixels among t0 .. t0 + 31
+  auto set_bits = [&](int t0) { return __ballot_sync(0xffffffffu, t0 + lane < end && mask[t0 + lane]); };
+  int at = 0;
+  if (warps > 1) {
+    int mine = 0;
+    for (int t0 = begin; t0 < end; t0 += 32) mine += __popc(set_bits(t0));
+    if (lane == 0) counts[warp] = mine;
+    __syncthreads();
+    for (int w = 0; w < warp; w++) at += counts[w];
   }
-  count = min(count, (total + 1) / 2);
-  __syncwarp();
-  const int p = blockIdx.x * kDensityThreads + lane;
+  for (int t0 = begin; t0 < end; t0 += 32) {
+    const unsigned bits = set_bits(t0);
+    const int t = t0 + lane, to = at + __popc(bits & ((1u << lane) - 1u));
+    if ((bits >> lane & 1u) && to < most) list[to] = make_uchar2((unsigned char)(t % m), (unsigned char)(t / m));
+    at += __popc(bits);
+  }
+  if (threadIdx.x == blockDim.x - 32) counts[0] = min(at, most);  // the last warp's end
+  __syncthreads();
+  const int count = counts[0];
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= total) return;
   const int cy = p / m, cx = p - cy * m;
   double s = 0.0;
@@ -837,12 +846,17 @@ int launch_blue_noise(int m, int n, const int* seed, double sigma, const double*
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k, a) == cudaSuccess;
   };
-  const unsigned dblocks = (unsigned)((total + kDensityThreads - 1) / kDensityThreads);
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return -1;
+  const int dthreads = 32 * blue_density_warps(m, sms);
+  const unsigned dblocks = (unsigned)((total + dthreads - 1) / dthreads);
   // the seed mask, its density, the seed pattern, its density, phases 1-2,
   // the complement's density, phase 3
   k_blue_clear<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(total, mask, dither);
   k_blue_seed_set<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, seed, mask);
-  k_blue_density<<<dblocks, kDensityThreads, dsmem, st>>>(m, table, mask, density);
+  k_blue_density<<<dblocks, dthreads, dsmem, st>>>(m, table, mask, density);
   if (tiles) {
     if (launch_blue_tiles(0, m, n, table, density, density0, mask, work, dither, st)) return -1;
   } else if (nc) {
@@ -850,7 +864,7 @@ int launch_blue_noise(int m, int n, const int* seed, double sigma, const double*
   } else {
     k_blue_seed<<<1, kBlueThreads, smem, st>>>(a);
   }
-  k_blue_density<<<dblocks, kDensityThreads, dsmem, st>>>(m, table, mask, density0);
+  k_blue_density<<<dblocks, dthreads, dsmem, st>>>(m, table, mask, density0);
   if (tiles) {
     if (launch_blue_tiles(1, m, n, table, density, density0, mask, work, dither, st)) return -1;
   } else if (nc) {
@@ -858,7 +872,7 @@ int launch_blue_noise(int m, int n, const int* seed, double sigma, const double*
   } else {
     k_blue_phases<<<1, kBlueThreads, smem, st>>>(a);
   }
-  k_blue_density<<<dblocks, kDensityThreads, dsmem, st>>>(m, table, work, density);
+  k_blue_density<<<dblocks, dthreads, dsmem, st>>>(m, table, work, density);
   if (tiles) {
     if (launch_blue_tiles(2, m, n, table, density, density0, mask, work, dither, st)) return -1;
   } else if (nc) {
