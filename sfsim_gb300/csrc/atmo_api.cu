@@ -1749,11 +1749,15 @@ int build_static_impl(const sfsim_atmo_config& cfg, float* T, float* E, float* S
   // the fitted sun rays where they fit as well, else every sun ray is integrated
   w.fits = fit_groups(&cfg, 1, d, &hp);
   if (carve<Real>(w, nullptr, d, false) > kStaticScratchBytes) w.fits = FitGroups::none(1);
-  // and the surface-radiance weights of as many lights at a time as fit: the
-  // count above has more room than one light's (directions per height, four
-  // coordinates per node)
+  // and the surface-radiance weights of as many lights at a time as fit.  One
+  // light's, 2 Th n3 values, always do: the count above has the heading rows of
+  // every (height, sun elevation) pair, at least 384 n3 values, and from Th =
+  // 192 on three values a half-sphere direction and height, 15 Th^2, against
+  // the fewer than 600 headings that shared memory allows.
   while (d.half_slab > 1 && carve<Real>(w, nullptr, d, false) > kStaticScratchBytes)
     d.half_slab = (d.half_slab + 1) / 2;
+  if (carve<Real>(w, nullptr, d, false) > kStaticScratchBytes)
+    return fail(SFSIM_ATMO_ETOOBIG, "the build's scratch tables exceed the 67108864-byte static array");
   carve<Real>(w, (char*)base, d, false);
   // every scratch table is written before it is read, so nothing is cleared;
   // parameters and quadrature directions are copied in on the caller's stream
