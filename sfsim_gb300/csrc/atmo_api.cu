@@ -1713,7 +1713,8 @@ template <class Real>
 long long static_margin(const BuildDims& d) {
   auto up = [](long long x) { return (long long)((x + 255) & ~255LL); };
   const long long n = d.P + 16, n8 = (n + 7) / 8 * 8, R = sizeof(Real), n4 = d.n4(), pairs = (long long)d.n0 * d.n2;
-  const long long gone = 1024 + up(sizeof(SphereDir<Real>) * d.n0 * (d.P + 1LL)) + up(sizeof(SphereDir<Real>) * d.n0 * n) +
+  const long long direction = R == 8 ? 96 : 56;
+  const long long gone = 1024 + up(direction * d.n0 * (d.P + 1LL)) + up(direction * d.n0 * n) +
                          up(d.n0 * ((n8 * (9 * R + 4) + 15) & ~15LL)) + up(sizeof(int2) * d.n0) +
                          up(R * pairs * 2 * n8 * (d.n3 + 2) * 3) + up(4 * (sizeof(int) + R) * n4) + up(3 * R * n4) +
                          up((R == 8 ? 96 : 64) * pairs) + up(R * 3LL * d.nE0 * d.Ph) + up((8 + 7 * R) * d.nE());

@@ -914,14 +914,4 @@ __device__ __forceinline__ Real sun_elevation_index_r(Real sin_el, Real scale) {
   return r > Real(0) ? r : Real(0);
 }
 
-// sun_elevation_index_r for two values: the same operations per lane.
-template <class Real>
-__device__ __forceinline__ V2<Real> sun_elevation_index_r2(V2<Real> sin_el, Real scale) {
-  const V2<Real> z = mul2(fma2(mk2(Real(3), Real(3)), sin_el, mk2(Real(0.6), Real(0.6))),
-                          mk2(Real(-1.4426950408889634), Real(-1.4426950408889634)));
-  const V2<Real> e = mk2(Bulk<Real>::exp2(z.x), Bulk<Real>::exp2(z.y));
-  const V2<Real> r = mul2(sub2(mk2(Real(1), Real(1)), e), mk2(scale, scale));
-  return mk2(r.x > Real(0) ? r.x : Real(0), r.y > Real(0) ? r.y : Real(0));
-}
-
 }  // namespace sfsim

@@ -66,10 +66,10 @@ __device__ void row_map(const AtmoParams* params, const BuildDims& d, Remap2<Rea
   rowmap[b * d.rows() + row] = m;
 }
 
-// The height and elevation coordinates of a node are its row's (k_row_info);
+// The height and elevation coordinates of a node are its row's (row_map);
 // its light direction l = index-to-sun-direction(v, sin(k), a) has
 // x.l = r sin(k) with x = (r, 0, 0), so its sun-elevation coordinate is the
-// (i, k) one of k_point_rows, which also holds sin(k).  Left per node are the
+// (i, k) one of point_row, which also holds sin(k).  Left per node are the
 // sun-angle coordinate and l itself.
 template <class Real>
 __global__ void k_remap4(BuildDims d, const RowInfo* info, const PointRow<Real>* prow,
@@ -453,7 +453,6 @@ __global__ void k_sphere_setup(const AtmoParams* params, BuildDims d, const DirL
   o.w[2] = (Real)omega.z;
   o.weight = (Real)dirs[w].w;
   o.surface = surface;
-  o.pad = 0;
   split_coord<Real>(elevation_to_index(P, d.n1, x, omega, !surface), d.n1, &o.u1, &o.s1);
   if (surface) {
     Real tau[3];
@@ -566,10 +565,11 @@ static inline dim3 grid1(long long n, int block, int B) { return dim3((unsigned)
 // The set-up tables that need nothing but the parameters and the quadrature
 // directions, in one launch: they are FP64 chains of 10 to 25 us each (small
 // tables), and nine launches one after another held the iterations of a small
-// build back by 150 of its 260 us; now 162 us (8x16x8x4 tables, FP32).  Blocks
-// of one warp, so that what work there is spreads over the SMs' FP64 units.
-// Where the work is large (16 atmospheres of 16x128x16x8) they take as long as
-// they did apart, 1.9 ms with the maps and view rows, bound by FP64.
+// build back by 150 of its 260 us, 162 with this launch (8x16x8x4 tables,
+// FP32; 127 with what came later).  Blocks of one warp, so that what work
+// there is spreads over the SMs' FP64 units.  Where the work is large (16
+// atmospheres of 16x128x16x8) they take as long as they did apart, 1.9 ms with
+// the maps and view rows, bound by FP64.
 struct SetupParts {
   int blocks[kSetupParts];  // blocks of each part, 0 where it is not asked for
 };
