@@ -46,8 +46,10 @@ namespace sfsim {
 
 // Samples whose constants are formed at a time.
 constexpr int kRayBatch = 128;
-// Threads of a block at most: one per column, and one per cell.
-constexpr int kRayThreads = 320;
+// Threads of a block at most: one per column, and one per cell.  Blocks of 320
+// go three to an SM, of 512 two, of 1024 one, 64 registers a thread all the
+// same in FP32.  Rows of more columns take passes (WIDE), 512 at a time.
+constexpr int kRayThreads = 320, kRayThreadsMore = 512, kRayThreadsMost = 1024;
 constexpr int kRayThreadsWide = 512;
 
 __host__ __device__ constexpr int ray_column(int n2) { return 4 * (((n2 + 4) / 4) | 1); }
@@ -111,13 +113,21 @@ __device__ __forceinline__ double mask_value(double, int m) { return __longlong_
 __device__ __forceinline__ int mask_of(float v) { return __float_as_int(v); }
 __device__ __forceinline__ int mask_of(double v) { return (int)__double_as_longlong(v); }
 
-// WIDE: more columns than kRayThreads; they go in passes (the planes are built
-// again for each) and the threads walk the cells without keeping corners.
+// WIDE: more columns than kRayThreadsMost; they go in passes (the planes are
+// built again for each) and the threads walk the cells without keeping corners.
+// 32x127 rows, 100 samples, five iterations, by the sun elevations and headings:
+//                                64x4  36x7  85x3  40x8  64x8  48x16  200x4 ms
+//   one thread a column or cell  2.16  2.20  2.45  2.53  4.25  5.81   -
+//   WIDE                         3.86  3.97  4.09  4.23  10.2  15.9   23.6
+//   gathers per node (4 texels)  2.49  2.42  2.23  6.02  9.29  25.7   41.2
+// Two or three headings have as many columns as the nodes have columns to read,
+// so a column each gains nothing there: 128x2 2.32 and 2.24.  FP64, two
+// iterations of 8x32 rows: 64x4 1.65 / 2.06 / 1.89, 64x8 2.88 / 4.90 / 4.75.
 constexpr int kRayBlocks = 3;  // blocks per SM: 4.60 ms of a production build, two 5.04
 constexpr int kRayUnroll = 2;  // samples whose new corners are on their way together
 // SPLIT: several groups of threads share the ray's samples.
-template <class Real, bool WIDE, bool SPLIT>
-__global__ void __launch_bounds__(WIDE ? kRayThreadsWide : kRayThreads, WIDE || sizeof(Real) == 8 ? 1 : kRayBlocks)
+template <class Real, int THREADS, int BLOCKS, bool WIDE, bool SPLIT>
+__global__ void __launch_bounds__(THREADS, BLOCKS)
     k_ray_scatter(BuildDims d, RayLayout lay, const RowInfo* rowinfo, const RowSample<Real>* rows,
                   const CellGeom<Real>* geom, const Coord<Real>* angle, const Vec4<Real>* J, Vec4<Real>* dS,
                   int ngroups) {
@@ -352,7 +362,8 @@ int launch_ray_scatter(const BuildDims& d, const RowInfo* rowinfo, const RowSamp
                        const CellGeom<Real>* geom, const Coord<Real>* angle, const Vec4<Real>* J, Vec4<Real>* dS,
                        cudaStream_t st) {
   const int ncol = d.n2 * (d.n3 + 2);
-  const bool wide = ncol > kRayThreads;
+  constexpr bool one = sizeof(Real) == 8;  // block per SM: FP64's registers
+  const bool wide = ncol > kRayThreadsMost;
   // Few columns and few rows leave the SMs with a warp or two each, one after
   // another along the ray: then up to four groups of a block share its samples.
   // 128 rows of 48 columns, 64 samples, two iterations, 1 / 2 / 4 groups: FP32 37 /
@@ -365,9 +376,11 @@ int launch_ray_scatter(const BuildDims& d, const RowInfo* rowinfo, const RowSamp
          d.rows() * (2 * groups * per / 32) <= 4864)  // 32 warps an SM
     groups *= 2;
   const int block = per * groups;
-  // the most planes per buffer that let two blocks share an SM, else that fit
+  // the most planes per buffer that let two blocks share an SM (blocks that have one for themselves: that
+  // fit), else that fit
   RayLayout lay = ray_layout<Real>(d, 8, groups);
-  for (int ch = 8; ch >= 2 && lay.bytes > 100 * 1024; ch /= 2) lay = ray_layout<Real>(d, ch, groups);
+  const unsigned room = (per > kRayThreadsMore ? 220 : 100) * 1024;
+  for (int ch = 8; ch >= 2 && lay.bytes > room; ch /= 2) lay = ray_layout<Real>(d, ch, groups);
   const dim3 grid((unsigned)d.rows(), d.B);
   auto go = [&](auto kernel) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.bytes) != cudaSuccess)
@@ -375,9 +388,11 @@ int launch_ray_scatter(const BuildDims& d, const RowInfo* rowinfo, const RowSamp
     kernel<<<grid, block, lay.bytes, st>>>(d, lay, rowinfo, rows, geom, angle, J, dS, groups);
     return 0;
   };
-  return wide ? go(k_ray_scatter<Real, true, false>)
-         : groups > 1 ? go(k_ray_scatter<Real, false, true>)
-                      : go(k_ray_scatter<Real, false, false>);
+  if (wide) return go(k_ray_scatter<Real, kRayThreadsWide, 1, true, false>);
+  if (groups > 1) return go(k_ray_scatter<Real, kRayThreads, one ? 1 : kRayBlocks, false, true>);
+  if (per <= kRayThreads) return go(k_ray_scatter<Real, kRayThreads, one ? 1 : kRayBlocks, false, false>);
+  if (per <= kRayThreadsMore) return go(k_ray_scatter<Real, kRayThreadsMore, one ? 1 : 2, false, false>);
+  return go(k_ray_scatter<Real, kRayThreadsMost, 1, false, false>);
 }
 
 template int launch_ray_scatter<float>(const BuildDims&, const RowInfo*, const RowSample<float>*,
