@@ -39,7 +39,10 @@ UNIT = "ray-scatter cells/s (full multi-order LUT build)"
 # build, mean over its five launches in one ncu capture of this workload
 # (dram__bytes_read.sum + dram__bytes_write.sum); ncu does not run here, so the
 # figure is a recorded capture, not a measurement of this run
-PS_DRAM_BYTES_PER_LAUNCH = 39_200_000
+PS_DRAM_BYTES_PER_LAUNCH = 38_900_000
+# shared-memory wavefronts (128 B each) of the five launches, from the same capture
+# (l1tex__data_pipe_lsu_wavefronts_mem_shared.sum)
+PS_SMEM_WAVEFRONTS = 546_600_000
 TABLES = ("transmittance", "surface_radiance", "ray_scatter", "mie_strength")
 SUN_FIT_NODES = 8192 * 8 * 6  # sun rays integrated for the fits: heights x segments x Chebyshev nodes
 WORKLOAD = ("production LUT build: T 255x255, E 16x64, S/M 32x255x32x8 RGB, 5 iterations, "
@@ -269,7 +272,8 @@ def run_ours(args):
     smem_peak = ctypes.c_double()
     _lib.check(L.sfsim_atmo_smem_peak(ctypes.byref(smem_peak)), "smem_peak")
     ps_ms = stages["point_scatter"]
-    ps_achieved = ps_bytes / (ps_ms * 1e-3) / 1e9
+    ps_achieved = 128 * PS_SMEM_WAVEFRONTS / (ps_ms * 1e-3) / 1e9
+    ps_gathered = ps_bytes / (ps_ms * 1e-3) / 1e9
     smem_peak_g = smem_peak.value / 1e9
     peak = ctypes.c_double()
     _lib.check(L.sfsim_atmo_sfu_peak(ctypes.byref(peak)), "sfu_peak")
@@ -322,11 +326,13 @@ def run_ours(args):
                          "peak": smem_peak_g, "unit": "GB/s", "frac": ps_achieved / smem_peak_g if smem_peak_g else None,
                          "traffic": PS_DRAM_BYTES_PER_LAUNCH,
                          "traffic_source": "ncu capture of this workload (recorded figure, not measured in this run)",
-                         "note": ("achieved = algorithmic shared-memory gather bytes of the point-scatter stage "
-                                  "(24 B per direction and inner heading for the ring's row, 24 B more in the first "
-                                  "iteration and on the ground, 24 B per direction for the two outer headings; "
-                                  "census counts) / its event time; lanes that share a record are served together, "
-                                  "and the FMA pipe is as busy; peak = "
+                         "gather_achieved": ps_gathered,
+                         "note": ("achieved = 128 B per shared-memory wavefront of the point-scatter stage (a recorded "
+                                  "ncu count of this workload) / its event time; gather_achieved = the gathers' bytes "
+                                  "by lane (24 B per direction and inner heading for the ring's row, 24 B more in the "
+                                  "first iteration and on the ground, 24 B per direction for the two outer headings; "
+                                  "census counts), of which lanes that share a record are served together; issue and "
+                                  "the FMA pipe are as busy; peak = "
                                   "conflict-free shared-memory read bandwidth measured live on this GPU by "
                                   "sfsim_atmo_smem_peak (no such figure in MEASURED_PEAKS.json); DRAM is not "
                                   "the bound (the tables live in L2); traffic = DRAM bytes read + written per "

@@ -197,7 +197,8 @@ int launch_first_order(const AtmoParams* params, const BuildDims& d, const RowIn
   // A row's lit cells are half of them on average and all of them at worst, so
   // few rows leave SMs idle at the end: its cells are split over blocks, each
   // warp a cell or more, until the SMs have several blocks each.  128 rows of
-  // 32 cells and 64 steps: FP32 24.8 us whole, 20.4 in four; FP64 1.53 -> 1.44 ms.
+  // 32 cells and 64 steps: FP32 24.8 us whole, 20.4 in four; FP64 1.53 -> 1.44 ms
+  // (1.09 since its exponentials come from a table).
   const int ncell = d.n2 * d.n3;
   int parts = 1;
   while ((long long)parts * d.rows() * d.B < 1216 && ncell > parts * WARPS) parts *= 2;

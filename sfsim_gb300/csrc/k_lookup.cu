@@ -110,8 +110,8 @@ __device__ __forceinline__ float q_weight(float f, int bits) {
 // contiguous bytes, read in 16-byte words.  The six 4-byte loads it replaces
 // each went through L1 for 32 scattered addresses, which bound the lookups: L1
 // 91 % busy, 10 of its cycles a load, the L2 a fifth.  Measured, 1049353
-// in-scatter lookups of 32x127x32x8 tables 141 -> 100 us, 524309 attenuated
-// rays 156 -> 119.  The tables start at 256-byte boundaries of one allocation,
+// in-scatter lookups of 32x127x32x8 tables 141 -> 103 us, 524309 attenuated
+// rays 156 -> 129.  The tables start at 256-byte boundaries of one allocation,
 // so a table's last word is inside it.
 __device__ __forceinline__ void texel_pair(const float* t, int w, int h, int x, int y, f3& a, f3& b) {
   const int xa = min(max(x, 0), w - 1), xb = min(max(x + 1, 0), w - 1), x0 = min(xa, w - 2);
@@ -251,8 +251,9 @@ __device__ f3 in_scatter_at_g(const GlslEnv& e, f3 l, f3 p, f3 d) {
 }
 
 // Blocks an SM that the lookups' registers are limited for: 1049353 lookups of
-// in-scatter took 109 / 103 / 100 / 102 us at 4 / 5 / 6 / 8; the attenuation, with
-// twice the lookups at a time, 119 / 119 / 119 / 128.
+// in-scatter took 111 / 105 / 102 / 104 us at 4 / 5 / 6 / 8; the attenuation, with
+// twice the lookups at a time, 121 / 121 / 119 / 129 (the same points again; 129
+// at 4 where they are new ones each time).
 constexpr int kLookupBlocks = 6, kAttenuationBlocks = 4;
 template <int KIND>
 __global__ void __launch_bounds__(128, kLookupBlocks)

@@ -288,7 +288,6 @@ __device__ int step(double* density, unsigned char* mask, const Walk& w, int tot
 // density-array (bluenoise.clj:79-96): pixel p sums the weights of the set
 // pixels in row-major order, as density-sample does.  One warp per pixel row
 // segment would reorder the sum; one thread per pixel keeps it, so the chain
-// segment would reorder the sum; one thread per pixel keeps it, so the chain
 // of additions is the cost.  Each block (blue_density.h: one warp, or as many as
 // fill the SMs in one wave) first lists the set pixels in order, a stretch of
 // them a warp, and the chain has no others.  64x64: 87 us (2048 set pixels, 40

@@ -27,11 +27,10 @@
 // reads 32 different banks, and the builder's stores (for 8 headings, 4 sun
 // elevations x 8 headings a warp) do too.
 //
-// What bounds it: the L1 data pipe, 90 % busy with 261M wavefronts a launch of
-// the production tables (32x255x32x8, 128 samples) before the corners' offsets
-// were read only where they are needed: of 250 a row and sample 60 are the
-// gathers, 58 the constants (10 fewer since), 48 the loads of J, 32 the stores.
-// 0.88 ms a launch, 4.42 ms of a build, 4.60 with the offsets of every sample;
+// What bounds it: the L1 data pipe, 85 % busy with 236M wavefronts a launch of
+// the production tables (32x255x32x8, 128 samples): of 226 a row and sample 60
+// are the gathers, 48 the constants, 48 the loads of J, 32 the stores.  0.89 ms a
+// launch, 4.43 ms of a build, 4.60 with the offsets of every sample (90 %, 261M);
 // with a bilinear gather per node (four texels, every heading) 5.70.  The
 // reference's tables (32x127x32x8, 100 samples) 2.20 -> 1.83 -> 1.75 ms; 16
 // atmospheres of 16x128x16x8 7.6 -> 6.9.  Separate builder and gatherer warps
