@@ -142,7 +142,9 @@ int sfsim_atmo_build_device(const sfsim_atmo_config* cfg, float* transmittance,
  * except where the fitted sun rays (3 MB or more, taken by FP32 builds whose
  * ray-scatter cells times ray steps exceed about 1.9e7) no longer fit beside
  * the scratch tables: then every sun ray is integrated directly and the two
- * agree within 2e-5 relative.  Stage timings are not recorded. */
+ * agree within 5e-5 of a value or of a millionth of its table's largest,
+ * whichever is more (3.7e-5 at most over 16 atmospheres; 2e-6 in the surface
+ * radiance).  Stage timings are not recorded. */
 int sfsim_atmo_build_static(const sfsim_atmo_config* cfg, float* transmittance,
                             float* surface_radiance, float* ray_scatter,
                             float* mie_strength, void* stream);
