@@ -143,7 +143,7 @@ int sfsim_atmo_build_device(const sfsim_atmo_config* cfg, float* transmittance,
  * ray-scatter cells times ray steps exceed about 1.9e7) no longer fit beside
  * the scratch tables: then every sun ray is integrated directly and the two
  * agree within 5e-5 of a value or of a millionth of its table's largest,
- * whichever is more (3.7e-5 at most over 16 atmospheres; 2e-6 in the surface
+ * whichever is more (3.7e-5 at most over 16 atmospheres, 2.5e-6 in the surface
  * radiance).  Stage timings are not recorded. */
 int sfsim_atmo_build_static(const sfsim_atmo_config* cfg, float* transmittance,
                             float* surface_radiance, float* ray_scatter,
